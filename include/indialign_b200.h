@@ -336,6 +336,18 @@ int indialign_selftest_rcp(int n, const double *x, double *y);
  * the counterpart of the reference's cov_to_rotation (indialign_c/core.h:64-90). */
 int indialign_selftest_rotation(int n, const double *H, double *R);
 
+/* Diagnostic: one alignment of host points by the chains' NW fill and
+ * traceback.  rt = {R[9], t[3]}; smode 0 distance score (cutoff cut2), 1 label
+ * identity, 2 distance score + 0.5 for equal labels; warps 1 or 4 (sharing
+ * the alignment).  ap / an: min(plen, nlen) ints, *na: aligned pairs. */
+int indialign_selftest_nw(int plen, int nlen, const double *pred, const double *native, const double *rt,
+                          const uint8_t *lp, const uint8_t *ln, int smode, float gap, float inv_d0sq,
+                          float cut2, int warps, int *ap, int *an, int *na);
+
+/* Diagnostic: floats of [1, 2^127) for which the fill's reciprocal is not the
+ * correctly rounded one. */
+int indialign_selftest_rcp_f32(unsigned long long *mismatches);
+
 /* ---- length buckets and kernel shapes (no counterpart in the reference,
  * whose only shape choice is the block size of its GPU seed-bank kernel by
  * N, indialign_c/gpu_kernels.cu:227-229).  Every pair's work runs with the

@@ -243,9 +243,8 @@ __global__ void k_plan_chain(DevBatch b, PlanCtx c) {
     // -1e30 / identity result, which the caller then rescores
     if (on && T.n_chains == 0 && (c.kind == CH_LOCAL || c.kind == CH_THREAD || c.kind == CH_SINGLE))
         rec_ident(S.rec[REC_STAGE], kScoreInit);
-    T.chunk = c.tune.of(I.N).chain_chunk;  // the shape of the pair's length bucket
     c.ctasks[s] = T;
-    c.counts[s] = (T.n_chains + T.chunk - 1) / T.chunk;
+    c.counts[s] = T.n_chains;
 }
 
 // ---- chain reductions (warp per pair) ---------------------------------------

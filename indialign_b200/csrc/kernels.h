@@ -89,23 +89,33 @@ cudaError_t bank_set_attributes();
 const void *bank_kernel_ptr(bool smem);
 
 // k_chain.cu
+// Scratch of a chain launch: per resident warp an NW trace block, a boundary
+// row and an alignment, each in shared memory instead where `flags` says so.
+struct ChainScratch {
+    uint32_t *gtrace;
+    size_t trace_words;  // per warp
+    float *gbh;          // per warp 4 floats per column pair
+    uint32_t *gal;
+    int pmax, nmax;      // longest pred / native of the launch
+    int flags;           // in shared memory: 1 columns and labels, 2 boundary, 4 alignment, 8 trace
+    int chunk;           // most chains a CTA pulls at a time
+    int coop_max;        // launches of at most this many chains run one chain per CTA
+};
 size_t chain_smem_bytes(int pmax, int nmax, int flags);
-void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chunk_begin, int ntasks,
-                  const ScanOut *scan, int *counter, uint32_t *gtrace, size_t trace_words,
-                  double *gbh, uint32_t *gal, int pmax, int nmax, int flags, int grid, bool emit,
+void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, int ntasks,
+                  const ScanOut *scan, int *counter, const ChainScratch &sc, int grid, bool emit,
                   cudaStream_t st);
 cudaError_t chain_set_attributes();
 const void *chain_kernel_ptr();
 size_t nw_trace_words(int np, int nn);
-// NW trace words of an np x nn problem in k_chain.cu's layout: per 64-row
+// NW trace words of an explicit np x nn matrix in k_chain.cu's layout: per 64-row
 // stripe a block of G step words x 64 rows, G = (P + 127) / 16 with period
 // P = max(nn + 1, 64).
 constexpr size_t nw_trace_words_for(int np, int nn) {
     return (size_t)((np + 63) / 64) * 64 * (size_t)(((nn + 1 > 64 ? nn + 1 : 64) + 127) / 16);
 }
 void launch_nw_explicit(const double *smat, int np, int nn, double gap, uint32_t *trace,
-                        double *bH, uint32_t *al, int *ap, int *an, int *na,
-                        unsigned long long *ctr, cudaStream_t st);
+                        double *bH, uint32_t *al, int *ap, int *an, int *na, cudaStream_t st);
 
 // k_learn.cu -------------------------------------------------------------------
 // Ranker parameters on device: FP32 biases / standardisation and BF16 weight

@@ -8,13 +8,12 @@
 // (k_nw_explicit) with its scratch in a fixed file-scope device array
 // instead, so it allocates nothing.
 //
-// The array holds the NW trace, the stripe boundary row, the reversed
-// alignment and the kernel's work counters for one problem of at most
-// kNoAllocMaxLen x kNoAllocMaxLen (about 1.1 MB, held on every GPU that loads
+// The array holds the NW trace, the stripe boundary row and the reversed
+// alignment for one problem of at most kNoAllocMaxLen x kNoAllocMaxLen (about 1.1 MB, held on every GPU that loads
 // this library until the process exits).  All calls share it: two calls whose
 // kernels overlap on the GPU race on it.  The kernel zeroes the boundary row
 // itself and writes every trace word it later reads, so no state carries over
-// from the previous call; the counters are never read.  The first call on a
+// from the previous call.  The first call on a
 // device looks up the array's device address (cudaGetSymbolAddress) with
 // that device current.  The call returns after `stream` synchronizes.
 #include <cuda_runtime.h>
@@ -31,8 +30,7 @@ constexpr int kNoAllocMaxLen = 2048;
 constexpr size_t kNATraceWords = nw_trace_words_for(kNoAllocMaxLen, kNoAllocMaxLen);
 constexpr size_t kNABhOff = ((kNATraceWords * 4 + 255) / 256) * 256;
 constexpr size_t kNAAlOff = kNABhOff + (((kNoAllocMaxLen + 1) * 8 + 255) / 256) * 256;
-constexpr size_t kNACtrOff = kNAAlOff + ((kNoAllocMaxLen * 4 + 255) / 256) * 256;
-constexpr size_t kNABytes = kNACtrOff + 256;
+constexpr size_t kNABytes = kNAAlOff + ((kNoAllocMaxLen * 4 + 255) / 256) * 256;
 
 static __device__ __align__(256) unsigned char g_nw_scratch[kNABytes];
 
@@ -73,8 +71,7 @@ extern "C" int indialign_nw_align_noalloc(const double *d_smat, int np, int nn, 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     ia::launch_nw_explicit(d_smat, np, nn, gap, reinterpret_cast<uint32_t *>(base),
                            reinterpret_cast<double *>(base + ia::kNABhOff),
-                           reinterpret_cast<uint32_t *>(base + ia::kNAAlOff), d_ap, d_an, d_na,
-                           reinterpret_cast<unsigned long long *>(base + ia::kNACtrOff), st);
+                           reinterpret_cast<uint32_t *>(base + ia::kNAAlOff), d_ap, d_an, d_na, st);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {

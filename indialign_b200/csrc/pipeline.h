@@ -143,7 +143,6 @@ struct ChainTask {
     double *alP, *alQ;   // EMIT: aligned coordinates (contiguous)
     int al_cap;          // capacity per EMIT start
     int n_chains;        // n_starts*gaps (0 = inactive)
-    int chunk;           // chains per CTA chunk (the pair's length bucket)
     int chain_base;      // first chain in the launch's chain space
 };
 
@@ -242,6 +241,7 @@ enum DevError {
     DERR_TMA_TIMEOUT = 1,
     DERR_CAPACITY = 2,
     DERR_TRACE_CAP = 4,
+    DERR_NW_TIMEOUT = 8,
 };
 
 }  // namespace ia

@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/indialign_b200.h"
+#include "fill_geom.h"
 #include "kernels.h"
 #include "sched.cuh"
 
@@ -94,11 +95,12 @@ struct Ctx {
     DBuf<ChainTask> ctasks;
     DBuf<int> counts, begins, counter;
     DBuf<ScanOut> scan;
-    DBuf<double> item_res, chain_res, alP, alQ, thread_rec, off_start, off_res, gbh, out, snap;
+    DBuf<double> item_res, chain_res, alP, alQ, thread_rec, off_start, off_res, out, snap;
     DBuf<int> lay_i, gidx, omap;
     DBuf<long long> lay_l;
     DBuf<unsigned long long> ctr;
     // learned window ranker
+    DBuf<float> gbh;  // NW boundary rows
     DBuf<float> blob, wscore, wfeat, wlabel;
     DBuf<MlpPacked> mlp;
     DBuf<int> wcount, wlist, wsel;
@@ -206,6 +208,7 @@ struct Cfg {
     unsigned long long seed = 0;
     TuneRows tune;              // kernel shapes per length bucket (per task)
     int chain_smem_trace = 1;  // NW traces in shared memory (the longest pair's bucket)
+    int chain_chunk = 16;      // NW chains a CTA pulls at a time (the longest pair's bucket)
 };
 
 // Host view of per-pair facts after k_prep / k_anchor.
@@ -466,7 +469,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
         if (I.nlen > nmax) nmax = I.nlen;
     }
     chain_flags_ = 0;
-    if ((size_t)nmax * 17 + pmax + 256 <= 96 * 1024) chain_flags_ |= 1;
+    if ((size_t)nmax * 13 + pmax + 256 <= 96 * 1024) chain_flags_ |= 1;
     if (nmax <= 512) chain_flags_ |= 2;
     if ((pmax < nmax ? pmax : nmax) <= 2048) chain_flags_ |= 4;
     size_t smem = chain_smem_bytes(pmax, nmax, chain_flags_);
@@ -474,7 +477,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, chain_kernel_ptr(), 32 * kChainWarps,
                                                      smem));
     if (per_sm < 1) per_sm = 1;
-    trace_words_ = nw_trace_words_for(pmax, nmax);  // NW trace block per warp (k_chain.cu)
+    trace_words_ = fill_trace_words(pmax, nmax);  // NW trace block per warp
     // short pairs: the warps' traces in shared memory, when that keeps the
     // number of resident CTAs
     if (cfg_.chain_smem_trace) {
@@ -497,7 +500,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     if (chain_grid_ < 1) chain_grid_ = 1;
     size_t nw = (size_t)chain_grid_ * kChainWarps;
     CK(c_->gtrace.ensure((chain_flags_ & 8) ? 1 : nw * trace_words_));
-    CK(c_->gbh.ensure((chain_flags_ & 2) ? 1 : nw * (nmax + 1)));
+    CK(c_->gbh.ensure((chain_flags_ & 2) ? 1 : nw * fill_boundary_floats(nmax)));
     CK(c_->gal.ensure((chain_flags_ & 4) ? 1 : nw * (pmax < nmax ? pmax : nmax)));
     CK(c_->alP.ensure(3 * 2 * (size_t)(c_->h_off.empty() ? 1 : c_->h_off.back() + 2)));
     CK(c_->alQ.ensure(3 * 2 * (size_t)(c_->h_off.empty() ? 1 : c_->h_off.back() + 2)));
@@ -593,8 +596,9 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
         cudaEventRecord(e0, c_->stream);
     }
     const bool emit = kind == CH_SS2 || kind == CH_SS4 || kind == CH_DP_EMIT;
-    launch_chain(b, c_->ctasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->gtrace.p,
-                 trace_words_, c_->gbh.p, c_->gal.p, pmax, nmax, chain_flags_, chain_grid_, emit,
+    const ChainScratch sc = {c_->gtrace.p, trace_words_, c_->gbh.p, c_->gal.p,        pmax,
+                             nmax,         chain_flags_, cfg_.chain_chunk, chain_grid_};
+    launch_chain(b, c_->ctasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, sc, chain_grid_, emit,
                  c_->stream);
     if (timing) {
         cudaEventRecord(e1, c_->stream);
@@ -1356,6 +1360,7 @@ static int run_search(int device, const Cfg &cfg0, const Source &src, double *re
         Cfg cfg = cfg0;
         cfg.tune = tt.rows();
         cfg.chain_smem_trace = tt.t[bucket_of(tt, Lmax)].chain_smem_trace;
+        cfg.chain_chunk = tt.t[bucket_of(tt, Lmax)].chain_chunk;
         Ctx *c = nullptr;
         int rc = acquire(device, &c);
         if (rc) return rc;
@@ -1395,6 +1400,7 @@ static int run_search(int device, const Cfg &cfg0, const Source &src, double *re
         P.cfg = cfg0;
         P.cfg.tune = tt.rows();
         P.cfg.chain_smem_trace = tt.t[b].chain_smem_trace;
+        P.cfg.chain_chunk = tt.t[b].chain_chunk;
         if (!src.host.empty()) {
             for (int p : I) P.src.host.push_back(src.host[p]);
         } else {
@@ -1619,15 +1625,14 @@ int indialign_nw_align(const double *d_smat, int np, int nn, double gap, int *d_
     rc = INDIALIGN_OK;
     do {
         const size_t words = ia::nw_trace_words(np, nn);
-        if (c->gtrace.ensure(words) != cudaSuccess || c->gbh.ensure((size_t)nn + 1) != cudaSuccess ||
-            c->gal.ensure((size_t)(np < nn ? np : nn)) != cudaSuccess ||
-            c->ctr.ensure(ia::kCounters) != cudaSuccess) {
+        if (c->gtrace.ensure(words) != cudaSuccess || c->gbh.ensure(2 * ((size_t)nn + 1)) != cudaSuccess ||
+            c->gal.ensure((size_t)(np < nn ? np : nn)) != cudaSuccess) {
             ia::g_last_error = "nw_align: workspace allocation failed";
             rc = INDIALIGN_E_CUDA;
             break;
         }
-        ia::launch_nw_explicit(d_smat, np, nn, gap, c->gtrace.p, c->gbh.p, c->gal.p, d_ap, d_an, d_na,
-                               c->ctr.p, st);
+        ia::launch_nw_explicit(d_smat, np, nn, gap, c->gtrace.p, reinterpret_cast<double *>(c->gbh.p), c->gal.p,
+                               d_ap, d_an, d_na, st);
         cudaError_t e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) {
