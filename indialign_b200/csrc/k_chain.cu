@@ -351,10 +351,11 @@ IA_DEV void put_rt(double *dst, const double *R, const double *t, int lane) {
 // chains leaves most of the chip idle with a warp per chain, and its time is
 // the longest chain's: then a CTA takes one chain at a time, its warps share
 // the fill's stripes, and warp 0 does the rest.  Measured, both with the fill
-// of nw_fill.cuh against the one before it: one pair of L = 1203 261 -> 70 ms
-// (its SS and dp_refine stages, one or two alignments at a time, 80 -> 18 ms),
-// learned search of 64 pairs of L 30-1500 285 -> 65 ms.  The line lies at one
-// chain per CTA slot of the chip: above it the slots are full either way.
+// of nw_fill.cuh against a warp per chain with the fill before it: one pair of
+// L = 1203 261 -> 60 ms (its SS and dp_refine stages, one or two alignments at
+// a time, 80 -> 18 ms), learned search of 64 pairs of L 30-1500 285 -> 60 ms.
+// The line lies at one chain per CTA slot of the chip: above it the slots are
+// full either way.
 template <bool EMIT>
 __global__ void __launch_bounds__(32 * kChainWarps, IA_CHAIN_MINB)
 k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__ chain_begin,
@@ -366,25 +367,24 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
     // shared memory so that no transform stays live in registers across the
     // NW fill
     __shared__ double s_rt[kChainWarps][24];
-    __shared__ float s_slot[kChainWarps][3 * 4 * 32];  // moved points of a warp's next stripe
     __shared__ int s_prog[kChainWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // shared layout: [native column pairs, 24 B][pred labels][native labels]
+    // shared layout: [native column pairs][pred labels][native labels]
     // (flag 1), then per warp the NW boundary row (flag 2), the alignment
     // (flag 4) and the NW trace block (flag 8, short pairs); the FP64 point
     // sets are read from global memory (L1)
     const int pmax = sc.pmax, nmax = sc.nmax, flags = sc.flags;
     const bool coord_smem = flags & 1, bh_smem = flags & 2, al_smem = flags & 4, tr_smem = flags & 8;
-    const uint32_t npmax = ((uint32_t)nmax + 1u) >> 1, qbytes = (npmax * 24u + 15u) & ~15u;
+    const uint32_t qfloats = (uint32_t)fill_column_floats(nmax), qbytes = (qfloats * 4u + 15u) & ~15u;
     const uint32_t plb = ((uint32_t)pmax + 47u) & ~15u, nlb = ((uint32_t)nmax + 47u) & ~15u;
-    char *sQ = smem;
-    char *sLp = sQ + (coord_smem ? qbytes : 0), *sLn = sLp + (coord_smem ? plb : 0);
+    char *sLp = smem + (coord_smem ? qbytes : 0), *sLn = sLp + (coord_smem ? plb : 0);
     char *wbase = sLn + (coord_smem ? nlb : 0);
-    const uint32_t bh_bytes = npmax * 16u;
+    float *cols = (coord_smem ? reinterpret_cast<float *>(smem) : sc.gcol + (size_t)blockIdx.x * qfloats) + 6 * kFillPad;
+    const uint32_t bh_floats = (uint32_t)fill_boundary_floats(nmax);
     const uint32_t al_bytes = ((uint32_t)min(pmax, nmax) * 4u + 15u) & ~15u;
-    float *bh0 = bh_smem ? reinterpret_cast<float *>(wbase)
-                         : sc.gbh + (size_t)blockIdx.x * kChainWarps * npmax * 4;  // the CTA's boundary rows
-    char *albase = wbase + (bh_smem ? kChainWarps * bh_bytes : 0);
+    float *bh0 = (bh_smem ? reinterpret_cast<float *>(wbase) : sc.gbh + (size_t)blockIdx.x * kChainWarps * bh_floats) +
+                 4 * kFillPad;  // the CTA's boundary rows
+    char *albase = wbase + (bh_smem ? kChainWarps * bh_floats * 4 : 0);
     char *trbase = albase + (al_smem ? kChainWarps * al_bytes : 0);
     uint32_t phase = 0;
     if (threadIdx.x == 0) {
@@ -406,11 +406,10 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
     const bool lead = !coop || warp == 0;  // does a chain's work beside the fill
     int staged = -1;
     FillArgs fa;
-    fa.qa = nullptr;
-    fa.qb = nullptr;
+    fa.q = cols;
     fa.trace = trace;
-    fa.bw = bh0 + (size_t)warp * npmax * 4;
-    fa.br = bh0 + (size_t)(coop ? (warp + kChainWarps - 1) % kChainWarps : warp) * npmax * 4;
+    fa.bw = bh0 + (size_t)warp * bh_floats;
+    fa.br = bh0 + (size_t)(coop ? (warp + kChainWarps - 1) % kChainWarps : warp) * bh_floats;
     fa.prog = s_prog;
     fa.err = b.err;
     for (;;) {
@@ -454,30 +453,20 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             fa.plen = plen;
             fa.nlen = nlen;
             fa.P = x.P;
-            fa.Q = x.Q;
             fa.Lp = gLp;
             fa.Ln = gLn;
-            if (coord_smem) {
-                if (EMIT) {
-                    Copy cp[2];
-                    char *dst[2] = {sLp, sLn};
-                    cp[0] = plan_copy(gLp, (uint32_t)plen);
-                    cp[1] = plan_copy(gLn, (uint32_t)nlen);
-                    stage_copies(cp, dst, 2, &bar, phase, b.err);
-                    fa.Lp = reinterpret_cast<const uint8_t *>(sLp + cp[0].lead);
-                    fa.Ln = reinterpret_cast<const uint8_t *>(sLn + cp[1].lead);
-                }
-                float4 *qa = reinterpret_cast<float4 *>(sQ);
-                float2 *qb = reinterpret_cast<float2 *>(sQ + 16 * (size_t)npmax);
-                for (int i = threadIdx.x; i < (nlen + 1) >> 1; i += blockDim.x) {
-                    const double *q0 = x.Q + 6 * (size_t)i, *q1 = 2 * i + 1 < nlen ? q0 + 3 : q0;
-                    qa[i] = make_float4(-(float)q0[0], -(float)q1[0], -(float)q0[1], -(float)q1[1]);
-                    qb[i] = make_float2(-(float)q0[2], -(float)q1[2]);
-                }
-                fa.qa = qa;
-                fa.qb = qb;
-                __syncthreads();
+            if (coord_smem && EMIT) {
+                Copy cp[2];
+                char *dst[2] = {sLp, sLn};
+                cp[0] = plan_copy(gLp, (uint32_t)plen);
+                cp[1] = plan_copy(gLn, (uint32_t)nlen);
+                stage_copies(cp, dst, 2, &bar, phase, b.err);
+                fa.Lp = reinterpret_cast<const uint8_t *>(sLp + cp[0].lead);
+                fa.Ln = reinterpret_cast<const uint8_t *>(sLn + cp[1].lead);
             }
+            // (all tasks of a launch share their score mode)
+            stage_columns(cols, x.Q, nlen, EMIT && T.smode == SMAT_SS4, threadIdx.x, blockDim.x);
+            __syncthreads();
             staged = T.pair;
         }
         // dp_refine_chunk / ss_nw_align need >= 3 valid residues on each side
@@ -504,12 +493,11 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             const int w = coop ? warp : 0;
             fa.gap = (float)gap;
             if (!EMIT || T.smode == SMAT_DP) {
-                if (gap == 0.0) nw_fill_r<SMAT_DP, false>(fa, geom, w, s_slot[warp]);
-                else nw_fill_r<SMAT_DP, true>(fa, geom, w, s_slot[warp]);
+                nw_fill_r<SMAT_DP>(fa, geom, w);
             } else if (T.smode == SMAT_SS4) {
-                nw_fill_r<SMAT_SS4, true>(fa, geom, w, s_slot[warp]);
+                nw_fill_r<SMAT_SS4>(fa, geom, w);
             } else {
-                nw_fill_r<SMAT_SS2, true>(fa, geom, w, s_slot[warp]);
+                nw_fill_r<SMAT_SS2>(fa, geom, w);
             }
             if (coop) __syncthreads();
             int na = 0;
@@ -660,12 +648,11 @@ void launch_nw_explicit(const double *smat, int np, int nn, double gap, uint32_t
 
 size_t chain_smem_bytes(int pmax, int nmax, int flags) {
     size_t s = 0;
-    const size_t npmax = ((size_t)nmax + 1) / 2;
     if (flags & 1) {
-        s += (npmax * 24 + 15) & ~size_t(15);
+        s += (fill_column_floats(nmax) * 4 + 15) & ~size_t(15);
         s += (((size_t)pmax + 47) & ~size_t(15)) + (((size_t)nmax + 47) & ~size_t(15));
     }
-    if (flags & 2) s += kChainWarps * npmax * 16;
+    if (flags & 2) s += kChainWarps * fill_boundary_floats(nmax) * 4;
     if (flags & 4) s += kChainWarps * (((size_t)min(pmax, nmax) * 4 + 15) & ~size_t(15));
     if (flags & 8) s += kChainWarps * fill_trace_words(pmax, nmax) * 4;
     return s;
@@ -696,22 +683,22 @@ namespace ia {
 
 // One alignment by the search's fill and traceback (warps: 1 or kChainWarps).
 __global__ void __launch_bounds__(32 * kChainWarps, IA_CHAIN_MINB)
-k_nw_selftest(FillArgs fa, int smode, int warps, uint32_t *al, int *na_out) {
-    __shared__ float s_slot[kChainWarps][3 * 4 * 32];
+k_nw_selftest(FillArgs fa, const double *Q, float *cols, int smode, int warps, uint32_t *al, int *na_out) {
     __shared__ int s_prog[kChainWarps];
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x < kChainWarps) s_prog[threadIdx.x] = 0;
+    fa.q = cols + 6 * kFillPad;
+    stage_columns(cols + 6 * kFillPad, Q, fa.nlen, smode == SMAT_SS4, threadIdx.x, blockDim.x);
     __syncthreads();
     const FillGeom g = fill_geom(fa.plen, fa.nlen, warps);
     const size_t row = fill_boundary_floats(fa.nlen);
-    float *bnd = fa.bw;
+    float *bnd = fa.bw + 4 * kFillPad;
     fa.prog = s_prog;
     fa.bw = bnd + warp * row;
     fa.br = bnd + (warps > 1 ? (warp + warps - 1) % warps : 0) * row;
-    if (smode == SMAT_SS2) nw_fill_r<SMAT_SS2, true>(fa, g, warp, s_slot[warp]);
-    else if (smode == SMAT_SS4) nw_fill_r<SMAT_SS4, true>(fa, g, warp, s_slot[warp]);
-    else if (fa.gap == 0.f) nw_fill_r<SMAT_DP, false>(fa, g, warp, s_slot[warp]);
-    else nw_fill_r<SMAT_DP, true>(fa, g, warp, s_slot[warp]);
+    if (smode == SMAT_SS2) nw_fill_r<SMAT_SS2>(fa, g, warp);
+    else if (smode == SMAT_SS4) nw_fill_r<SMAT_SS4>(fa, g, warp);
+    else nw_fill_r<SMAT_DP>(fa, g, warp);
     __syncthreads();
     if (warp == 0) {
         const int na = nw_traceback(fa.trace, g, fa.plen, fa.nlen, al);
@@ -741,14 +728,14 @@ extern "C" int indialign_selftest_nw(int plen, int nlen, const double *pred, con
         !na || (warps != 1 && warps != kChainWarps) || smode < 0 || smode > SMAT_SS4)
         return INDIALIGN_E_INPUT;
     const size_t words = fill_trace_words(plen, nlen), row = fill_boundary_floats(nlen);
-    const size_t sizes[8] = {24 * (size_t)plen, 24 * (size_t)nlen, 96, (size_t)plen, (size_t)nlen,
-                             4 * words, 16 * row, 4 * (size_t)(plen < nlen ? plen : nlen) + 16};
-    size_t at[9] = {0};
-    for (int k = 0; k < 8; k++) at[k + 1] = at[k] + (sizes[k] + 255) / 256 * 256;
+    const size_t sizes[9] = {24 * (size_t)plen, 24 * (size_t)nlen, 96, (size_t)plen, (size_t)nlen, 4 * words,
+                             16 * row, 4 * fill_column_floats(nlen), 4 * (size_t)(plen < nlen ? plen : nlen) + 16};
+    size_t at[10] = {0};
+    for (int k = 0; k < 9; k++) at[k + 1] = at[k] + (sizes[k] + 255) / 256 * 256;
     char *d = nullptr;
-    if (cudaMalloc(&d, at[8]) != cudaSuccess) return INDIALIGN_E_CUDA;
+    if (cudaMalloc(&d, at[9]) != cudaSuccess) return INDIALIGN_E_CUDA;
     const void *src[5] = {pred, native, rt, lp, ln};
-    cudaError_t e = cudaMemset(d, 0, at[8]);
+    cudaError_t e = cudaMemset(d, 0, at[9]);
     for (int k = 0; k < 5 && e == cudaSuccess; k++) e = cudaMemcpy(d + at[k], src[k], sizes[k], cudaMemcpyHostToDevice);
     std::vector<uint32_t> al(plen < nlen ? plen : nlen);
     int out[2] = {0, 0};
@@ -757,7 +744,6 @@ extern "C" int indialign_selftest_nw(int plen, int nlen, const double *pred, con
         fa.plen = plen;
         fa.nlen = nlen;
         fa.P = reinterpret_cast<const double *>(d + at[0]);
-        fa.Q = reinterpret_cast<const double *>(d + at[1]);
         fa.rt = reinterpret_cast<const double *>(d + at[2]);
         fa.Lp = reinterpret_cast<const uint8_t *>(d + at[3]);
         fa.Ln = reinterpret_cast<const uint8_t *>(d + at[4]);
@@ -766,10 +752,11 @@ extern "C" int indialign_selftest_nw(int plen, int nlen, const double *pred, con
         fa.cut2 = cut2;
         fa.trace = reinterpret_cast<uint32_t *>(d + at[5]);
         fa.bw = reinterpret_cast<float *>(d + at[6]);
-        uint32_t *dal = reinterpret_cast<uint32_t *>(d + at[7]);
-        int *dna = reinterpret_cast<int *>(d + at[7] + (at[8] - at[7]) - 16);
+        uint32_t *dal = reinterpret_cast<uint32_t *>(d + at[8]);
+        int *dna = reinterpret_cast<int *>(d + at[9] - 16);
         fa.err = dna + 1;
-        k_nw_selftest<<<1, 32 * warps>>>(fa, smode, warps, dal, dna);
+        k_nw_selftest<<<1, 32 * warps>>>(fa, reinterpret_cast<const double *>(d + at[1]),
+                                         reinterpret_cast<float *>(d + at[7]), smode, warps, dal, dna);
         e = cudaMemcpy(out, dna, sizeof out, cudaMemcpyDeviceToHost);
         if (e == cudaSuccess) e = cudaMemcpy(al.data(), dal, al.size() * 4, cudaMemcpyDeviceToHost);
     }

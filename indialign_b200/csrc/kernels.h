@@ -90,11 +90,13 @@ const void *bank_kernel_ptr(bool smem);
 
 // k_chain.cu
 // Scratch of a chain launch: per resident warp an NW trace block, a boundary
-// row and an alignment, each in shared memory instead where `flags` says so.
+// row and an alignment, per CTA its pair's staged columns, each in shared
+// memory instead where `flags` says so.
 struct ChainScratch {
     uint32_t *gtrace;
     size_t trace_words;  // per warp
-    float *gbh;          // per warp 4 floats per column pair
+    float *gbh;          // per warp fill_boundary_floats(nmax)
+    float *gcol;         // per CTA fill_column_floats(nmax)
     uint32_t *gal;
     int pmax, nmax;      // longest pred / native of the launch
     int flags;           // in shared memory: 1 columns and labels, 2 boundary, 4 alignment, 8 trace

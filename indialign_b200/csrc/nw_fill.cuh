@@ -3,28 +3,40 @@
 // computed on the fly from the transformed pred rows and the native columns
 // (indialign_c/nw.h:10-68, align.h:86-98, ss.h:56-136).
 //
-// Shape.  A lane owns R consecutive rows (R <= 4) of a stripe of 32 R rows and
-// computes a block of R rows x 2 columns per step; lane l trails lane l-1 by
-// one step, so the two bottom values of a lane reach the next lane by a
-// shuffle of the step before.  The fill is bound by instruction issue and the
-// half-rate ALU pipe, so the block is shaped to spend as few instructions per
-// cell as possible:
+// Shape.  A lane owns R consecutive rows of a stripe of 32 R rows and computes
+// a block of R rows x 2 columns per step; lane l trails lane l-1 by one step,
+// so the two bottom values of a lane reach the next lane by a shuffle of the
+// step before.  The fill is bound by instruction issue and instruction fetch
+// (the chip's warps run several loops at once and each loop's code competes
+// for the instruction cache), so the step is shaped to be short, in issue
+// slots per cell and in code:
 //   * the two columns of a row share paired FP32 instructions for the score
 //     entry (difference, d2, 1 + d2/d0^2, and the reciprocal's Newton step):
 //     half an instruction per cell each, with the native columns staged
-//     negated in pairs so that a step loads them with two shared-memory reads;
-//   * one step's bookkeeping (shuffles, loads, loop, boundary) is shared by
-//     2 R cells;
+//     negated in pairs;
 //   * a direction is two bits in two planes, "not diagonal" and "left < up",
 //     each taken from the sign of one subtraction (FMA pipe) and shifted into
 //     its word by one funnel shift, instead of compares and selects (ALU pipe).
-//     All values are finite and >= 0 there, so a difference is +0 or positive
-//     exactly when the comparison holds.
-// A warp walks stripes w, w + W, w + 2W, ... (W warps share one alignment, or
-// W = 1); its lanes wrap into the next stripe without draining, with period
-// P2 steps.  The stripe's last row goes to the next stripe through a boundary
-// row in memory; with W > 1 the producer publishes its step count once per 16
-// steps and the consumer waits (bounded) before it starts a group of 16.
+//     All values are finite there, so a difference is +0 or positive exactly
+//     when the comparison holds;
+//   * one step's bookkeeping (shuffles, loads, loop) is shared by 2 R cells and
+//     has no branch: a stripe's lanes start together, and a lane whose first
+//     column has not come yet works on staged NaN columns, on which a cell
+//     leaves H = 0, the boundary value; columns and the boundary row carry
+//     padding on both sides, so no index is clamped.
+// Stripes run one after the other (31 idle lane steps each).  The stripe's last
+// row goes to the next stripe through a boundary row in memory.  W warps may
+// share one alignment: warp w takes stripes w, w + W, ..., publishes per 16
+// steps how many boundary pairs it has written, and waits (bounded) for those
+// of the stripe above before it starts a group of 16.
+//
+// Measured (B200) against two rows per lane and one column per step with
+// scalar entries, compare / select directions and a cell-by-cell traceback:
+// fill 14 -> 3.3 warp cycles per cell on 48 pairs of L 30-1500, 19.5 -> 4.3 on
+// 64 pairs of L 40-300 (whose last stripes are emptier); traceback 0.8 -> 0.14
+// and 2.9 -> 0.72.  Lanes that wrap into the next stripe without draining, with
+// the entry code inside the step loop, took 4.4 and 8.7 (half of the warps'
+// time without an instruction to issue); unrolling that loop twice, 6.3 and 15.
 #pragma once
 #include "dmath.cuh"
 #include "fill_geom.h"
@@ -39,17 +51,41 @@ struct FillArgs {
     int plen, nlen;
     const double *P;          // compact pred xyz
     const double *rt;         // transform {R[9], t[3]}
-    const float4 *qa;         // native column pairs {-x0, -x1, -y0, -y1} ...
-    const float2 *qb;         // ... {-z0, -z1} (shared memory), or null:
-    const double *Q;          // compact native xyz, converted on load
+    const float *q;           // native column pairs (stage_columns), pair 0
     const uint8_t *Lp, *Ln;   // SS labels (SS modes)
     float gap, inv_d0sq, cut2;
     uint32_t *trace;          // the alignment's trace block
-    float *bw;                // boundary row this warp writes
+    float *bw;                // boundary row this warp writes, pair 0
     const float *br;          // boundary row of the stripe above (W = 1: the same row)
-    volatile int *prog;       // W > 1: per warp, steps whose boundary values are written
+    volatile int *prog;       // W > 1: per warp, boundary pairs written
     int *err;
 };
+
+// Native column pair k as {-x0, -x1, -y0, -y1, -z0, -z1} at dst + 6 k, for
+// k = -kFillPad .. pairs + kFillPad - 1: NaN left of the matrix (see
+// fill_cell), the last pair's values right of it.  A non-finite coordinate
+// becomes a point 2e30 away from any other (moved_row puts non-finite rows on
+// the other side), whose squared distance is infinite: beyond the cutoff, as
+// the comparison with NaN or infinity makes it.  The SS4 mode has no cutoff
+// and takes the values as they are.
+IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int tid, int nthreads) {
+    const int pairs = (nlen + 1) >> 1;
+    for (int e = tid; e < 2 * (pairs + 2 * kFillPad); e += nthreads) {
+        const int k = (e >> 1) - kFillPad, half = e & 1;
+        float x = NAN, y = NAN, z = NAN;
+        if (k >= 0) {
+            const double *q = Q + 3 * (size_t)min(2 * k + half, nlen - 1);
+            x = (float)q[0];
+            y = (float)q[1];
+            z = (float)q[2];
+            if (!raw && !(isfinite(x) && isfinite(y) && isfinite(z))) x = y = z = 1e30f;
+        }
+        float *o = dst + 6 * k + half;
+        o[0] = -x;
+        o[2] = -y;
+        o[4] = -z;
+    }
+}
 
 // 1/x for x in [1, 2^127), correctly rounded: the hardware approximation
 // (within 1 ulp) and one Newton-Raphson step with a fused residual, which
@@ -62,33 +98,39 @@ IA_DEV float rcp_f32(float x) {
 }
 
 // Score entries of one row (its point in every half of mx, my, mz) and two
-// columns: 1/(1 + d2/d0^2), or 0 beyond the cutoff (distance mode); plus 0.5
-// for equal labels (SS4); label identity (SS2).  Operation order of a term:
-// d2 = fma(dz, dz, fma(dx, dx, dy dy)), fma(d2, 1/d0^2, 1).
+// columns: 1/(1 + d2/d0^2), or 0 beyond the cutoff (distance mode; NaN left of
+// the matrix); plus 0.5 for equal labels (SS4); label identity (SS2).
+// Operation order of a term: d2 = fma(dz, dz, fma(dx, dx, dy dy)),
+// fma(d2, 1/d0^2, 1).
 template <int SMODE>
-IA_DEV float2 score_pair(float2 mx, float2 my, float2 mz, float4 qa, float2 qb, float2 ninv, float2 none, float inv,
-                         float cut2, uint8_t lp, uint8_t ln0, uint8_t ln1) {
-    if (SMODE == SMAT_SS2) return make_float2(lp == ln0 ? 1.f : 0.f, lp == ln1 ? 1.f : 0.f);
-    const float2 dx = __fadd2_rn(mx, make_float2(qa.x, qa.y)), dy = __fadd2_rn(my, make_float2(qa.z, qa.w)),
-                 dz = __fadd2_rn(mz, qb);
+IA_DEV float2 score_pair(float2 mx, float2 my, float2 mz, float2 qx, float2 qy, float2 qz, float2 ninv, float inv,
+                         float cut2, uint8_t lp, uint8_t ln0, uint8_t ln1, bool left_of) {
+    float2 r;
+    if (SMODE == SMAT_SS2) {
+        r = make_float2(lp == ln0 ? 1.f : 0.f, lp == ln1 ? 1.f : 0.f);
+        return left_of ? make_float2(NAN, NAN) : r;
+    }
+    const float2 dx = __fadd2_rn(mx, qx), dy = __fadd2_rn(my, qy), dz = __fadd2_rn(mz, qz);
     const float2 d2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
     if (SMODE == SMAT_SS4) {  // no cutoff: infinite and NaN distances reach the reciprocal
         const float r0 = __frcp_rn(fmaf(d2.x, inv, 1.f)), r1 = __frcp_rn(fmaf(d2.y, inv, 1.f));
-        return make_float2(lp == ln0 ? r0 + 0.5f : r0, lp == ln1 ? r1 + 0.5f : r1);
+        r = make_float2(lp == ln0 ? r0 + 0.5f : r0, lp == ln1 ? r1 + 0.5f : r1);
+        return left_of ? make_float2(NAN, NAN) : r;
     }
-    const float2 nden = __ffma2_rn(d2, ninv, none);  // -(1 + d2/d0^2)
+    const float2 nden = __ffma2_rn(d2, ninv, make_float2(-1.f, -1.f));  // -(1 + d2/d0^2)
     float2 y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-nden.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-nden.y));
-    const float2 r = __ffma2_rn(y, __ffma2_rn(nden, y, make_float2(1.f, 1.f)), y);
-    return make_float2(d2.x <= cut2 ? r.x : 0.f, d2.y <= cut2 ? r.y : 0.f);
+    r = __ffma2_rn(y, __ffma2_rn(nden, y, make_float2(1.f, 1.f)), y);
+    return make_float2(d2.x > cut2 ? 0.f : r.x, d2.y > cut2 ? 0.f : r.y);
 }
 
 // One cell (indialign_c/nw.h:20-35): diag wins ties, then left, then up; a gap
 // move out of a cell that was reached diagonally pays `gap`, so a cell hands
 // on its H and, for gap moves, hp = H (+ gap if diagonal).  `a` and `b` take
-// the bits "not diagonal" and "left < up".
-template <int SMODE, bool GAP>
+// the bits "not diagonal" and "left < up".  A NaN score left of the matrix
+// (left = up = 0) gives H = hp = 0.
+template <int SMODE>
 IA_DEV void fill_cell(float diag_src, float sc, float up, float left, float gap, float &h, float &hp, uint32_t &a,
                       uint32_t &b) {
     const float diag = diag_src + sc;
@@ -106,8 +148,7 @@ IA_DEV void fill_cell(float diag_src, float sc, float up, float left, float gap,
     a = __funnelshift_l(__float_as_uint(x), a, 1);
     b = __funnelshift_l(__float_as_uint(y), b, 1);
     h = fmaxf(diag, m);
-    if (GAP) hp = diag >= m ? diag + gap : m;
-    else hp = h;
+    hp = diag >= m ? diag + gap : m;
 }
 
 // A lane's 2R trace words of one 16-step group, shifted left by sh.
@@ -123,206 +164,144 @@ IA_DEV void store_words(uint32_t *p, const uint32_t (&a)[R], const uint32_t (&b)
     }
 }
 
-// Fill the trace of the stripes of warp w.  slot: 3 R x 32 floats of shared
-// memory of this warp (the moved points of its next stripe).  Called by whole
-// warps; with W > 1 by all W warps of the alignment, prog[] zeroed before.
-template <int SMODE, bool GAP, int R>
-__device__ __noinline__ void nw_fill(const FillArgs &A, const FillGeom G, int w, float *slot) {
+// Row i of the matrix: the moved pred point, FP64, rounded once.
+IA_DEV float3 moved_row(const FillArgs &A, int i, bool raw) {
+    const double *p = A.P + 3 * (size_t)i;
+    double x, y, z;
+    xform(A.rt, A.rt + 9, p[0], p[1], p[2], x, y, z);
+    float3 m = make_float3((float)x, (float)y, (float)z);
+    if (!raw && !(isfinite(m.x) && isfinite(m.y) && isfinite(m.z))) m.x = m.y = m.z = -1e30f;
+    return m;
+}
+
+// Fill the trace of the stripes of warp w.  Called by whole warps; with W > 1
+// by all W warps of the alignment, prog[] zeroed before.
+template <int SMODE, int R>
+__device__ __noinline__ void nw_fill(const FillArgs &A, const FillGeom G, int w) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int plen = A.plen, nlen = A.nlen, W = G.W, P2 = G.P2, S = G.S;
+    const int plen = A.plen, nlen = A.nlen, W = G.W, S = G.S;
     const int np = (nlen + 1) >> 1;
-    const int nq = S > w ? (S - w + W - 1) / W : 0;  // stripes of this warp
-    if (nq == 0) return;
-    const int k_last = w + (nq - 1) * W;
-    const int last_lane = k_last == S - 1 ? (plen - 1 - k_last * 32 * R) / R : 31;
-    const int total = (nq - 1) * P2 + last_lane + np;
     const float gap = A.gap, inv = A.inv_d0sq, cut2 = A.cut2;
-    const float2 ninv = make_float2(-inv, -inv), none = make_float2(-1.f, -1.f);
-    const float4 *qa = A.qa;
-    const float2 *qb = A.qb;
-    float2 mx[R], my[R], mz[R];
-    uint8_t lp[R];
-    float h[R], hp[R];
-    uint32_t ta[R], tb[R];
+    const float2 ninv = make_float2(-inv, -inv);
+    for (int k = w; k < S; k += W) {
+        const int row0 = (k * 32 + lane) * R;
+        const bool ok = row0 < plen;  // the lane has a row of the matrix
+        float2 mx[R], my[R], mz[R];
+        uint8_t lp[R];
+        float h[R], hp[R];
+        uint32_t ta[R], tb[R];
 #pragma unroll
-    for (int r = 0; r < R; r++) {
-        mx[r] = my[r] = mz[r] = make_float2(0.f, 0.f);
-        h[r] = hp[r] = 0.f;
-        ta[r] = tb[r] = 0u;
-        lp[r] = 0;
-    }
-    float upprev = 0.f, hb0 = 0.f, hb1 = 0.f, pb0 = 0.f, pb1 = 0.f;
-    float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);  // lane 0: the boundary values of its next pair
-    int s = P2 - lane, q = -1;                    // column pair, stripe of this lane
-    bool ok = false;                              // the lane has a row of the matrix
-    int wlim = 0, rlim = 0;                       // pairs whose boundary this lane writes / reads
-    uint32_t *wp = A.trace;
-    int tq = 0, qn = 0;  // step at which lane 0 enters its next stripe, and that stripe
-    for (int t0 = 0; t0 < total; t0 += 16) {
-        if (tq < t0 + 16 && qn < nq) {
-            // moved points of the stripe entered next (FP64 transform, rounded
-            // once), for all lanes together; the last reader of the slot's old
-            // content entered at tq - P2 + 31 < t0 (fill_min_period)
-            double Rm[9], tm[3];
-#pragma unroll
-            for (int a = 0; a < 9; a++) Rm[a] = A.rt[a];
-#pragma unroll
-            for (int a = 0; a < 3; a++) tm[a] = A.rt[9 + a];
-            const int row0 = ((w + qn * W) * 32 + lane) * R;
+        for (int r = 0; r < R; r++) {
+            const int i = min(row0 + r, plen - 1);
             if (SMODE != SMAT_SS2) {
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    const double *p = A.P + 3 * (size_t)min(row0 + r, plen - 1);
-                    double ax, ay, az;
-                    xform(Rm, tm, p[0], p[1], p[2], ax, ay, az);
-                    slot[(3 * r) * 32 + lane] = (float)ax;
-                    slot[(3 * r + 1) * 32 + lane] = (float)ay;
-                    slot[(3 * r + 2) * 32 + lane] = (float)az;
-                }
+                const float3 m = moved_row(A, i, SMODE == SMAT_SS4);
+                mx[r] = make_float2(m.x, m.x);
+                my[r] = make_float2(m.y, m.y);
+                mz[r] = make_float2(m.z, m.z);
+            } else {
+                mx[r] = my[r] = mz[r] = make_float2(0.f, 0.f);
             }
-            tq += P2;
-            qn++;
+            lp[r] = SMODE == SMAT_SS2 || SMODE == SMAT_SS4 ? A.Lp[i] : (uint8_t)0;
+            h[r] = hp[r] = 0.f;
+            ta[r] = tb[r] = 0u;
         }
-        if (W > 1) {
-            // the boundary pairs that lane 0 reads in this group (one ahead)
-            int ql = t0 / P2, sl = t0 - ql * P2 + 16;
-            if (sl >= P2) {
-                ql++;
-                sl -= P2;
-            }
-            if (ql >= nq) {
-                ql = nq - 1;
-                sl = np;
-            }
-            const int qp = w > 0 ? ql : ql - 1, wprod = w > 0 ? w - 1 : W - 1;
-            if (qp >= 0) {
-                const int need = qp * P2 + 32 + min(sl, np - 1);
+        float upprev = 0.f, hb0 = 0.f, hb1 = 0.f, pb0 = 0.f, pb1 = 0.f;
+        // lane 0 reads the boundary row of the stripe above, one pair ahead;
+        // lane 31 writes this stripe's
+        const bool rd = lane == 0 && k > 0, wr = lane == 31 && k + 1 < S;
+        const float *qp = A.q - 6 * lane, *rp = A.br;
+        float *wp = A.bw - 4 * 31;
+        uint32_t *tp = A.trace + ((size_t)k * G.G * 32 + lane) * (2 * R);
+        const int steps = np + (k == S - 1 ? (plen - 1 - k * 32 * R) / R : 31);
+        const int qw = k / W, span = np + 64;  // progress: stripes of a warp, pairs
+        float4 bn = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t0 = 0; t0 < steps; t0 += 16) {
+            if (W > 1 && k > 0) {
+                // pairs that lane 0 reads in this group (one ahead), written by
+                // the warp of stripe k - 1
+                const int need = (w > 0 ? qw : qw - 1) * span + min(t0 + 17, np);
+                const int wprod = w > 0 ? w - 1 : W - 1;
                 uint32_t it = 0;
                 while (A.prog[wprod] < need && ++it < kFillWaitLimit) {
                 }
                 if (it >= kFillWaitLimit && lane == 0) atomicOr(A.err, DERR_NW_TIMEOUT);
                 __threadfence_block();
             }
+            __syncwarp();
+            if (t0 == 0 && rd) bn = *reinterpret_cast<const float4 *>(rp);
+            const int n16 = min(16, steps - t0);
+#pragma unroll 1
+            for (int u = n16; u > 0; u--) {
+                float up0 = __shfl_up_sync(kFull, hb0, 1), up1 = __shfl_up_sync(kFull, hb1, 1);
+                float pu0 = __shfl_up_sync(kFull, pb0, 1), pu1 = __shfl_up_sync(kFull, pb1, 1);
+                if (lane == 0) {
+                    up0 = bn.x;
+                    up1 = bn.z;
+                    pu0 = bn.y;
+                    pu1 = bn.w;
+                }
+                rp += 4;
+                if (rd) bn = *reinterpret_cast<const float4 *>(rp);
+                float2 qx, qy, qz;
+                uint8_t ln0 = 0, ln1 = 0;
+                bool left_of = false;
+                if (SMODE != SMAT_SS2) {
+                    qx = reinterpret_cast<const float2 *>(qp)[0];
+                    qy = reinterpret_cast<const float2 *>(qp)[1];
+                    qz = reinterpret_cast<const float2 *>(qp)[2];
+                }
+                if (SMODE == SMAT_SS2 || SMODE == SMAT_SS4) {
+                    const int s = t0 + n16 - u - lane;
+                    left_of = s < 0;
+                    ln0 = A.Ln[min(max(2 * s, 0), nlen - 1)];
+                    ln1 = A.Ln[min(max(2 * s + 1, 0), nlen - 1)];
+                }
+                qp += 6;
+                float2 e[R];
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    e[r] = score_pair<SMODE>(mx[r], my[r], mz[r], qx, qy, qz, ninv, inv, cut2, lp[r], ln0, ln1, left_of);
+                float n0[R], p0[R];
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    fill_cell<SMODE>(r == 0 ? upprev : h[r > 0 ? r - 1 : 0], e[r].x, r == 0 ? pu0 : p0[r > 0 ? r - 1 : 0],
+                                     hp[r], gap, n0[r], p0[r], ta[r], tb[r]);
+#pragma unroll
+                for (int r = 0; r < R; r++)
+                    fill_cell<SMODE>(r == 0 ? up0 : n0[r > 0 ? r - 1 : 0], e[r].y, r == 0 ? pu1 : hp[r > 0 ? r - 1 : 0],
+                                     p0[r], gap, h[r], hp[r], ta[r], tb[r]);
+                upprev = up1;
+                hb0 = n0[R - 1];
+                hb1 = h[R - 1];
+                pb0 = p0[R - 1];
+                pb1 = hp[R - 1];
+                if (wr) *reinterpret_cast<float4 *>(wp) = make_float4(hb0, pb0, hb1, pb1);
+                wp += 4;
+            }
+            if (ok) store_words<R>(tp, ta, tb, 2 * (16 - n16));
+            tp += 64 * R;
+#pragma unroll
+            for (int r = 0; r < R; r++) ta[r] = tb[r] = 0u;
+            if (W > 1) {
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) A.prog[w] = qw * span + max(t0 + n16 - 31, 0);
+            }
         }
         __syncwarp();
-        const int n16 = min(16, total - t0);
-#pragma unroll 1
-        for (int u = 0; u < n16; u++) {
-            float up0 = __shfl_up_sync(kFull, hb0, 1), up1 = __shfl_up_sync(kFull, hb1, 1);
-            float pu0 = up0, pu1 = up1;
-            if (GAP) {
-                pu0 = __shfl_up_sync(kFull, pb0, 1);
-                pu1 = __shfl_up_sync(kFull, pb1, 1);
-            }
-            if (s == P2) {  // enter the next stripe (once per P2 steps)
-                if (ok && u > 0) store_words<R>(wp, ta, tb, 2 * (16 - u));
-                s = 0;
-                q++;
-                const int k = w + q * W, row0 = (k * 32 + lane) * R;
-                ok = q < nq && row0 < plen;
-                upprev = 0.f;
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    h[r] = hp[r] = 0.f;
-                    ta[r] = tb[r] = 0u;
-                    const float a = slot[(3 * r) * 32 + lane], b = slot[(3 * r + 1) * 32 + lane],
-                                c = slot[(3 * r + 2) * 32 + lane];
-                    mx[r] = make_float2(a, a);
-                    my[r] = make_float2(b, b);
-                    mz[r] = make_float2(c, c);
-                    if (SMODE == SMAT_SS2 || SMODE == SMAT_SS4) lp[r] = A.Lp[min(row0 + r, plen - 1)];
-                }
-                wp = A.trace + ((size_t)(k * G.G + ((t0 + u) >> 4) - ((q * P2) >> 4)) * 32 + lane) * (2 * R);
-                wlim = lane == 31 && ok && k + 1 < S ? np : 0;
-                rlim = lane == 0 && ok && k > 0 ? np : 0;
-                bn = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (rlim > 0) {
-                    if (GAP) bn = *reinterpret_cast<const float4 *>(A.br);
-                    else {
-                        const float2 v = *reinterpret_cast<const float2 *>(A.br);
-                        bn.x = v.x;
-                        bn.z = v.y;
-                    }
-                }
-            }
-            if (lane == 0) {
-                up0 = bn.x;
-                up1 = bn.z;
-                pu0 = GAP ? bn.y : bn.x;
-                pu1 = GAP ? bn.w : bn.z;
-            }
-            if ((unsigned)(s + 1) < (unsigned)rlim) {  // lane 0: prefetch
-                if (GAP) bn = reinterpret_cast<const float4 *>(A.br)[s + 1];
-                else {
-                    const float2 v = reinterpret_cast<const float2 *>(A.br)[s + 1];
-                    bn.x = v.x;
-                    bn.z = v.y;
-                }
-            }
-            // column pair; a pair outside the matrix is computed on the last
-            // one and never read by a cell inside it
-            const int sc = (int)min((unsigned)s, (unsigned)(np - 1));
-            float4 va = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 vb = make_float2(0.f, 0.f);
-            uint8_t ln0 = 0, ln1 = 0;
-            if (SMODE != SMAT_SS2) {
-                if (qa) {
-                    va = qa[sc];
-                    vb = qb[sc];
-                } else {
-                    const double *q0 = A.Q + 6 * (size_t)sc, *q1 = 2 * sc + 1 < nlen ? q0 + 3 : q0;
-                    va = make_float4(-(float)q0[0], -(float)q1[0], -(float)q0[1], -(float)q1[1]);
-                    vb = make_float2(-(float)q0[2], -(float)q1[2]);
-                }
-            }
-            if (SMODE == SMAT_SS2 || SMODE == SMAT_SS4) {
-                ln0 = A.Ln[2 * sc];
-                ln1 = A.Ln[min(2 * sc + 1, nlen - 1)];
-            }
-            float2 e[R];
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                e[r] = score_pair<SMODE>(mx[r], my[r], mz[r], va, vb, ninv, none, inv, cut2, lp[r], ln0, ln1);
-            float n0[R], p0[R];
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                fill_cell<SMODE, GAP>(r == 0 ? upprev : h[r > 0 ? r - 1 : 0], e[r].x, r == 0 ? pu0 : p0[r > 0 ? r - 1 : 0],
-                                      hp[r], gap, n0[r], p0[r], ta[r], tb[r]);
-#pragma unroll
-            for (int r = 0; r < R; r++)
-                fill_cell<SMODE, GAP>(r == 0 ? up0 : n0[r > 0 ? r - 1 : 0], e[r].y, r == 0 ? pu1 : hp[r > 0 ? r - 1 : 0],
-                                      p0[r], gap, h[r], hp[r], ta[r], tb[r]);
-            upprev = up1;
-            hb0 = n0[R - 1];
-            hb1 = h[R - 1];
-            pb0 = p0[R - 1];
-            pb1 = hp[R - 1];
-            if ((unsigned)s < (unsigned)wlim) {  // lane 31: the stripe's last row
-                if (GAP) reinterpret_cast<float4 *>(A.bw)[s] = make_float4(hb0, pb0, hb1, pb1);
-                else reinterpret_cast<float2 *>(A.bw)[s] = make_float2(hb0, hb1);
-            }
-            s++;
-        }
-        if (ok) store_words<R>(wp, ta, tb, 2 * (16 - n16));
-        wp += 64 * R;
-#pragma unroll
-        for (int r = 0; r < R; r++) ta[r] = tb[r] = 0u;
-        if (W > 1) {
-            __threadfence_block();
-            __syncwarp();
-            if (lane == 0) A.prog[w] = t0 + n16;
-        }
     }
-    __syncwarp();
 }
 
-template <int SMODE, bool GAP>
-IA_DEV void nw_fill_r(const FillArgs &A, const FillGeom &G, int w, float *slot) {
-    if (G.R == 4) nw_fill<SMODE, GAP, 4>(A, G, w, slot);
-    else if (G.R == 3) nw_fill<SMODE, GAP, 3>(A, G, w, slot);
-    else if (G.R == 2) nw_fill<SMODE, GAP, 2>(A, G, w, slot);
-    else nw_fill<SMODE, GAP, 1>(A, G, w, slot);
+// One code for every gap penalty: without one, hp = H + 0.  A version without
+// the hp values has fewer instructions, but half of a launch's chains run it
+// beside the other half's, and the two loops together cost more in instruction
+// fetch than they save (k_chain of 64 pairs of L 40-300: 74.0 ms against 60.3).
+template <int SMODE>
+IA_DEV void nw_fill_r(const FillArgs &A, const FillGeom &G, int w) {
+    if (G.R == 4) nw_fill<SMODE, 4>(A, G, w);
+    else if (G.R == 3) nw_fill<SMODE, 3>(A, G, w);
+    else nw_fill<SMODE, 2>(A, G, w);
 }
 
 // The path from (plen, nlen) by the trace's bits (indialign_c/nw.h:42-68);
@@ -334,7 +313,7 @@ IA_DEV void nw_fill_r(const FillArgs &A, const FillGeom &G, int w, float *slot) 
 // ballot along the column.
 __device__ __noinline__ inline int nw_traceback(const uint32_t *trace, const FillGeom G, int plen, int nlen, uint32_t *al) {
     constexpr unsigned kFull = 0xffffffffu;
-    const int lane = threadIdx.x & 31, R = G.R, W = G.W;
+    const int lane = threadIdx.x & 31, R = G.R;
     int i = plen, j = nlen, cnt = 0;
     while (i > 0 && j > 0) {
         const int r = i - lane;  // this lane's row (1-based)
@@ -342,13 +321,13 @@ __device__ __noinline__ inline int nw_traceback(const uint32_t *trace, const Fil
         int c = 0;  // position of column jj in the plane words: c - jj
         if (r >= 1) {
             const int k = (r - 1) / (32 * R), ri = (r - 1) - k * 32 * R, l = ri / R, rr = ri - l * R;
-            const int base = (k / W) * G.P2, first = (base + l) >> 4, word = (base + l + ((j - 1) >> 1)) >> 4;
-            const uint32_t *p = trace + ((size_t)(k * G.G + word - (base >> 4)) * 32 + l) * (2 * R) + 2 * rr;
+            const int word = (l + ((j - 1) >> 1)) >> 4;
+            const uint32_t *p = trace + ((size_t)(k * G.G + word) * 32 + l) * (2 * R) + 2 * rr;
             uint2 lo = *reinterpret_cast<const uint2 *>(p), hi = make_uint2(0u, 0u);
-            if (word > first) hi = *reinterpret_cast<const uint2 *>(p - 64 * R);
+            if (word > 0) hi = *reinterpret_cast<const uint2 *>(p - 64 * R);
             pa = ((unsigned long long)hi.x << 32) | lo.x;
             pb = ((unsigned long long)hi.y << 32) | lo.y;
-            c = 32 * word + 32 - 2 * (base + l);
+            c = 32 * word + 32 - 2 * l;
         }
         int q = 0;  // lane of row i
         for (;;) {
@@ -371,8 +350,8 @@ __device__ __noinline__ inline int nw_traceback(const uint32_t *trace, const Fil
             }
             code = __shfl_sync(kFull, code, q);
             if (code == 0) break;
-            if (code > 0) {
-                j -= code;
+            if (code > 0) {  // (the bits left of the matrix are arbitrary)
+                j = max(j - code, 0);
             } else {
                 const int pu = c - j;
                 const bool up = lane >= q && r >= 1 && pu < 64 && ((pa & pb) >> pu & 1ull);

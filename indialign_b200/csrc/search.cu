@@ -100,7 +100,7 @@ struct Ctx {
     DBuf<long long> lay_l;
     DBuf<unsigned long long> ctr;
     // learned window ranker
-    DBuf<float> gbh;  // NW boundary rows
+    DBuf<float> gbh, gcol;  // NW boundary rows, staged columns
     DBuf<float> blob, wscore, wfeat, wlabel;
     DBuf<MlpPacked> mlp;
     DBuf<int> wcount, wlist, wsel;
@@ -469,7 +469,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
         if (I.nlen > nmax) nmax = I.nlen;
     }
     chain_flags_ = 0;
-    if ((size_t)nmax * 13 + pmax + 256 <= 96 * 1024) chain_flags_ |= 1;
+    if ((size_t)nmax * 13 + pmax + 2048 <= 96 * 1024) chain_flags_ |= 1;
     if (nmax <= 512) chain_flags_ |= 2;
     if ((pmax < nmax ? pmax : nmax) <= 2048) chain_flags_ |= 4;
     size_t smem = chain_smem_bytes(pmax, nmax, chain_flags_);
@@ -501,6 +501,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     size_t nw = (size_t)chain_grid_ * kChainWarps;
     CK(c_->gtrace.ensure((chain_flags_ & 8) ? 1 : nw * trace_words_));
     CK(c_->gbh.ensure((chain_flags_ & 2) ? 1 : nw * fill_boundary_floats(nmax)));
+    CK(c_->gcol.ensure((chain_flags_ & 1) ? 1 : (size_t)chain_grid_ * fill_column_floats(nmax)));
     CK(c_->gal.ensure((chain_flags_ & 4) ? 1 : nw * (pmax < nmax ? pmax : nmax)));
     CK(c_->alP.ensure(3 * 2 * (size_t)(c_->h_off.empty() ? 1 : c_->h_off.back() + 2)));
     CK(c_->alQ.ensure(3 * 2 * (size_t)(c_->h_off.empty() ? 1 : c_->h_off.back() + 2)));
@@ -596,8 +597,8 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
         cudaEventRecord(e0, c_->stream);
     }
     const bool emit = kind == CH_SS2 || kind == CH_SS4 || kind == CH_DP_EMIT;
-    const ChainScratch sc = {c_->gtrace.p, trace_words_, c_->gbh.p, c_->gal.p,        pmax,
-                             nmax,         chain_flags_, cfg_.chain_chunk, chain_grid_};
+    const ChainScratch sc = {c_->gtrace.p, trace_words_, c_->gbh.p,    c_->gcol.p,       c_->gal.p,
+                             pmax,         nmax,         chain_flags_, cfg_.chain_chunk, chain_grid_};
     launch_chain(b, c_->ctasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, sc, chain_grid_, emit,
                  c_->stream);
     if (timing) {

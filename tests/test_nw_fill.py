@@ -2,11 +2,10 @@
 wavefront of R rows x 2 columns per lane and step, the trace words, the
 boundary rows between stripes, and W warps sharing one alignment.
 
-Checked: every store lies inside the trace block that the host sizes
-(fill_trace_words); every boundary pair is read after it was written, across a
-16-step group boundary; the warps never wait for one another in a circle; and
-the directions and the path read back from the words are those of a row-by-row
-fill of the same matrix."""
+Checked: every access lies inside the trace block, the staged columns and the
+boundary rows that the host sizes; boundary pairs are read after they were
+written; the warps never wait for one another in a circle; and the directions
+read back from the words are those of a row-by-row fill of the same matrix."""
 from __future__ import annotations
 
 import ctypes
@@ -14,154 +13,115 @@ import ctypes
 import numpy as np
 import pytest
 
-LAG = 49
-
-
-def min_period(W):
-    return 32 * W + 32 if W > 1 else 50
+LAG, PAD = 49, 33
 
 
 def geom(plen, nlen, W, R=None):
     """fill_geom; with R given, that choice of rows per lane."""
     n32, np_ = (plen + 31) >> 5, (nlen + 1) >> 1
     best = None
-    for r in (4, 3, 2, 1) if R is None else (R,):
+    for r in (4, 3, 2) if R is None else (R,):
         S = (n32 + r - 1) // r
-        rounds = (S + W - 1) // W
-        P2 = min_period(W) if rounds > 1 and np_ < min_period(W) else np_
-        cost = (rounds * P2 + (min(S, W) - 1) * LAG + 31) * (25 + 34 * r)
+        cost = ((S + W - 1) // W * (np_ + 31) + (min(S, W) - 1) * LAG) * (20 + 32 * r)
         if best is None or cost < best[0]:
-            best = (cost, r, S, P2)
-    _, r, S, P2 = best
-    return {"R": r, "S": S, "W": W, "P2": P2, "G": (P2 + 45) // 16 + 1}
+            best = (cost, r, S)
+    return {"R": best[1], "S": best[2], "W": W, "G": (np_ + 46) // 16}
 
 
 def trace_words(np_, nn):
-    P2 = max((nn + 1) // 2, min_period(4))
-    return ((np_ + 31) // 32 + 3) * 64 * ((P2 + 45) // 16 + 1)
+    return ((np_ + 31) // 32 + 3) * 64 * (((nn + 1) // 2 + 46) // 16)
 
 
 def cell(ds, sc, up, left, gap):
+    """fill_cell; a NaN score (left of the matrix) leaves max(left, up)."""
     diag = ds + sc
     m = max(left, up)
-    h = max(diag, m)
-    hp = (diag + gap if diag >= m else m) if gap else h
-    return h, hp, int(diag < m), int(left < up)
+    isd = diag >= m
+    h = diag if isd else m
+    return h, diag + gap if isd else m, int(not isd), int(left < up)
 
 
 class Warp:
-    """The state of nw_fill for one warp, advanced one 16-step group at a time."""
+    """nw_fill of one warp, as a generator of its 16-step groups."""
 
     def __init__(self, M, gap, g, w, mem, bnd, prog, size):
         self.M, self.gap, self.g, self.w, self.mem, self.bnd, self.prog, self.size = M, gap, g, w, mem, bnd, prog, size
-        plen, nlen = M.shape
-        R, S, W, P2 = g["R"], g["S"], g["W"], g["P2"]
-        self.np = (nlen + 1) >> 1
-        self.nq = (S - w + W - 1) // W if S > w else 0
-        k_last = w + (self.nq - 1) * W
-        last = (plen - 1 - k_last * 32 * R) // R if k_last == S - 1 else 31
-        self.total = (self.nq - 1) * P2 + last + self.np if self.nq else 0
-        self.t0, self.tq, self.qn, self.slot = 0, 0, 0, None
-        z = lambda: [0.0] * R  # noqa: E731
-        self.L = [dict(s=P2 - l, q=-1, ok=False, wlim=0, rlim=0, wp=0, h=z(), hp=z(), ta=[0] * R, tb=[0] * R, upprev=0.0,
-                       hb=(0.0, 0.0), pb=(0.0, 0.0), bn=None, row0=None) for l in range(32)]
+        self.np = (M.shape[1] + 1) >> 1
+        self.todo = [(k, t0) for k in range(w, g["S"], g["W"]) for t0 in range(0, self.steps(k), 16)]
 
-    def done(self):
-        return self.t0 >= self.total
+    def steps(self, k):
+        last = (self.M.shape[0] - 1 - k * 32 * self.g["R"]) // self.g["R"] if k == self.g["S"] - 1 else 31
+        return self.np + last
 
     def ready(self):
-        """The wait at a group's start (W > 1)."""
-        g = self.g
-        if g["W"] == 1:
+        k, t0 = self.todo[0]
+        W, w = self.g["W"], self.w
+        if W == 1 or k == 0:
             return True
-        P2 = g["P2"]
-        ql, sl = self.t0 // P2, self.t0 % P2 + 16
-        if sl >= P2:
-            ql, sl = ql + 1, sl - P2
-        if ql >= self.nq:
-            ql, sl = self.nq - 1, self.np
-        qp, wprod = (ql, self.w - 1) if self.w > 0 else (ql - 1, g["W"] - 1)
-        return qp < 0 or self.prog[wprod] >= qp * P2 + 32 + min(sl, self.np - 1)
+        need = (k // W if w > 0 else k // W - 1) * (self.np + 64) + min(t0 + 17, self.np)
+        return self.prog[w - 1 if w > 0 else W - 1] >= need
 
-    def store(self, c, sh):
-        R = self.g["R"]
-        for r in range(R):
-            for p, word in ((0, c["ta"][r]), (1, c["tb"][r])):
-                a = c["wp"] + 2 * r + p
-                assert 0 <= a < self.size
-                self.mem[a] = (word << sh) & 0xFFFFFFFF
+    def publish(self):
+        k, t0 = self.todo.pop(0)
+        self.prog[self.w] = k // self.g["W"] * (self.np + 64) + max(min(t0 + 16, self.steps(k)) - 31, 0)
 
-    def read_boundary(self, k, s, stamp):
-        (h0, p0, h1, p1), src, wrote = self.bnd[(k - 1) % self.g["W"]][s]
+    def boundary(self, k, s):
+        assert -PAD <= s < self.np + PAD
+        if s >= self.np:
+            return (7.0,) * 4  # never reaches the matrix
+        v, src = self.bnd[(k - 1) % self.g["W"]][s]
         assert src == k - 1, "boundary of another stripe"
-        # same warp: written in an earlier group; another warp: before its published count
-        assert wrote < self.t0 if self.g["W"] == 1 else wrote < self.prog[(k - 1) % self.g["W"]]
-        return h0, p0, h1, p1
+        return v
 
     def group(self):
-        g, M, gap = self.g, self.M, self.gap
+        g, M, gap, w = self.g, self.M, self.gap, self.w
         plen, nlen = M.shape
-        R, S, W, P2, w = g["R"], g["S"], g["W"], g["P2"], self.w
-        t0 = self.t0
-        if self.tq < t0 + 16 and self.qn < self.nq:
-            for c in self.L:  # nobody still has to load the slot's old content
-                assert self.slot is None or c["q"] >= self.slot
-            self.slot = self.qn
-            self.tq += P2
-            self.qn += 1
-        n16 = min(16, self.total - t0)
+        R, S = g["R"], g["S"]
+        k, t0 = self.todo[0]
+        if t0 == 0:
+            z = lambda: [0.0] * R  # noqa: E731
+            self.L = [dict(h=z(), hp=z(), ta=[0] * R, tb=[0] * R, upprev=0.0, hb=(0.0, 0.0), pb=(0.0, 0.0))
+                      for _ in range(32)]
+            self.bn = self.boundary(k, 0) if k > 0 else (0.0,) * 4
+        n16 = min(16, self.steps(k) - t0)
         for u in range(n16):
             old = [(c["hb"], c["pb"]) for c in self.L]
-            writes = []
+            out = None
             for l, c in enumerate(self.L):
                 (up0, up1), (pu0, pu1) = old[max(l - 1, 0)]
-                if c["s"] == P2:
-                    if c["ok"] and u > 0:
-                        self.store(c, 2 * (16 - u))
-                    c["s"], c["q"] = 0, c["q"] + 1
-                    k = w + c["q"] * W
-                    c["row0"] = (k * 32 + l) * R
-                    c["ok"] = c["q"] < self.nq and c["row0"] < plen
-                    if c["ok"]:
-                        assert self.slot == c["q"]
-                    c["h"], c["hp"], c["ta"], c["tb"], c["upprev"] = [0.0] * R, [0.0] * R, [0] * R, [0] * R, 0.0
-                    c["wp"] = ((k * g["G"] + ((t0 + u) >> 4) - ((c["q"] * P2) >> 4)) * 32 + l) * 2 * R
-                    c["wlim"] = self.np if l == 31 and c["ok"] and k + 1 < S else 0
-                    c["rlim"] = self.np if l == 0 and c["ok"] and k > 0 else 0
-                    c["bn"] = self.read_boundary(k, 0, t0 + u) if c["rlim"] else (0.0,) * 4
                 if l == 0:
-                    up0, pu0, up1, pu1 = c["bn"]
-                s = c["s"]
-                if 0 <= s + 1 < c["rlim"]:
-                    c["bn"] = self.read_boundary(w + c["q"] * W, s + 1, t0 + u)
-                sc = s if 0 <= s < self.np else self.np - 1
-                rows = [min((c["row0"] or 0) + r, plen - 1) for r in range(R)]
-                c0, c1 = 2 * sc, min(2 * sc + 1, nlen - 1)
-                n0, p0 = [0.0] * R, [0.0] * R
-                hold = list(c["h"])
-                for r in range(R):
-                    n0[r], p0[r], a, b = cell(c["upprev"] if r == 0 else hold[r - 1], M[rows[r], c0],
-                                              pu0 if r == 0 else p0[r - 1], c["hp"][r], gap)
-                    c["ta"][r], c["tb"][r] = (c["ta"][r] << 1 | a) & 0xFFFFFFFF, (c["tb"][r] << 1 | b) & 0xFFFFFFFF
-                nh, nhp = [0.0] * R, [0.0] * R
-                for r in range(R):
-                    nh[r], nhp[r], a, b = cell(up0 if r == 0 else n0[r - 1], M[rows[r], c1],
-                                               pu1 if r == 0 else nhp[r - 1], p0[r], gap)
-                    c["ta"][r], c["tb"][r] = (c["ta"][r] << 1 | a) & 0xFFFFFFFF, (c["tb"][r] << 1 | b) & 0xFFFFFFFF
+                    up0, pu0, up1, pu1 = self.bn
+                s = t0 + u - l
+                assert -PAD <= s < self.np + PAD
+                row0 = (k * 32 + l) * R
+                c0, c1 = min(2 * s, nlen - 1), min(2 * s + 1, nlen - 1)
+                e = [(M[min(row0 + r, plen - 1), c0], M[min(row0 + r, plen - 1), c1]) if s >= 0 else (np.nan, np.nan)
+                     for r in range(R)]
+                n0, p0, nh, nhp = [0.0] * R, [0.0] * R, [0.0] * R, [0.0] * R
+                for col, (h, hp) in enumerate(((n0, p0), (nh, nhp))):
+                    for r in range(R):
+                        ds = (c["upprev"], up0)[col] if r == 0 else (c["h"], n0)[col][r - 1]
+                        h[r], hp[r], a, b = cell(ds, e[r][col], (pu0, pu1)[col] if r == 0 else hp[r - 1],
+                                                 (c["hp"], p0)[col][r], gap)
+                        c["ta"][r], c["tb"][r] = (c["ta"][r] << 1 | a) & 0xFFFFFFFF, (c["tb"][r] << 1 | b) & 0xFFFFFFFF
                 c["h"], c["hp"], c["upprev"] = nh, nhp, up1
                 c["hb"], c["pb"] = (n0[R - 1], nh[R - 1]), (p0[R - 1], nhp[R - 1])
-                if 0 <= s < c["wlim"]:
-                    writes.append((s, (n0[R - 1], p0[R - 1], nh[R - 1], nhp[R - 1]), w + c["q"] * W))
-                c["s"] += 1
-            for s, v, k in writes:
-                self.bnd[w][s] = (v, k, t0 + u)
-        for c in self.L:
-            if c["ok"]:
-                self.store(c, 2 * (16 - n16))
-            c["wp"] += 64 * R
+                if l == 31 and k + 1 < S:
+                    assert s < self.np + PAD
+                    out = (s, (n0[R - 1], p0[R - 1], nh[R - 1], nhp[R - 1]))
+            if k > 0:
+                self.bn = self.boundary(k, t0 + u + 1)
+            if out:
+                self.bnd[w][out[0]] = (out[1], k)
+        for l, c in enumerate(self.L):
+            if (k * 32 + l) * R < plen:
+                at = ((k * g["G"] + t0 // 16) * 32 + l) * 2 * R
+                for r in range(R):
+                    for p, word in ((0, c["ta"][r]), (1, c["tb"][r])):
+                        assert 0 <= at + 2 * r + p < self.size
+                        self.mem[at + 2 * r + p] = (word << 2 * (16 - n16)) & 0xFFFFFFFF
             c["ta"], c["tb"] = [0] * R, [0] * R
-        self.t0 += n16
-        self.prog[w] = self.t0
+        self.publish()
 
 
 def fill(M, gap, g):
@@ -169,10 +129,10 @@ def fill(M, gap, g):
     size = trace_words(*M.shape)
     mem, bnd, prog = {}, [{} for _ in range(g["W"])], [0] * g["W"]
     warps = [Warp(M, gap, g, w, mem, bnd, prog, size) for w in range(g["W"])]
-    while not all(x.done() for x in warps):
+    while any(x.todo for x in warps):
         moved = False
         for x in reversed(warps):
-            if not x.done() and x.ready():
+            if x.todo and x.ready():
                 x.group()
                 moved = True
         assert moved, "the warps wait for one another"
@@ -180,12 +140,12 @@ def fill(M, gap, g):
 
 
 def direction(mem, g, i, j):
-    R, W = g["R"], g["W"]
+    R = g["R"]
     k, ri = (i - 1) // (32 * R), (i - 1) % (32 * R)
-    l, rr, base = ri // R, ri % R, (k // W) * g["P2"]
-    word = (base + l + ((j - 1) >> 1)) >> 4
-    a = ((k * g["G"] + word - (base >> 4)) * 32 + l) * 2 * R + 2 * rr
-    pos = 32 * word + 32 - 2 * (base + l) - j
+    l, rr = ri // R, ri % R
+    word = (l + ((j - 1) >> 1)) >> 4
+    a = ((k * g["G"] + word) * 32 + l) * 2 * R + 2 * rr
+    pos = 32 * word + 32 - 2 * l - j
     if not (mem[a] >> pos) & 1:
         return 0
     return 1 if (mem[a + 1] >> pos) & 1 else 2  # up : left
@@ -202,9 +162,9 @@ def direct(M, gap):
     return out
 
 
-SIZES = [(3, 3, 1, None, 0.0), (3, 3, 4, None, -0.6), (7, 41, 1, None, -0.6), (33, 31, 1, 1, 0.0), (64, 64, 1, 2, -0.6),
-         (97, 20, 1, 3, 0.0), (129, 64, 1, 4, -0.6), (130, 101, 1, 2, -0.6), (100, 130, 1, 1, 0.0),
-         (65, 66, 4, 1, -0.6), (150, 40, 4, 1, 0.0), (200, 90, 4, 1, -0.6), (260, 50, 4, 2, 0.0), (300, 35, 4, 1, -1.0)]
+SIZES = [(3, 3, 1, None, 0.0), (3, 3, 4, None, -0.6), (7, 41, 1, None, -0.6), (33, 31, 1, 2, 0.0), (64, 64, 1, 2, -0.6),
+         (97, 20, 1, 3, 0.0), (129, 64, 1, 4, -0.6), (130, 101, 1, 2, -0.6), (100, 130, 1, 3, 0.0),
+         (65, 66, 4, 2, -0.6), (330, 40, 4, 2, 0.0), (200, 90, 4, 2, -0.6), (520, 50, 4, 3, 0.0), (300, 35, 4, 2, -1.0)]
 
 
 @pytest.mark.parametrize("plen,nlen,W,R,gap", SIZES)
@@ -218,18 +178,17 @@ def test_fill_equals_a_row_by_row_fill(plen, nlen, W, R, gap):
 def test_warps_never_wait_in_a_circle():
     """Every shape of the shared fill, by its step counts alone."""
     for plen in (1, 65, 129, 300, 513, 700, 1100, 2100):
-        for nlen in (1, 2, 30, 31, 64, 99, 160, 161, 319, 320, 321, 640, 1001):
-            for R in (1, 2, 3, 4):
+        for nlen in (1, 2, 30, 31, 64, 99, 160, 161, 319, 321, 640, 1001):
+            for R in (2, 3, 4):
                 g = geom(plen, nlen, 4, R)
-                M = np.broadcast_to(0.0, (plen, nlen))
                 prog = [0] * 4
-                warps = [Warp(M, 0.0, g, w, {}, [], prog, 0) for w in range(4)]
-                while not all(x.done() for x in warps):
+                warps = [Warp(np.broadcast_to(0.0, (plen, nlen)), 0.0, g, w, {}, [], prog, 0) for w in range(4)]
+                while any(x.todo for x in warps):
                     moved = False
                     for x in warps:
-                        while not x.done() and x.ready():
-                            x.t0 += min(16, x.total - x.t0)
-                            prog[x.w], moved = x.t0, True
+                        while x.todo and x.ready():
+                            x.publish()
+                            moved = True
                     assert moved, (plen, nlen, R)
                 assert g["S"] * g["R"] * 64 * g["G"] <= trace_words(plen, nlen)
 
