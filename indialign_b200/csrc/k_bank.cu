@@ -20,6 +20,16 @@
 // FP64 TM-score of the returned (R, t).  The oracle rebuilt with this
 // arithmetic in its seed banks stayed within 2e-8 of the reference build's
 // final TM-scores on 560 pairs.
+//
+// k_bank is bound by the FMA pipe (62 % busy on the main bank of 61 pairs, the
+// rest is the chunk barrier and the launch's tail): a residue visit is 15
+// operations of distance, paired over two residues, and 15 of sums.  The sums
+// sit under one predicate per residue without a branch and the sweep is
+// unrolled four times, so that distances of later residues fill the sums'
+// latency: 167 -> 136 ms over the bank launches of a learned search of 1024
+// pairs of L 40-1000 (a branch around the sums 152, unrolled twice 150; eight
+// times gained 1.5 % more in a third more code; skipping a pair no lane wants
+// by a vote 131, but 10 % slower on single pairs).
 #include "dmath.cuh"
 #include "stage.cuh"
 #include "pipeline.h"
@@ -57,6 +67,22 @@ struct MomentsF {
         h[3] = fmaf(py, qx, h[3]); h[4] = fmaf(py, qy, h[4]); h[5] = fmaf(py, qz, h[5]);
         h[6] = fmaf(pz, qx, h[6]); h[7] = fmaf(pz, qy, h[7]); h[8] = fmaf(pz, qz, h[8]);
         w++;
+    }
+    // add() if d2 <= lim, every instruction under the one predicate: no branch
+    // around the sums, so the next residues' distances overlap them
+    IA_DEV void add_if(float d2, float lim, float px, float py, float pz, float qx, float qy, float qz) {
+        asm("{\n\t.reg .pred p;\n\t"
+            "setp.le.f32 p, %16, %17;\n\t"
+            "@p add.rn.f32 %0, %0, %18;\n\t@p add.rn.f32 %1, %1, %19;\n\t@p add.rn.f32 %2, %2, %20;\n\t"
+            "@p add.rn.f32 %3, %3, %21;\n\t@p add.rn.f32 %4, %4, %22;\n\t@p add.rn.f32 %5, %5, %23;\n\t"
+            "@p fma.rn.f32 %6, %18, %21, %6;\n\t@p fma.rn.f32 %7, %18, %22, %7;\n\t@p fma.rn.f32 %8, %18, %23, %8;\n\t"
+            "@p fma.rn.f32 %9, %19, %21, %9;\n\t@p fma.rn.f32 %10, %19, %22, %10;\n\t"
+            "@p fma.rn.f32 %11, %19, %23, %11;\n\t@p fma.rn.f32 %12, %20, %21, %12;\n\t"
+            "@p fma.rn.f32 %13, %20, %22, %13;\n\t@p fma.rn.f32 %14, %20, %23, %14;\n\t"
+            "@p add.s32 %15, %15, 1;\n\t}"
+            : "+f"(sp[0]), "+f"(sp[1]), "+f"(sp[2]), "+f"(sq[0]), "+f"(sq[1]), "+f"(sq[2]), "+f"(h[0]), "+f"(h[1]),
+              "+f"(h[2]), "+f"(h[3]), "+f"(h[4]), "+f"(h[5]), "+f"(h[6]), "+f"(h[7]), "+f"(h[8]), "+r"(w)
+            : "f"(d2), "f"(lim), "f"(px), "f"(py), "f"(pz), "f"(qx), "f"(qy), "f"(qz));
     }
     // Kabsch in FP64 from these sums (identity below 3 pairs)
     IA_DEV void kabsch(double *R, double *t) const {
@@ -187,14 +213,16 @@ IA_DEV void points_mean(const double *src, int n, double *out, double *red) {
 // points [128r, 128r+128) before any thread writes them; its writes end at
 // byte 16*128(r+1) + 16, below the first byte (24*128(r+1)) that a later
 // round reads; the pairs of n points take 32*ceil(n/2) <= 16n + 16 bytes,
-// inside the 24n + 32 bytes of the staged region.
-IA_DEV void points_to_f32(const double *src, float4 *dst4, int n, const double *off, const uint8_t *V) {
+// inside the 24n + 32 bytes of the staged region.  `out` (native points): a
+// residue outside the mask, and the point after an odd set, become NaN, so
+// that their distance is never within a cutoff.
+IA_DEV void points_to_f32(const double *src, float4 *dst4, int n, const double *off, const uint8_t *V, bool out) {
     float *dst = reinterpret_cast<float *>(dst4);
     for (int base = 0; base < n; base += kBankChunk) {
         const int i = base + (int)threadIdx.x;
-        double x = 0.0, y = 0.0, z = 0.0;
+        double x = out ? NAN : 0.0, y = 0.0, z = 0.0;
         float w = 0.f;
-        if (i < n) {
+        if (i < n && !(out && V != nullptr && V[i] == 0)) {
             x = src[3 * i] - off[0];
             y = src[3 * i + 1] - off[1];
             z = src[3 * i + 2] - off[2];
@@ -212,11 +240,91 @@ IA_DEV void points_to_f32(const double *src, float4 *dst4, int n, const double *
     __syncthreads();
 }
 
+// Each seed's own Kabsch, the start of its items at every cutoff: CTA (task,
+// block of 128 seeds), thread per seed, {R[9], t[3]} in the tasks' centred
+// frame to seed_rt[item_base / kDetC + seed] (a task has at least kDetC items
+// per seed, so the tasks' ranges are disjoint).  Solved here over the seed's
+// own residues, once for all its cutoffs, instead of per (seed, cutoff) item in
+// k_bank with a sweep over the whole set.  The sums run in residue order, so a
+// long window is a serial chain: points staged as FP32 with the mask as a
+// number, {x, y, z, 0 if valid} and {x, y, z, 0 if valid & 1}, keep it free of
+// branches (SMEM; point sets too large for it are read from global memory).
+template <bool SMEM>
+__global__ void __launch_bounds__(kBankChunk) k_bank_seeds(const BankTask *__restrict__ tasks, double *__restrict__ seed_rt) {
+    extern __shared__ __align__(16) char smem[];
+    __shared__ double oP[3], oQ[3], red[6 * (kBankChunk / 32)];
+    const BankTask &T = tasks[blockIdx.x];
+    const int C = T.C > 0 ? T.C : 1, K = T.n_items / C, sk = blockIdx.y * kBankChunk + threadIdx.x, n = T.n;
+    if ((int)(blockIdx.y * kBankChunk) >= K) return;
+    points_mean(T.P, n, oP, red);
+    points_mean(T.Q, n, oQ, red);
+    const uint8_t *V = T.V;
+    float4 *sP = reinterpret_cast<float4 *>(smem), *sQ = sP + n;
+    auto load = [&](int i, float4 &p, float4 &q) {
+        if (SMEM) {
+            p = sP[i];
+            q = sQ[i];
+            return;
+        }
+        p = point<false>(nullptr, T.P, oP, nullptr, i);
+        q = point<false>(nullptr, T.Q, oQ, nullptr, i);
+        const int v = V ? V[i] : 1;
+        p.w = v != 0 ? 0.f : 1.f;
+        q.w = v & 1 ? 0.f : 1.f;
+    };
+    if (SMEM) {
+        for (int i = threadIdx.x; i < n; i += kBankChunk) {
+            const float4 p = point<false>(nullptr, T.P, oP, nullptr, i), q = point<false>(nullptr, T.Q, oQ, nullptr, i);
+            const int v = V ? V[i] : 1;
+            sP[i] = make_float4(p.x, p.y, p.z, v != 0 ? 0.f : 1.f);
+            sQ[i] = make_float4(q.x, q.y, q.z, v & 1 ? 0.f : 1.f);
+        }
+        __syncthreads();
+    }
+    if (sk >= K) return;
+    const int k = T.slist ? T.slist[sk] : sk;
+    MomentsF m;
+    m.clear();
+    int s = 0, len = 0;
+    if (T.mode == SEED_TABLE) {
+        const int2 e = T.table[k];
+        s = e.x;
+        len = e.y;
+    } else {
+        arith_seed(n, T.ms, k, s, len);
+    }
+    float4 p, q;
+    if (s < 0) {  // bitmask seed: its bit and 1 & valid
+        const uint32_t *row = T.bits + (size_t)(-1 - s) * T.words;
+        for (int w = 0; w < T.words; w++)
+            for (uint32_t x = row[w]; x; x &= x - 1) {
+                const int i = w * 32 + __ffs(x) - 1;
+                if (i >= n) break;
+                load(i, p, q);
+                m.add_if(q.w, 0.f, p.x, p.y, p.z, q.x, q.y, q.z);
+            }
+    } else {  // window of the valid residues
+        const int end = min(s + len, n);
+#pragma unroll 4
+        for (int i = s; i < end; i++) {
+            load(i, p, q);
+            m.add_if(p.w, 0.f, p.x, p.y, p.z, q.x, q.y, q.z);
+        }
+    }
+    double R[9], t[3];
+    m.kabsch(R, t);
+    double *o = seed_rt + 12 * ((size_t)(T.item_base / kDetC) + sk);
+#pragma unroll
+    for (int a = 0; a < 9; a++) o[a] = R[a];
+#pragma unroll
+    for (int a = 0; a < 3; a++) o[9 + a] = t[a];
+}
+
 template <bool SMEM>
 __global__ void __launch_bounds__(kBankChunk, IA_BANK_MINB)
 k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
        int ntasks, const ScanOut *__restrict__ scan, int *counter,
-       double *__restrict__ item_res, int *err, int nmax, unsigned long long *ctr) {
+       const double *__restrict__ seed_rt, double *__restrict__ item_res, int *err, int nmax, unsigned long long *ctr) {
     extern __shared__ __align__(16) char smem[];
     __shared__ BankSmem ctl;
     __shared__ uint64_t bar;
@@ -274,8 +382,8 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
                 points_mean(dQ, n, oQ, red);
                 int k = 2;
                 V = T.V ? reinterpret_cast<const uint8_t *>(sV + cp[k++].lead) : nullptr;
-                points_to_f32(dP, reinterpret_cast<float4 *>(sP), n, oP, V);
-                points_to_f32(dQ, reinterpret_cast<float4 *>(sQ), n, oQ, nullptr);
+                points_to_f32(dP, reinterpret_cast<float4 *>(sP), n, oP, V, false);
+                points_to_f32(dQ, reinterpret_cast<float4 *>(sQ), n, oQ, V, true);
                 Pf = reinterpret_cast<const float4 *>(sP);
                 Qf = reinterpret_cast<const float4 *>(sQ);
                 PV = T.PV ? reinterpret_cast<const uint8_t *>(sPV + cp[k++].lead) : nullptr;
@@ -301,7 +409,7 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
         const int pi = gi + lane;  // processing order within the task
         const bool active = pi < ce;
         const int C = T.C > 0 ? T.C : 1;
-        // item (seed k, cutoff ci) and its record slot li = k*C + ci: seed
+        // item (seed sk, cutoff ci) and its record slot li = sk*C + ci: seed
         // major (the slot order), or cutoff major (a warp refines one cutoff
         // over 32 seeds; measured 1.38x faster than seed major on the
         // learned16384 step, because a warp iterates until its slowest item
@@ -319,88 +427,63 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
             }
         }
         const int li = sk * C + ci;
-        const int k = active ? (T.slist ? T.slist[sk] : sk) : 0;
         const double cut = T.cut[ci];
         const float cut2 = (float)(cut * cut);
         double R[9], t[3];
         MomentsF m;
-        m.clear();
         bool skip = false;
-        // ---- initial Kabsch on the seed ----
         if (T.mode == SEED_SHIFT) {
-            const int o = offset_at(T.shift_lo, T.shift_stride, k);
-            for (int i = 0; i < n; i++) {
-                int j = i - o;
-                bool sel = active && j >= 0 && j < n && PV[i] != 0 && NV[j] != 0;
-                if (sel) {
-                    const float4 pp = point<SMEM>(Pf, Pd, oP, V, i), qq = point<SMEM>(Qf, Qd, oQ, nullptr, j);
+            const int o = offset_at(T.shift_lo, T.shift_stride, sk);
+            m.clear();
+            for (int i = max(0, o); i < min(n, n + o); i++) {
+                const int j = i - o;
+                if (active && PV[i] != 0 && NV[j] != 0) {
+                    const float4 pp = point<SMEM>(Pf, Pd, oP, V, i), qq = point<false>(nullptr, T.Q, oQ, nullptr, j);
                     m.add(pp.x, pp.y, pp.z, qq.x, qq.y, qq.z);
                 }
             }
             skip = m.w < T.shift_min;
+            if (active && !skip) m.kabsch(R, t);
+            else set_identity(R, t);
         } else {
-            int s = 0, len = 0, bitrow = -1;
-            if (active) {
-                if (T.mode == SEED_TABLE) {
-                    int2 e = T.table[k];
-                    if (e.x >= 0) { s = e.x; len = e.y; }
-                    else { bitrow = -1 - e.x; s = 0; len = n; }
-                } else {
-                    arith_seed(n, T.ms, k, s, len);
-                }
-            }
-            const uint32_t *brow = bitrow >= 0 ? T.bits + (size_t)bitrow * T.words : nullptr;
-            for (int i = 0; i < n; i++) {
-                uint8_t v = V ? V[i] : (uint8_t)1;
-                bool sel;
-                if (brow) sel = ((brow[i >> 5] >> (i & 31)) & 1u) && (v & 1u);  // 1 & valid
-                else sel = i >= s && i < s + len && v != 0;                    // valid & valid
-                if (active && sel) {
-                    const float4 pp = point<SMEM>(Pf, Pd, oP, V, i), qq = point<SMEM>(Qf, Qd, oQ, nullptr, i);
-                    m.add(pp.x, pp.y, pp.z, qq.x, qq.y, qq.z);
-                }
-            }
+            const double *o = seed_rt + 12 * ((size_t)(T.item_base / kDetC) + sk);
+#pragma unroll
+            for (int a = 0; a < 9; a++) R[a] = o[a];
+#pragma unroll
+            for (int a = 0; a < 3; a++) t[a] = o[9 + a];
         }
-        if (active && !skip) m.kabsch(R, t);
-        else set_identity(R, t);
         // ---- cutoff iterations: select d2 <= cut^2, Kabsch, stop on a
         // repeated count ----
         bool running = active && !skip && T.max_iter > 0;
         int prev = -1, iter = 0;
         while (__any_sync(0xffffffffu, running)) {
-            float Rf[9], tf[3];
-#pragma unroll
-            for (int a = 0; a < 9; a++) Rf[a] = (float)R[a];
-#pragma unroll
-            for (int a = 0; a < 3; a++) tf[a] = (float)t[a];
             m.clear();
-            int cnt = 0;
+            const float lim = running ? cut2 : -1.f;
             if constexpr (SMEM) {
                 // two residues per step: distances by paired instructions,
-                // the accumulate per residue in residue order
+                // the accumulate per residue in residue order (a residue
+                // outside the mask is staged with a NaN native point)
                 XformF2 X;
                 X.set(R, t);
+#pragma unroll 4
                 for (int k2 = 0; k2 < (n + 1) >> 1; k2++) {
                     const float4 PA = Pf[2 * k2], PB = Pf[2 * k2 + 1], QA = Qf[2 * k2], QB = Qf[2 * k2 + 1];
                     const float2 d2 = dist2_pair(PA, PB, QA, QB, X);
-                    if (running && PB.z != 0.f && d2.x <= cut2) {
-                        m.add(PA.x, PA.z, PB.x, QA.x, QA.z, QB.x);
-                        cnt++;
-                    }
-                    if (running && PB.w != 0.f && d2.y <= cut2) {
-                        m.add(PA.y, PA.w, PB.y, QA.y, QA.w, QB.y);
-                        cnt++;
-                    }
+                    m.add_if(d2.x, lim, PA.x, PA.z, PB.x, QA.x, QA.z, QB.x);
+                    m.add_if(d2.y, lim, PA.y, PA.w, PB.y, QA.y, QA.w, QB.y);
                 }
             } else {
+                float Rf[9], tf[3];
+#pragma unroll
+                for (int a = 0; a < 9; a++) Rf[a] = (float)R[a];
+#pragma unroll
+                for (int a = 0; a < 3; a++) tf[a] = (float)t[a];
                 for (int i = 0; i < n; i++) {
                     const float4 pp = point<SMEM>(Pf, Pd, oP, V, i), qq = point<SMEM>(Qf, Qd, oQ, nullptr, i);
-                    if (running && pp.w != 0.f && dist2_f32(pp, qq, Rf, tf) <= cut2) {
-                        m.add(pp.x, pp.y, pp.z, qq.x, qq.y, qq.z);
-                        cnt++;
-                    }
+                    if (pp.w != 0.f && dist2_f32(pp, qq, Rf, tf) <= lim) m.add(pp.x, pp.y, pp.z, qq.x, qq.y, qq.z);
                 }
             }
+            const int cnt = m.w;
             if (running) {
                 if (cnt >= 3) m.kabsch(R, t);
                 ++iter;
@@ -449,8 +532,9 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
             score = (double)sum / fmax(T.lnorm, 1.0);
         }
         {
-            // residue visits: seed pass + `iter` cutoff passes + score pass
-            unsigned long long visits = active && !skip ? (unsigned long long)(iter + 2) * n : 0ull;
+            // residue visits: `iter` cutoff passes + score pass (the seeds'
+            // own windows, in k_bank_seeds or here, are not counted)
+            unsigned long long visits = active && !skip ? (unsigned long long)(iter + 1) * n : 0ull;
             unsigned long long items = active ? 1ull : 0ull;
 #pragma unroll
             for (int o2 = 16; o2 > 0; o2 >>= 1) {
@@ -552,15 +636,21 @@ size_t bank_smem_bytes(int nmax) {
 }
 
 void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks,
-                 const ScanOut *scan, int *counter, double *item_res, int *err,
+                 const ScanOut *scan, int *counter, double *seed_rt, int seed_blocks, double *item_res, int *err,
                  int nmax, int grid, unsigned long long *ctr, cudaStream_t st) {
+    if (seed_blocks > 0) {
+        const size_t ss = (size_t)nmax * 2 * sizeof(float4);
+        const dim3 g(ntasks, seed_blocks);
+        if (ss <= kBankSmemMax) k_bank_seeds<true><<<g, kBankChunk, ss, st>>>(tasks, seed_rt);
+        else k_bank_seeds<false><<<g, kBankChunk, 0, st>>>(tasks, seed_rt);
+    }
     size_t sm = bank_smem_bytes(nmax);
     if (sm <= kBankSmemMax) {
         k_bank<true><<<grid, kBankChunk, sm, st>>>(tasks, chunk_begin, ntasks, scan, counter,
-                                                   item_res, err, nmax, ctr);
+                                                   seed_rt, item_res, err, nmax, ctr);
     } else {
         k_bank<false><<<grid, kBankChunk, 0, st>>>(tasks, chunk_begin, ntasks, scan, counter,
-                                                   item_res, err, nmax, ctr);
+                                                   seed_rt, item_res, err, nmax, ctr);
     }
 }
 
@@ -578,6 +668,8 @@ const void *bank_kernel_ptr(bool smem) {
 cudaError_t bank_set_attributes() {
     cudaError_t e = cudaFuncSetAttribute(k_bank<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kBankSmemMax);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_bank_seeds<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBankSmemMax);
     return e;
 }
 

@@ -80,8 +80,10 @@ void launch_scan(const int *counts, int *begins, int ntasks, ScanOut *out, int *
 
 // k_bank.cu
 size_t bank_smem_bytes(int nmax);
+// seed_rt: 12 doubles per seed at item_base / kDetC; seed_blocks: blocks of
+// 128 seeds of the task with most (0: a launch of offset items)
 void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks, const ScanOut *scan,
-                 int *counter, double *item_res, int *err, int nmax, int grid,
+                 int *counter, double *seed_rt, int seed_blocks, double *item_res, int *err, int nmax, int grid,
                  unsigned long long *ctr, cudaStream_t st);
 void launch_reduce_bank(const BankTask *tasks, int ntasks, const double *item_res,
                         PairState *state, cudaStream_t st);

@@ -95,7 +95,7 @@ struct Ctx {
     DBuf<ChainTask> ctasks;
     DBuf<int> counts, begins, counter;
     DBuf<ScanOut> scan;
-    DBuf<double> item_res, chain_res, alP, alQ, thread_rec, off_start, off_res, out, snap;
+    DBuf<double> item_res, seed_rt, chain_res, alP, alQ, thread_rec, off_start, off_res, out, snap;
     DBuf<int> lay_i, gidx, omap;
     DBuf<long long> lay_l;
     DBuf<unsigned long long> ctr;
@@ -303,6 +303,7 @@ class Runner {
     Layout L_pair, L_main, L_detss, L_detdp, L_gapless, L_thread, L_topk, L_localn, L_locald,
         L_threadch, L_single, L_offdp, L_offslots, L_cand[kCandKinds];
     long long koff_[kCandKinds + 1] = {0, 0, 0, 0, 0, 0};
+    int kmain_ = 0, kthread_ = 0;  // most seeds of a pair's main bank / of a threading offset
     long long max_items_ = 0, max_chain_recs_ = 0, n_thread_ = 0, n_off_ = 0;
     int chain_grid_ = 0, chain_flags_ = 0, rank_grid_ = 1;
     size_t trace_words_ = 0;
@@ -329,6 +330,8 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     L_pair.base.assign(0, 0);
     L_pair.ntasks = n;
     perpair(L_main, [](const PairInfo &I) { return (long long)I.K * I.C; });
+    for (auto &I : info)
+        if (!I.status && I.K > kmain_) kmain_ = I.K;
     perpair(L_detss, [](const PairInfo &I) {
         int m = I.plen < I.nlen ? I.plen : I.nlen;
         return (long long)kdet_max(m) * kDetC;
@@ -367,7 +370,9 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
             thread_at(I.plen, I.nlen, o, ps, ns, ov);
             L_thread.pair.push_back(p);
             L_thread.aux.push_back(o);
-            L_thread.base.push_back(ov >= 3 ? (long long)arith_seed_count(ov, 5, true) * kDetC : 0);
+            const int seeds = ov >= 3 ? arith_seed_count(ov, 5, true) : 0;
+            L_thread.base.push_back((long long)seeds * kDetC);
+            if (seeds > kthread_) kthread_ = seeds;
         }
     }
     finish_layout(L_thread);
@@ -458,6 +463,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     CK(c_->scan.ensure(1));
     CK(c_->counter.ensure(1));
     CK(c_->item_res.ensure((size_t)(max_items_ > 0 ? max_items_ : 1) * kRec));
+    CK(c_->seed_rt.ensure((size_t)(max_items_ / kDetC + 1) * 12));
     CK(c_->chain_res.ensure((size_t)(max_chain_recs_ > 0 ? max_chain_recs_ : 1) * kRec));
     CK(c_->thread_rec.ensure((size_t)(n_thread_ > 0 ? n_thread_ : 1) * kRec));
     CK(c_->off_start.ensure((size_t)(n_off_ > 0 ? n_off_ : 1) * kRec));
@@ -541,24 +547,37 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
     pc.wcount = wcount;
     pc.wlist = wlist;
     pc.tune = cfg_.tune;
-    launch_plan_bank(b, pc, c_->stream);
-    launch_scan(c_->counts.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->stream);
-    launches_ += 4;
-    bank_launches_++;
-    int nmx = Nmax;
-    size_t sm = bank_smem_bytes(nmx);
+    const size_t sm = bank_smem_bytes(Nmax);
     int per_sm = 0;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bank_kernel_ptr(sm <= kBankSmemMax),
                                                      kBankChunk, sm <= kBankSmemMax ? sm : 0));
     if (per_sm < 1) per_sm = 1;
+    const int grid = c_->sms * per_sm;
+    // a launch that cannot fill the grid with 256-item chunks takes 128, one
+    // group of 32 per warp: its time is the longest warp's, and a second group
+    // would come on top (one 64-residue pair: 0.73 against 1.02 ms
+    // over its nine launches; with more items the two measure the same)
+    if (L.total <= 256LL * grid)
+        for (Tune &t : pc.tune.t) t.bank_chunk = std::min(t.bank_chunk, kBankChunk);
+    launch_plan_bank(b, pc, c_->stream);
+    launch_scan(c_->counts.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->stream);
+    launches_ += kind == BK_GAPLESS ? 4 : 5;
+    bank_launches_++;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing) {
         e0 = new_event();
         e1 = new_event();
         cudaEventRecord(e0, c_->stream);
     }
-    launch_bank(c_->btasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->item_res.p,
-                c_->err.p, nmx, c_->sms * per_sm, b.ctr, c_->stream);
+    // blocks of 128 seeds of the task with most
+    const int seeds = kind == BK_GAPLESS ? 0
+                      : kind == BK_MAIN  ? kmain_
+                      : kind == BK_TOPK  ? 1
+                      : kind == BK_THREAD ? kthread_
+                                          : kdet_max(pmax < nmax ? pmax : nmax);
+    launch_bank(c_->btasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->seed_rt.p,
+                (seeds + kBankChunk - 1) / kBankChunk, c_->item_res.p, c_->err.p,
+                Nmax, grid, b.ctr, c_->stream);
     if (timing) {
         cudaEventRecord(e1, c_->stream);
         bank_ev.push_back({e0, e1});
