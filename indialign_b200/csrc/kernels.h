@@ -62,7 +62,8 @@ void set_last_error_text(const char *msg);
 
 // k_misc.cu
 void launch_prep(const DevBatch &b, int use_frag, cudaStream_t st);
-void launch_anchor(const DevBatch &b, cudaStream_t st);
+void launch_anchor(const DevBatch &b, int Nmax, cudaStream_t st);
+cudaError_t misc_set_attributes();
 void launch_ss(const DevBatch &b, cudaStream_t st);
 void launch_topk(const DevBatch &b, cudaStream_t st);
 void launch_weighted(const DevBatch &b, cudaStream_t st);

@@ -169,6 +169,7 @@ static int acquire(int device, Ctx **out, int tag = 0) {
         attr_err = bank_set_attributes();
         if (attr_err == cudaSuccess) attr_err = chain_set_attributes();
         if (attr_err == cudaSuccess) attr_err = rank_set_attributes();
+        if (attr_err == cudaSuccess) attr_err = misc_set_attributes();
     });
     CK(attr_err);
     *out = c;
@@ -1098,7 +1099,7 @@ static int run_batch(Ctx *c, const Cfg &cfg, const Source &src, double *results,
     r.stage_event(0);
     // ---- seeds ----
     launch_prep(b, cfg.use_frag, st);
-    launch_anchor(b, st);
+    launch_anchor(b, Nmax, st);
     r.launches_ += 2;
     CK(cudaGetLastError());
     std::vector<PairInfo> info(n);

@@ -35,13 +35,14 @@ def test_seed_bank_best_matches_the_oracle(oracle, L, values):
 
 
 def test_global_path_equals_the_shared_one():
-    """6800 residues do not fit k_bank_seeds' shared memory, 6000 do: the same
-    chain, invalid beyond 900 residues, scores the same from both."""
+    """6800 residues do not fit k_bank_seeds' shared memory and 12100 not
+    k_anchor's, 6000 fit both: the same chain, invalid beyond 900 residues,
+    scores the same on every path."""
     rng = np.random.default_rng(9)
     base = W.make_pair(900, 2.0, rng)
     out = []
-    for N in (6000, 6800):
+    for N in (6000, 6800, 12100):
         pad = lambda a: np.concatenate([a, np.zeros((N - 900,) + a.shape[1:], a.dtype)])  # noqa: E731
         p = W.Pair(pad(base.pred), pad(base.native), *(pad(base.valid) for _ in range(3)), 900.0)
         out.append(ia.search([p])[0][0])
-    assert out[0] == pytest.approx(out[1], abs=1e-6)
+    assert out[1:] == pytest.approx([out[0]] * 2, abs=1e-6)
