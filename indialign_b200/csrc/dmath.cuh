@@ -117,6 +117,16 @@ IA_DEV double rcp_nr(double x) {
     return fma(y, e, y);
 }
 
+// a / b for y = 1 / b correctly rounded: Markstein's final step (a quotient
+// within an ulp, its exact residual, one fused correction) rounds like the
+// division itself, so six quotients by one divisor cost one division.  The
+// bits matter: the covariance of exactly collinear points leaves the rotation
+// about their line to the last bits of its entries.
+IA_DEV double div_by(double a, double b, double y) {
+    const double q = a * y;
+    return fma(fma(-b, q, a), y, q);
+}
+
 IA_DEV void horn_matrix(const double (&H)[3][3], double (&A)[4][4]) {
     A[0][0] = H[0][0] + H[1][1] + H[2][2];
     A[0][1] = A[1][0] = H[1][2] - H[2][1];
@@ -182,79 +192,70 @@ IA_DEV void jacobi_reference(double (&A)[4][4], double (&V)[4][4]) {
     }
 }
 
-IA_DEV double det3(double a, double b, double c, double d, double e, double f, double g, double h, double i) {
-    return a * (e * i - f * h) - b * (d * i - f * g) + c * (d * h - e * g);
-}
-
-// Determinant of A without row `row` and column `col`.
-template <int row, int col>
-IA_DEV double minor3(const double (&A)[4][4]) {
-    constexpr int r0 = row == 0 ? 1 : 0, r1 = row <= 1 ? 2 : 1, r2 = row <= 2 ? 3 : 2;
-    constexpr int c0 = col == 0 ? 1 : 0, c1 = col <= 1 ? 2 : 1, c2 = col <= 2 ? 3 : 2;
-    return det3(A[r0][c0], A[r0][c1], A[r0][c2], A[r1][c0], A[r1][c1], A[r1][c2], A[r2][c0], A[r2][c1],
-                A[r2][c2]);
-}
-
-// Column c of adj(A): adj[r][c] = (-1)^(r+c) * minor(c, r).
-template <int c>
-IA_DEV void adj_column(const double (&A)[4][4], double (&v)[4]) {
-    v[0] = ((0 + c) & 1 ? -1.0 : 1.0) * minor3<c, 0>(A);
-    v[1] = ((1 + c) & 1 ? -1.0 : 1.0) * minor3<c, 1>(A);
-    v[2] = ((2 + c) & 1 ? -1.0 : 1.0) * minor3<c, 2>(A);
-    v[3] = ((3 + c) & 1 ? -1.0 : 1.0) * minor3<c, 3>(A);
-}
-
-// Dominant eigenvector of Horn's key matrix F by its characteristic
-// polynomial -- the QCP method (Theobald 2005, "Rapid calculation of RMSDs
-// using a quaternion-based characteristic polynomial").  F is traceless, so
-// P(x) = x^4 + c2 x^2 + c1 x + c0 with c2 = -tr(F^2)/2, c1 = -tr(F^3)/3,
-// c0 = det F.  The largest root l1 comes from Newton's method started at
-// sqrt(tr(F^2)) >= l1, where P is increasing and convex, so the iterates
-// fall monotonically onto l1.  P'(l1) is the product of the gaps to the
+// Dominant eigenvector of Horn's key matrix F of a covariance H by its
+// characteristic polynomial -- the QCP method (Theobald 2005, "Rapid
+// calculation of RMSDs using a quaternion-based characteristic polynomial").
+// F is traceless, so P(x) = x^4 + c2 x^2 + c1 x + c0 with c2 = -2 |H|^2 (half
+// of -tr(F^2)), c1 = -8 det H (a third of -tr(F^3)), c0 = det F.  The largest
+// root l1 comes from Halley's method started at sqrt(3/4 tr(F^2)) >= l1 (four
+// numbers of sum 0 and square sum s reach at most sqrt(3/4 s)); for a
+// polynomial with real roots only, the iterates fall monotonically onto the
+// largest root from above, with cubic convergence, so the loop ends once a step
+// is below 1e-9 of the scale (3-5 iterations; Newton's method from
+// sqrt(tr(F^2)) took 7-9).  P'(l1) is the product of the gaps to the
 // other eigenvalues, each at most 2 sqrt(tr(F^2)); when it cannot prove
-// l1 - l2 >= 1e-4 sqrt(tr(F^2)), l2 is found the same way on P(x)/(x - l1).
-// A top pair closer than that returns false: the eigenvector inside a
-// (near-)degenerate pair depends on the solver, and the caller reruns the
-// reference's Jacobi sequence.  Otherwise the eigenvector is the adjugate
-// column of F - l1 I with the largest diagonal entry.  A CPU build of the
-// oracle with this eigen-solve matched the reference build's final scores to
-// 3e-16 on 560 pairs, Jacobi rerunning in ~6e-5 of the solves.
-IA_DEV bool qcp_rotation(const double (&F)[4][4], double *R) {
-    double p2 = 0.0, p3 = 0.0;
+// l1 - l2 >= 1e-4 sqrt(tr(F^2)), l2 is found by Newton's method on P(x)/(x - l1).
+// A top pair closer than that returns false, as does a scale whose sixth power
+// would leave the double range: the eigenvector inside a (near-)degenerate pair
+// depends on the solver, and the caller reruns the reference's Jacobi sequence.
+// Otherwise the eigenvector is the column of adj(F - l1 I) with the largest
+// diagonal entry: the adjugate of the symmetric matrix whole (14 two-by-two
+// minors, 10 cofactors), so that lanes with different columns do not diverge,
+// and the rotation's entries divided by |v|^2 once instead of normalising v.
+// A CPU build of the oracle with a characteristic-polynomial solve matched the
+// reference build's final scores to 3e-16 on 560 pairs, Jacobi rerunning in
+// ~6e-5 of the solves.  The solve is a serial chain of FP64 operations; this
+// form took k_bank's launches on one 64-residue pair from 0.75 to 0.68 ms and k_chain
+// on 64 pairs of L 40-300 from 60.3 to 57.2 ms.
+IA_DEV bool qcp_rotation(const double (&H)[3][3], double *R) {
+    double n2 = 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int r = 0; r < 3; r++)
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            double f2 = 0.0;
-#pragma unroll
-            for (int j = 0; j < 4; j++) f2 = fma(F[i][j], F[j][k], f2);
-            p3 = fma(f2, F[k][i], p3);
-            p2 = fma(F[i][k], F[i][k], p2);
-        }
-    const double s0 = F[0][0] * F[1][1] - F[1][0] * F[0][1], s1 = F[0][0] * F[1][2] - F[1][0] * F[0][2];
-    const double s2 = F[0][0] * F[1][3] - F[1][0] * F[0][3], s3 = F[0][1] * F[1][2] - F[1][1] * F[0][2];
-    const double s4 = F[0][1] * F[1][3] - F[1][1] * F[0][3], s5 = F[0][2] * F[1][3] - F[1][2] * F[0][3];
-    const double k5 = F[2][2] * F[3][3] - F[3][2] * F[2][3], k4 = F[2][1] * F[3][3] - F[3][1] * F[2][3];
-    const double k3 = F[2][1] * F[3][2] - F[3][1] * F[2][2], k2 = F[2][0] * F[3][3] - F[3][0] * F[2][3];
-    const double k1 = F[2][0] * F[3][2] - F[3][0] * F[2][2], k0 = F[2][0] * F[3][1] - F[3][0] * F[2][1];
-    const double c0 = s0 * k5 - s1 * k4 + s2 * k3 + s3 * k2 - s4 * k1 + s5 * k0;
-    const double c2 = -0.5 * p2, c1 = -p3 * (1.0 / 3.0);
-    if (!(p2 > 0.0)) return false;
+        for (int c = 0; c < 3; c++) n2 = fma(H[r][c], H[r][c], n2);
+    const double p2 = 4.0 * n2;  // tr(F^2)
+    if (!(p2 > 1e-80 && p2 < 1e80)) return false;
+    const double a01 = H[1][2] - H[2][1], a02 = H[2][0] - H[0][2], a03 = H[0][1] - H[1][0];
+    const double a12 = H[0][1] + H[1][0], a13 = H[2][0] + H[0][2], a23 = H[1][2] + H[2][1];
+    double a00 = H[0][0] + H[1][1] + H[2][2], a11 = H[0][0] - H[1][1] - H[2][2];
+    double a22 = -H[0][0] + H[1][1] - H[2][2], a33 = -H[0][0] - H[1][1] + H[2][2];
+    const double detH = H[0][0] * (H[1][1] * H[2][2] - H[1][2] * H[2][1]) -
+                        H[0][1] * (H[1][0] * H[2][2] - H[1][2] * H[2][0]) +
+                        H[0][2] * (H[1][0] * H[2][1] - H[1][1] * H[2][0]);
+    const double c2 = -2.0 * n2, c1 = -8.0 * detH;
+    double c0;
+    {
+        const double b1 = a22 * a33 - a23 * a23, b2 = a12 * a33 - a13 * a23, b3 = a12 * a23 - a13 * a22;
+        const double d1 = a11 * a33 - a13 * a13, d2 = a11 * a23 - a12 * a13, d3 = a11 * a22 - a12 * a12;
+        c0 = a00 * (a11 * b1 - a12 * b2 + a13 * b3) - a01 * (a01 * b1 - a02 * b2 + a03 * b3) +
+             a02 * (a01 * b2 - a02 * d1 + a03 * d2) - a03 * (a01 * b3 - a02 * d2 + a03 * d3);
+    }
     const double scale = sqrt(p2);
-    double l1 = scale, dp = 0.0;
+    double l1 = 0.8660254037844387 * scale;
 #pragma unroll 1
     for (int it = 0; it < 64; it++) {
         const double x2 = l1 * l1;
         const double g = fma(fma(x2 + c2, l1, c1), l1, c0);
-        dp = fma(fma(4.0 * x2, 1.0, 2.0 * c2), l1, c1);
-        if (!(dp > 0.0)) break;
-        const double nx = l1 - g * rcp_nr(dp);
+        const double dg = fma(fma(4.0, x2, 2.0 * c2), l1, c1);
+        const double hg = fma(6.0, x2, c2);  // P''/2
+        if (!(dg > 0.0)) break;
+        const double nx = l1 - g * dg * rcp_nr(fma(dg, dg, -g * hg));
         if (!(nx < l1)) break;
-        const bool done = l1 - nx <= 1e-16 * scale;
+        const bool done = l1 - nx <= 1e-9 * scale;
         l1 = nx;
         if (done) break;
     }
-    dp = fma(fma(4.0 * l1 * l1, 1.0, 2.0 * c2), l1, c1);  // P'(l1)
+    const double dp = fma(fma(4.0 * l1, l1, 2.0 * c2), l1, c1);  // P'(l1)
     if (!(dp >= 4e-4 * p2 * scale)) {
         // second eigenvalue: largest root of x^3 + l1 x^2 + (c2 + l1^2) x + (c1 + l1 c2 + l1^3)
         const double b2 = l1, b1 = fma(l1, l1, c2), b0 = fma(l1, b1, c1);
@@ -272,44 +273,52 @@ IA_DEV bool qcp_rotation(const double (&F)[4][4], double *R) {
         }
         if (!(l1 - x >= 1e-4 * scale)) return false;
     }
-    double A[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) A[i][j] = i == j ? F[i][j] - l1 : F[i][j];
-    // adj(A) = P'(l1) q q^T: its largest diagonal entry marks the best column
-    const double a0 = fabs(minor3<0, 0>(A)), a1 = fabs(minor3<1, 1>(A)), a2 = fabs(minor3<2, 2>(A)),
-                 a3 = fabs(minor3<3, 3>(A));
-    double v[4];
-    if (a0 >= a1 && a0 >= a2 && a0 >= a3) adj_column<0>(A, v);
-    else if (a1 >= a2 && a1 >= a3) adj_column<1>(A, v);
-    else if (a2 >= a3) adj_column<2>(A, v);
-    else adj_column<3>(A, v);
-    const double n2 = v[0] * v[0] + v[1] * v[1] + v[2] * v[2] + v[3] * v[3];
-    if (!(n2 > 0.0)) return false;
-    const double inv = 1.0 / sqrt(n2);
-    const double q0 = v[0] * inv, q1 = v[1] * inv, q2 = v[2] * inv, q3 = v[3] * inv;
-    R[0] = q0 * q0 + q1 * q1 - q2 * q2 - q3 * q3;
-    R[1] = 2 * (q1 * q2 + q0 * q3);
-    R[2] = 2 * (q1 * q3 - q0 * q2);
-    R[3] = 2 * (q1 * q2 - q0 * q3);
-    R[4] = q0 * q0 - q1 * q1 + q2 * q2 - q3 * q3;
-    R[5] = 2 * (q2 * q3 + q0 * q1);
-    R[6] = 2 * (q1 * q3 + q0 * q2);
-    R[7] = 2 * (q2 * q3 - q0 * q1);
-    R[8] = q0 * q0 - q1 * q1 - q2 * q2 + q3 * q3;
+    a00 -= l1;
+    a11 -= l1;
+    a22 -= l1;
+    a33 -= l1;
+    const double b1 = a22 * a33 - a23 * a23, b2 = a12 * a33 - a13 * a23, b3 = a12 * a23 - a13 * a22;
+    const double d1 = a11 * a33 - a13 * a13, d2 = a11 * a23 - a12 * a13, d3 = a11 * a22 - a12 * a12;
+    const double e1 = a02 * a33 - a03 * a23, e2 = a02 * a23 - a03 * a22, e3 = a02 * a13 - a12 * a03;
+    const double f1 = a01 * a33 - a13 * a03, f2 = a01 * a13 - a11 * a03, f3 = a01 * a22 - a12 * a02;
+    const double f4 = a01 * a12 - a11 * a02, f5 = a01 * a23 - a12 * a03;
+    const double k00 = a11 * b1 - a12 * b2 + a13 * b3, k01 = -(a01 * b1 - a02 * b2 + a03 * b3);
+    const double k02 = a01 * b2 - a02 * d1 + a03 * d2, k03 = -(a01 * b3 - a02 * d2 + a03 * d3);
+    const double k11 = a00 * b1 - a02 * e1 + a03 * e2, k12 = -(a00 * b2 - a01 * e1 + a03 * e3);
+    const double k13 = a00 * b3 - a01 * e2 + a02 * e3, k22 = a00 * d1 - a01 * f1 + a03 * f2;
+    const double k23 = -(a00 * d2 - a01 * f5 + a02 * f2), k33 = a00 * d3 - a01 * f3 + a02 * f4;
+    // adj(F - l1 I) = P'(l1) q q^T: its largest diagonal entry marks the best column
+    double v0 = k00, v1 = k01, v2 = k02, v3 = k03, top = fabs(k00);
+    if (fabs(k11) > top) { v0 = k01; v1 = k11; v2 = k12; v3 = k13; top = fabs(k11); }
+    if (fabs(k22) > top) { v0 = k02; v1 = k12; v2 = k22; v3 = k23; top = fabs(k22); }
+    if (fabs(k33) > top) { v0 = k03; v1 = k13; v2 = k23; v3 = k33; }
+    const double vv = v0 * v0 + v1 * v1 + v2 * v2 + v3 * v3;
+    if (!(vv > 0.0)) return false;
+    const double inv = rcp_nr(vv), two = 2.0 * inv;
+    R[0] = (v0 * v0 + v1 * v1 - v2 * v2 - v3 * v3) * inv;
+    R[1] = two * (v1 * v2 + v0 * v3);
+    R[2] = two * (v1 * v3 - v0 * v2);
+    R[3] = two * (v1 * v2 - v0 * v3);
+    R[4] = (v0 * v0 - v1 * v1 + v2 * v2 - v3 * v3) * inv;
+    R[5] = two * (v2 * v3 + v0 * v1);
+    R[6] = two * (v1 * v3 + v0 * v2);
+    R[7] = two * (v2 * v3 - v0 * v1);
+    R[8] = (v0 * v0 - v1 * v1 - v2 * v2 + v3 * v3) * inv;
     return true;
 }
 
 // Horn's 4x4 from the 3x3 covariance H -> dominant eigenvector -> rotation
 // (indialign_c/core.h:64-90): the characteristic-polynomial solve above, or
-// the reference's Jacobi sequence when the top eigenvalue is not separated.
-IA_DEV void cov_to_rotation(const double (&H)[3][3], double *R) {
+// the reference's Jacobi sequence when the top eigenvalue is not separated
+// (rare, and large: out of line).
+static __device__ __noinline__ void jacobi_rotation(const double (&H)[3][3], double *R) {
     double A[4][4], V[4][4];
     horn_matrix(H, A);
-    if (qcp_rotation(A, R)) return;
     jacobi_reference(A, V);
     quat_to_rotation(A, V, R);
+}
+IA_DEV void cov_to_rotation(const double (&H)[3][3], double *R) {
+    if (!qcp_rotation(H, R)) jacobi_rotation(H, R);
 }
 
 // Raw first and second moments of a selected point set.
@@ -366,10 +375,11 @@ static __device__ __noinline__ void kabsch_from_moments(const Moments &m, double
         return;
     }
     double cP[3], cQ[3], H[3][3];
+    const double inv_w = 1.0 / m.w;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        cP[d] = m.sp[d] / m.w;
-        cQ[d] = m.sq[d] / m.w;
+        cP[d] = div_by(m.sp[d], m.w, inv_w);
+        cQ[d] = div_by(m.sq[d], m.w, inv_w);
     }
 #pragma unroll
     for (int r = 0; r < 3; r++)
