@@ -317,6 +317,12 @@ int indialign_gemm_bf16(const void *d_a, int lda, int a_mn, const void *d_b, int
 /* One Adam step (bias-corrected, step >= 1) on the trained blob entries. */
 int indialign_mlp_adam(float *d_blob, const float *d_grad, float *d_m, float *d_v, int step,
                        float lr, float beta1, float beta2, float eps, void *stream);
+/* One whole training step: forward, loss, backward, Adam and repack, as the
+ * calls above in sequence (d_y, d_dy, d_loss, d_grad written, d_blob, d_m, d_v
+ * and d_packed updated; d_save and d_work are scratch of their sizes for n). */
+int indialign_mlp_step(float *d_blob, void *d_packed, const float *d_x, const float *d_t, int n, float lambda,
+                       float *d_y, float *d_dy, float *d_loss, float *d_grad, float *d_m, float *d_v, int step,
+                       float lr, float beta1, float beta2, float eps, void *d_save, void *d_work, void *stream);
 
 /* Measured FP64 FMA throughput of the device in TFLOP/s (the roofline
  * denominator for the FP64 SIMT kernels: NW chains, Kabsch). */

@@ -137,7 +137,10 @@ def load(path: str | None = None) -> ctypes.CDLL:
                                      ctypes.c_int, ctypes.c_int, vp, ctypes.c_int, ctypes.c_int, vp, ctypes.c_int,
                                      vp], ctypes.c_int),
             ("indialign_mlp_adam", [vp, vp, vp, vp, ctypes.c_int, ctypes.c_float, ctypes.c_float,
-                                    ctypes.c_float, ctypes.c_float, vp], ctypes.c_int)):
+                                    ctypes.c_float, ctypes.c_float, vp], ctypes.c_int),
+            ("indialign_mlp_step", [vp, vp, vp, vp, ctypes.c_int, ctypes.c_float, vp, vp, vp, vp, vp, vp,
+                                    ctypes.c_int, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                                    vp, vp, vp], ctypes.c_int)):
         f = getattr(lib, name)
         f.argtypes = args
         f.restype = res

@@ -28,6 +28,9 @@
 //             in block order; Adam on FP32 master weights.
 #include <cuda_bf16.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "dmath.cuh"
 #include "pipeline.h"
 #include "kernels.h"
@@ -79,15 +82,34 @@ IA_DEV float gelu_grad(float x) {
     return 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * kGeluC * (1.0f + 3.0f * kGeluA * x * x);
 }
 
+// GELU and its derivative from one tanh.
+IA_DEV void gelu_both(float x, float &g, float &dg) {
+    const float u = kGeluC * (x + kGeluA * x * x * x);
+    const float th = tanhf(u);
+    g = 0.5f * x * (1.0f + th);
+    dg = 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * kGeluC * (1.0f + 3.0f * kGeluA * x * x);
+}
+
+// Rows of `words` packed BF16 pairs into padded shared rows, 16 bytes a load
+// (4 where the caller's packed buffer is not aligned).
+IA_DEV void load_weight_rows(const uint16_t *g, uint32_t *dst, int rows, int words, int stride) {
+    if (reinterpret_cast<uintptr_t>(g) & 15) {
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(g);
+        for (int i = threadIdx.x; i < rows * words; i += blockDim.x) dst[(i / words) * stride + i % words] = src[i];
+        return;
+    }
+    const uint4 *src = reinterpret_cast<const uint4 *>(g);
+    const int per = words / 4, total = rows * per;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < total; i += blockDim.x)
+        *reinterpret_cast<uint4 *>(dst + (i / per) * stride + 4 * (i % per)) = src[i];
+}
+
 // Copy the packed parameters into the fragment-friendly shared layout (all
 // threads of the CTA; caller synchronises).
 IA_DEV void load_mlp_smem(const MlpPacked *g, MlpSmem *s) {
-    const uint32_t *w1 = reinterpret_cast<const uint32_t *>(g->W1T);
-    const uint32_t *w2 = reinterpret_cast<const uint32_t *>(g->W2T);
-    for (int i = threadIdx.x; i < kHidden * (kFeatures / 2); i += blockDim.x)
-        s->w1t[i / (kFeatures / 2)][i % (kFeatures / 2)] = w1[i];
-    for (int i = threadIdx.x; i < kHidden * (kHidden / 2); i += blockDim.x)
-        s->w2t[i / (kHidden / 2)][i % (kHidden / 2)] = w2[i];
+    load_weight_rows(g->W1T, s->w1t[0], kHidden, kFeatures / 2, kW1Words);
+    load_weight_rows(g->W2T, s->w2t[0], kHidden, kHidden / 2, kW2Words);
     for (int i = threadIdx.x; i < kHidden; i += blockDim.x) {
         s->b1[i] = g->b1[i];
         s->b2[i] = g->b2[i];
@@ -649,7 +671,11 @@ __global__ void k_mlp_pack(const float *__restrict__ blob, MlpPacked *out) {
     if (i == 0) out->b3 = blob[kBlobB3];
 }
 
-// Forward over n raw feature rows (row-major [n][16]); 4 warps x 16 rows per CTA.
+// Forward over n raw feature rows (row-major [n][16]): a warp takes 16-row
+// tiles, a CTA keeps the weights in shared memory for all tiles of its warps
+// (the grid is at most the resident CTAs).  Bound by the 256 tanhf of a row,
+// two thirds of the instructions.  Measured with weights loaded per 64 rows in
+// 4-byte words before: 200003 rows 90 -> 76 us.
 __global__ void __launch_bounds__(128) k_mlp_forward(const MlpPacked *mlp, const float *__restrict__ x, int n,
                                                      float *y, MlpSave sv, int save) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -657,21 +683,23 @@ __global__ void __launch_bounds__(128) k_mlp_forward(const MlpPacked *mlp, const
     float *xt = reinterpret_cast<float *>(smem_raw + sizeof(MlpSmem)) + (threadIdx.x >> 5) * 256;
     load_mlp_smem(mlp, &S);
     __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const long long row0 = (long long)blockIdx.x * 64 + (threadIdx.x >> 5) * 16;
-    if (row0 >= n) return;
-    const int nvalid = n - row0 < 16 ? (int)(n - row0) : 16;
-    for (int e = lane; e < 256; e += 32) {
-        const int r = e >> 4, j = e & 15;
-        xt[e] = r < nvalid ? (x[(row0 + r) * kFeatures + j] - S.mean[j]) * S.inv_std[j] : 0.f;
-    }
-    __syncwarp();
-    float y0, y8;
-    mlp_tile(S, xt, y0, y8, save ? &sv : nullptr, row0, nvalid);
-    const int g = lane >> 2;
-    if ((lane & 3) == 0) {
-        if (g < nvalid) y[row0 + g] = y0;
-        if (g + 8 < nvalid) y[row0 + g + 8] = y8;
+    const int lane = threadIdx.x & 31, g = lane >> 2;
+    const int tiles = (n + 15) / 16, step = gridDim.x * 4;
+    for (int tile = blockIdx.x * 4 + (threadIdx.x >> 5); tile < tiles; tile += step) {
+        const long long row0 = (long long)tile * 16;
+        const int nvalid = n - row0 < 16 ? (int)(n - row0) : 16;
+        for (int e = lane; e < 256; e += 32) {
+            const int r = e >> 4, j = e & 15;
+            xt[e] = r < nvalid ? (x[(row0 + r) * kFeatures + j] - S.mean[j]) * S.inv_std[j] : 0.f;
+        }
+        __syncwarp();
+        float y0, y8;
+        mlp_tile(S, xt, y0, y8, save ? &sv : nullptr, row0, nvalid);
+        if ((lane & 3) == 0) {
+            if (g < nvalid) y[row0 + g] = y0;
+            if (g + 8 < nvalid) y[row0 + g + 8] = y8;
+        }
+        __syncwarp();
     }
 }
 
@@ -806,7 +834,261 @@ __global__ void k_adam(float *w, const float *__restrict__ g, float *m, float *v
     w[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
 }
 
+// ---- one training step ------------------------------------------------------------
+// Forward, loss, its gradient (the ranking term pairs rows 2i, 2i + 1, both in
+// a tile) and dz2 = dy w3 gelu'(z2) of 16 rows per warp, in registers: one tanh
+// per activation serves the forward and the backward, and of the FP32
+// activations only gelu'(z1) goes to memory.  The operands of the three
+// products (xn, h1, dz2 in BF16) are left to k_gemm_tc_act and k_gemm_tc_pair;
+// the column sums (db2, dw3), the sum of dy and the loss go to
+// red[block * kStepRed], per CTA, added in block order by k_step_finish.
+//
+// A step is latency-bound (4 launches here against 15 with a kernel per
+// operation): batch 8192 91 -> 52 us, batch 1003 85 -> 46 us.
+struct StepSmem {
+    MlpSmem w;
+    float col[4][2 * kHidden];  // per warp: column sums of dz2, dy gelu(z2)
+    float sc[4][2];             // per warp: sum of dy, loss
+    float xt[4][256];
+};
+
+// v summed over the eight row groups of a fragment (lanes of equal lane % 4).
+IA_DEV float sum_groups(float v) {
+#pragma unroll
+    for (int o = 4; o < 32; o <<= 1) v += __shfl_xor_sync(kAllLanes, v, o);
+    return v;
+}
+
+__global__ void __launch_bounds__(128) k_step_rows(const MlpPacked *mlp, StepRows a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    StepSmem &S = *reinterpret_cast<StepSmem *>(smem_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, n = a.n;
+    const int row0 = (blockIdx.x * 4 + warp) * 16, rg = row0 + g, rg8 = rg + 8;
+    const bool st_g = rg < n, st_g8 = rg8 < n;
+    load_mlp_smem(mlp, &S.w);
+    __syncthreads();
+    float *xt = S.xt[warp];
+    for (int e = lane; e < 256; e += 32) {
+        const int r = e >> 4, j = e & 15;
+        xt[e] = row0 + r < n ? (a.x[(size_t)(row0 + r) * kFeatures + j] - S.w.mean[j]) * S.w.inv_std[j] : 0.f;
+    }
+    __syncwarp();
+    // layer 1
+    uint32_t A[4];
+    A[0] = pack_bf16(xt[g * 16 + 2 * c], xt[g * 16 + 2 * c + 1]);
+    A[1] = pack_bf16(xt[(g + 8) * 16 + 2 * c], xt[(g + 8) * 16 + 2 * c + 1]);
+    A[2] = pack_bf16(xt[g * 16 + 2 * c + 8], xt[g * 16 + 2 * c + 9]);
+    A[3] = pack_bf16(xt[(g + 8) * 16 + 2 * c + 8], xt[(g + 8) * 16 + 2 * c + 9]);
+    // the lane's words of a 16-column chunk kk of two rows of a [n][128] BF16 matrix
+    auto put = [&](uint16_t *m, int kk, const uint32_t (&f)[4]) {
+        if (st_g) {
+            uint32_t *o = reinterpret_cast<uint32_t *>(m + (size_t)rg * kHidden + 16 * kk);
+            o[c] = f[0];
+            o[4 + c] = f[2];
+        }
+        if (st_g8) {
+            uint32_t *o = reinterpret_cast<uint32_t *>(m + (size_t)rg8 * kHidden + 16 * kk);
+            o[c] = f[1];
+            o[4 + c] = f[3];
+        }
+    };
+    if (st_g) {
+        uint32_t *o = reinterpret_cast<uint32_t *>(a.xn + (size_t)rg * kFeatures);
+        o[c] = A[0];
+        o[4 + c] = A[2];
+    }
+    if (st_g8) {
+        uint32_t *o = reinterpret_cast<uint32_t *>(a.xn + (size_t)rg8 * kFeatures);
+        o[c] = A[1];
+        o[4 + c] = A[3];
+    }
+    uint32_t h[8][4];
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++) {
+        float ge[2][4];
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const int nt = 2 * kk + half, col = 8 * nt + 2 * c;
+            float d[4] = {S.w.b1[col], S.w.b1[col + 1], S.w.b1[col], S.w.b1[col + 1]}, dg[4];
+            mma_bf16(d, A, S.w.w1t[8 * nt + g][c], S.w.w1t[8 * nt + g][c + 4]);
+#pragma unroll
+            for (int e = 0; e < 4; e++) gelu_both(d[e], ge[half][e], dg[e]);
+            if (st_g) *reinterpret_cast<float2 *>(a.g1 + (size_t)rg * kHidden + col) = make_float2(dg[0], dg[1]);
+            if (st_g8) *reinterpret_cast<float2 *>(a.g1 + (size_t)rg8 * kHidden + col) = make_float2(dg[2], dg[3]);
+        }
+        h[kk][0] = pack_bf16(ge[0][0], ge[0][1]);
+        h[kk][1] = pack_bf16(ge[0][2], ge[0][3]);
+        h[kk][2] = pack_bf16(ge[1][0], ge[1][1]);
+        h[kk][3] = pack_bf16(ge[1][2], ge[1][3]);
+        put(a.h1, kk, h[kk]);
+    }
+    // layer 2 and the head
+    float ge[16][4], dg[16][4], y0 = 0.f, y8 = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < 16; nt++) {
+        const int col = 8 * nt + 2 * c;
+        float d[4] = {S.w.b2[col], S.w.b2[col + 1], S.w.b2[col], S.w.b2[col + 1]};
+        const uint32_t *wr = S.w.w2t[8 * nt + g];
+#pragma unroll
+        for (int kk = 0; kk < 8; kk++) mma_bf16(d, h[kk], wr[8 * kk + c], wr[8 * kk + c + 4]);
+#pragma unroll
+        for (int e = 0; e < 4; e++) gelu_both(d[e], ge[nt][e], dg[nt][e]);
+        y0 += ge[nt][0] * S.w.w3[col] + ge[nt][1] * S.w.w3[col + 1];
+        y8 += ge[nt][2] * S.w.w3[col] + ge[nt][3] * S.w.w3[col + 1];
+    }
+    y0 += __shfl_xor_sync(kAllLanes, y0, 1);
+    y0 += __shfl_xor_sync(kAllLanes, y0, 2);
+    y8 += __shfl_xor_sync(kAllLanes, y8, 1);
+    y8 += __shfl_xor_sync(kAllLanes, y8, 2);
+    y0 += S.w.b3;
+    y8 += S.w.b3;
+    // loss (k_mlp_loss): rows 2i, 2i + 1 are lanes g, g ^ 1
+    const int m = n / 2;
+    const float inv_n = 1.0f / (float)n, inv_m = 1.0f / (float)(m > 0 ? m : 1);
+    float loss = 0.f;
+    auto row_dy = [&](int r, float y) {
+        const float t = r < n ? a.t[r] : 0.f, yo = __shfl_xor_sync(kAllLanes, y, 4), to = __shfl_xor_sync(kAllLanes, t, 4);
+        if (r >= n) return 0.f;
+        const float e = y - t;
+        float d = 2.f * e * inv_n;
+        loss += e * e * inv_n;
+        const float sign = (r & 1) ? -1.f : 1.f, dt = sign * (t - to);  // t[2i] - t[2i + 1]
+        if (r < 2 * m && fabsf(dt) > 1e-6f) {
+            const float sgn = dt > 0.f ? 1.f : -1.f, z = -sgn * (sign * (y - yo));
+            const float sig = 1.f / (1.f + expf(-z));
+            d += -sign * a.lambda * sgn * sig * inv_m;
+            if (!(r & 1)) loss += a.lambda * (z > 20.f ? z : log1pf(expf(z))) * inv_m;
+        }
+        return d;
+    };
+    const float dy0 = row_dy(rg, y0), dy8 = row_dy(rg8, y8);
+    if (c == 0) {
+        if (st_g) {
+            a.y[rg] = y0;
+            a.dy[rg] = dy0;
+        }
+        if (st_g8) {
+            a.y[rg8] = y8;
+            a.dy[rg8] = dy8;
+        }
+    }
+    const float sdy = sum_groups(dy0 + dy8), sl = sum_groups(loss);
+    if (lane == 0) {
+        S.sc[warp][0] = sdy;
+        S.sc[warp][1] = sl;
+    }
+    // dz2 and the sums of db2, dw3
+    float *col_out = S.col[warp];
+#pragma unroll
+    for (int kk = 0; kk < 8; kk++) {
+        float v[2][4];
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const int nt = 2 * kk + half, col = 8 * nt + 2 * c;
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[half][e] = (e < 2 ? dy0 : dy8) * S.w.w3[col + (e & 1)] * dg[nt][e];
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const float b2 = sum_groups(v[half][e] + v[half][e + 2]);
+                const float w3 = sum_groups(dy0 * ge[nt][e] + dy8 * ge[nt][e + 2]);
+                if (g == 0) {
+                    col_out[col + e] = b2;
+                    col_out[kHidden + col + e] = w3;
+                }
+            }
+        }
+        const uint32_t f[4] = {pack_bf16(v[0][0], v[0][1]), pack_bf16(v[0][2], v[0][3]), pack_bf16(v[1][0], v[1][1]),
+                               pack_bf16(v[1][2], v[1][3])};
+        put(a.dz2, kk, f);
+    }
+    __syncthreads();
+    float *red = a.red + (size_t)blockIdx.x * kStepRed;
+    for (int j = threadIdx.x; j < 2 * kHidden; j += blockDim.x)
+        red[j] = S.col[0][j] + S.col[1][j] + S.col[2][j] + S.col[3][j];
+    if (threadIdx.x < 2)
+        red[2 * kHidden + threadIdx.x] =
+            S.sc[0][threadIdx.x] + S.sc[1][threadIdx.x] + S.sc[2][threadIdx.x] + S.sc[3][threadIdx.x];
+}
+
+// Gradient of every parameter from the partial sums (split-K tiles of dW2 and
+// of dW1 transposed, per-CTA sums of the rest, in a fixed order), the Adam
+// update and the packed copy, a thread per parameter.
+__global__ void __launch_bounds__(256) k_step_finish(StepFinish f, MlpPacked *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int b = 0; b < f.blocks; b++) s += f.red[(size_t)b * kStepRed + 2 * kHidden + 1];
+        *f.loss = s;
+    }
+    if (i < kFeatures) {
+        out->mean[i] = f.blob[kBlobMean + i];
+        const float sd = f.blob[kBlobStd + i];
+        out->inv_std[i] = sd > 0.f ? 1.0f / sd : 1.0f;
+    }
+    if (i < kBlobW1) f.grad[i] = 0.f;
+    if (i < kBlobW1 || i >= kBlobSize) return;
+    // where this parameter's partial sums stand: count, first, distance
+    int cnt = f.blocks, o = 0;
+    size_t stride = kStepRed;
+    const float *src = f.red;
+    if (i < kBlobB1) {
+        o = i - kBlobW1;
+        cnt = f.splits;
+        stride = kHidden * kFeatures;
+        src = f.part1 + (o % kHidden) * kFeatures + o / kHidden;
+    } else if (i < kBlobW2) {
+        cnt = f.blocks1;
+        stride = kHidden;
+        src = f.red1 + (i - kBlobB1);
+    } else if (i < kBlobB2) {
+        cnt = f.splits;
+        stride = kHidden * kHidden;
+        src = f.part2 + (i - kBlobW2);
+    } else if (i < kBlobW3) {
+        src += i - kBlobB2;
+    } else if (i < kBlobB3) {
+        src += kHidden + (i - kBlobW3);
+    } else {
+        src += 2 * kHidden;
+    }
+    float gi = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < cnt; k++) gi += src[(size_t)k * stride];
+    f.grad[i] = gi;
+    const float mi = f.b1 * f.m[i] + (1.f - f.b1) * gi;
+    const float vi = f.b2 * f.v[i] + (1.f - f.b2) * gi * gi;
+    f.m[i] = mi;
+    f.v[i] = vi;
+    const float w = f.blob[i] - f.lr * (mi / f.bc1) / (sqrtf(vi / f.bc2) + f.eps);
+    f.blob[i] = w;
+    const uint16_t wb = __bfloat16_as_ushort(__float2bfloat16_rn(w));
+    if (i < kBlobB1) {
+        out->W1T[(o % kHidden) * kFeatures + o / kHidden] = wb;
+    } else if (i < kBlobW2) {
+        out->b1[i - kBlobB1] = w;
+    } else if (i < kBlobB2) {
+        const int e = i - kBlobW2;
+        out->W2[e] = wb;
+        out->W2T[(e % kHidden) * kHidden + e / kHidden] = wb;
+    } else if (i < kBlobW3) {
+        out->b2[i - kBlobB2] = w;
+    } else if (i < kBlobB3) {
+        out->w3[i - kBlobW3] = w;
+    } else {
+        out->b3 = w;
+    }
+}
+
 // ---- launch wrappers ------------------------------------------------------------
+void launch_step_rows(const MlpPacked *mlp, const StepRows &a, cudaStream_t st) {
+    k_step_rows<<<step_blocks(a.n), 128, sizeof(StepSmem), st>>>(mlp, a);
+}
+
+void launch_step_finish(const StepFinish &f, MlpPacked *out, cudaStream_t st) {
+    k_step_finish<<<(kBlobSize + 255) / 256, 256, 0, st>>>(f, out);
+}
+
 size_t rank_smem_bytes() { return sizeof(MlpSmem) + 4 * 256 * sizeof(float); }
 
 const void *rank_kernel_ptr() { return (const void *)k_rank; }
@@ -848,11 +1130,43 @@ void launch_mlp_pack(const float *blob, MlpPacked *out, cudaStream_t st) {
     k_mlp_pack<<<(kHidden * kHidden + 255) / 256, 256, 0, st>>>(blob, out);
 }
 
+// Resident CTAs of k_mlp_forward on the current device, and the shared-memory
+// limit of k_step_rows raised there, once per device.
+static int forward_grid() {
+    static std::mutex mu;
+    static int grid[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    std::lock_guard<std::mutex> lk(mu);
+    if (!grid[dev]) {
+        int sms = 148, per = 1;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mlp_forward, 128, rank_smem_bytes()) != cudaSuccess ||
+            per < 1)
+            per = 1;
+        grid[dev] = sms * per;
+    }
+    return grid[dev];
+}
+
+bool step_attributes() {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    const uint64_t bit = 1ull << dev;
+    if (done.load() & bit) return true;
+    if (cudaFuncSetAttribute(k_step_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem)) != cudaSuccess)
+        return false;
+    done.fetch_or(bit);
+    return true;
+}
+
 void launch_mlp_forward(const MlpPacked *mlp, const float *x, int n, float *y, const MlpSave *save,
                         cudaStream_t st) {
     if (n <= 0) return;
     MlpSave sv = save ? *save : MlpSave{nullptr, nullptr, nullptr, nullptr};
-    k_mlp_forward<<<(n + 63) / 64, 128, rank_smem_bytes(), st>>>(mlp, x, n, y, sv, save ? 1 : 0);
+    const int tiles4 = (n + 63) / 64, most = forward_grid();
+    k_mlp_forward<<<tiles4 < most ? tiles4 : most, 128, rank_smem_bytes(), st>>>(mlp, x, n, y, sv, save ? 1 : 0);
 }
 
 void launch_mlp_loss(const float *y, const float *t, int n, float lambda, float *dy, float *loss,

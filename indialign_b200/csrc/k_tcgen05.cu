@@ -31,6 +31,7 @@
 // wait, writes NaN over its output tile (so the loss and gradients show the
 // failure), and still frees its TMEM columns.
 #include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
@@ -95,12 +96,20 @@ struct TcArgs {
     int *err;
 };
 
-__global__ void __launch_bounds__(128, 1)
-k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcArgs a) {
+// The epilogue of k_gemm_tc_act: out = C * scale in BF16, and the tile's column sums.
+struct ActArgs {
+    const float *scale;  // [M][N]
+    uint16_t *out;       // [M][N]
+    float *red;          // [tiles][N]
+};
+
+template <bool ACT>
+IA_DEV void gemm_tile(const CUtensorMap &tmA, const CUtensorMap &tmB, const TcArgs &a, const ActArgs &act) {
     extern __shared__ __align__(1024) unsigned char tc_raw[];
     __shared__ uint64_t full[kTcStages], done[kTcStages];
     __shared__ uint32_t tmem_base;
     __shared__ int failed;
+    __shared__ float colsum[ACT ? 4 : 1][ACT ? kHidden : 1];
     unsigned char *base =
         reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~uintptr_t(1023));
     const uint32_t stage_bytes = kTcABytes + b_slab_bytes(a.nmma, a.b_mn);
@@ -222,10 +231,46 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
               "=r"(v[15])
             : "r"(addr));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (row >= a.M) continue;
         float f[16];
 #pragma unroll
         for (int j = 0; j < 16; j++) f[j] = fl ? fill : __uint_as_float(v[j]);
+        if constexpr (ACT) {
+            uint32_t pk[8];
+#pragma unroll
+            for (int j = 0; j < 16; j += 4) {
+                const float4 q = row < a.M ? *reinterpret_cast<const float4 *>(act.scale + (size_t)row * a.N + c0 + j)
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+                f[j] *= q.x;
+                f[j + 1] *= q.y;
+                f[j + 2] *= q.z;
+                f[j + 3] *= q.w;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+                pk[j] = *reinterpret_cast<const uint32_t *>(&b2);
+            }
+            if (row < a.M) {
+                uint4 *o = reinterpret_cast<uint4 *>(act.out + (size_t)row * a.N + c0);
+                o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+                o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+            }
+            // column sums over the warp's 32 rows: halve the columns a lane
+            // holds with each exchange, then add the last pair of lanes
+#pragma unroll
+            for (int w = 8; w > 0; w >>= 1) {
+                const bool up = lane & w;
+#pragma unroll
+                for (int j = 0; j < w; j++) {
+                    const float keep = up ? f[j + w] : f[j], send = up ? f[j] : f[j + w];
+                    f[j] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+                }
+            }
+            f[0] += __shfl_xor_sync(0xffffffffu, f[0], 16);
+            if (lane < 16) colsum[warp][c0 + lane] = f[0];
+            continue;
+        }
+        if (row >= a.M) continue;
         if (vec && c0 + 16 <= a.N) {
             float4 *o = reinterpret_cast<float4 *>(out + (size_t)row * a.ldo + c0);
 #pragma unroll
@@ -243,9 +288,35 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    if constexpr (ACT) {
+        for (int j = threadIdx.x; j < a.N; j += blockDim.x)
+            act.red[(size_t)blockIdx.x * a.N + j] = colsum[0][j] + colsum[1][j] + colsum[2][j] + colsum[3][j];
+    }
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(a.tmem_cols)
                      : "memory");
+}
+
+__global__ void __launch_bounds__(128, 1)
+k_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TcArgs a) {
+    gemm_tile<false>(tmA, tmB, a, ActArgs{});
+}
+
+// A product whose epilogue is the backward of an activation: no FP32 tile goes
+// to memory and back.
+__global__ void __launch_bounds__(128, 1)
+k_gemm_tc_act(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ TcArgs a,
+              ActArgs act) {
+    gemm_tile<true>(tmA, tmB, a, act);
+}
+
+// Two products of one K range side by side (gridDim.y = 2).
+__global__ void __launch_bounds__(128, 1)
+k_gemm_tc_pair(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmB0,
+               const __grid_constant__ TcArgs a0, const __grid_constant__ CUtensorMap tmA1,
+               const __grid_constant__ CUtensorMap tmB1, const __grid_constant__ TcArgs a1) {
+    if (blockIdx.y == 0) gemm_tile<false>(tmA0, tmB0, a0, ActArgs{});
+    else gemm_tile<false>(tmA1, tmB1, a1, ActArgs{});
 }
 
 // C (row stride ldo, or transposed) = sum over z of part[z][M][N], in z order.
@@ -304,7 +375,11 @@ bool ensure_attributes() {
     const uint64_t bit = 1ull << dev;
     if (done.load() & bit) return true;
     if (cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)gemm_tc_smem_bytes(256, 1)) != cudaSuccess)
+                             (int)gemm_tc_smem_bytes(256, 1)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_gemm_tc_act, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)gemm_tc_smem_bytes(kHidden, 0)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_gemm_tc_pair, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)gemm_tc_smem_bytes(kHidden, 1)) != cudaSuccess)
         return false;
     done.fetch_or(bit);
     return true;
@@ -343,6 +418,34 @@ int launch_gemm_tc(const uint16_t *A, int lda, int a_mn, const uint16_t *B, int 
     const dim3 grid((M + kTcBM - 1) / kTcBM, 1, splits);
     k_gemm_tc<<<grid, 128, gemm_tc_smem_bytes(N, b_mn), st>>>(ma, mb, t);
     if (splits > 1) k_splitk_sum_tc<<<(M * N + 255) / 256, 256, 0, st>>>(partial, splits, M, N, C, ldc, c_trans);
+    return cudaPeekAtLastError() == cudaSuccess ? 0 : -3;
+}
+
+int launch_gemm_tc_act(const uint16_t *dz2, const uint16_t *W2, int n, const float *g1, uint16_t *dz1, float *red1,
+                       cudaStream_t st) {
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, dz2, kHidden, n, kHidden, kTcBK, kTcBM) || !make_map(&mb, W2, kHidden, kHidden, kHidden, kTcBK, kHidden))
+        return -2;
+    if (!ensure_attributes()) return -3;
+    const TcArgs t{n, kHidden, kHidden, kHidden, kHidden, 0, 0, nullptr, 0, kHidden, 0, 128, nullptr};
+    k_gemm_tc_act<<<act_blocks(n), 128, gemm_tc_smem_bytes(kHidden, 0), st>>>(ma, mb, t, ActArgs{g1, dz1, red1});
+    return cudaPeekAtLastError() == cudaSuccess ? 0 : -3;
+}
+
+int launch_gemm_tc_step(const uint16_t *h1, const uint16_t *dz2, const uint16_t *dz1, const uint16_t *xn, int n,
+                        float *part2, float *part1, int *splits, cudaStream_t st) {
+    CUtensorMap a2, b2, a1, b1;
+    if (!make_map(&a2, h1, kHidden, n, kHidden, 64, kTcBK) || !make_map(&b2, dz2, kHidden, n, kHidden, 64, kTcBK) ||
+        !make_map(&a1, dz1, kHidden, n, kHidden, 64, kTcBK) || !make_map(&b1, xn, kFeatures, n, kFeatures, 64, kTcBK))
+        return -2;
+    if (!ensure_attributes()) return -3;
+    int kper = (n + *splits - 1) / *splits;
+    kper = (kper + kTcBK - 1) / kTcBK * kTcBK;
+    *splits = (n + kper - 1) / kper;
+    const TcArgs t2{kHidden, kHidden, kHidden, n, kper, 1, 1, part2, (size_t)kHidden * kHidden, kHidden, 0, 128, nullptr};
+    const TcArgs t1{kHidden, kFeatures, nmma_of(kFeatures, 1), n, kper, 1, 1, part1, (size_t)kHidden * kFeatures,
+                    kFeatures, 0, 64, nullptr};
+    k_gemm_tc_pair<<<dim3(1, 2, *splits), 128, gemm_tc_smem_bytes(kHidden, 1), st>>>(a2, b2, t2, a1, b1, t1);
     return cudaPeekAtLastError() == cudaSuccess ? 0 : -3;
 }
 

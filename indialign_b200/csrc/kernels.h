@@ -212,6 +212,30 @@ void launch_mlp_head_bwd(const MlpPacked *mlp, const float *dy, const float *z2,
                          float *red, float *grad, cudaStream_t st);
 void launch_mlp_act_bwd(const float *dh, const float *z, int n, uint16_t *dz, float *red, float *dbias,
                         cudaStream_t st);
+// One training step (k_learn.cu): the row-local part up to dz2, 64 rows a CTA,
+// and the finish (gradients from partial sums, Adam, packed copy).
+constexpr int kStepRed = 2 * kHidden + 4;  // per CTA: db2, dw3 columns, sum of dy, loss
+inline int step_blocks(int n) { return (n + 63) / 64; }
+inline int act_blocks(int n) { return (n + 127) / 128; }
+struct StepRows {
+    const float *x, *t;
+    int n;
+    float lambda;
+    float *y, *dy;
+    uint16_t *xn, *h1, *dz2;  // bf16 [n][16], [n][128] x 2
+    float *g1;                // [n][128] gelu'(z1)
+    float *red;               // [step_blocks][kStepRed]
+};
+struct StepFinish {
+    const float *part2, *part1;  // [splits][128][128], [splits][128][16]
+    const float *red, *red1;     // [blocks][kStepRed], [blocks1][128] (db1)
+    int splits, blocks, blocks1;
+    float *blob, *grad, *m, *v, *loss;
+    float lr, b1, b2, eps, bc1, bc2;
+};
+bool step_attributes();
+void launch_step_rows(const MlpPacked *mlp, const StepRows &a, cudaStream_t st);
+void launch_step_finish(const StepFinish &f, MlpPacked *out, cudaStream_t st);
 // k_tcgen05.cu: C[M][N] = A[M][K] . B[N][K]^T on the tcgen05 tensor cores,
 // BF16 in, FP32 out.  A is K-major ([M][lda], a_mn = 0) or MN-major
 // ([K][lda], a_mn = 1, M <= 128); B likewise with N (N <= 256); lda, ldb
@@ -221,6 +245,14 @@ void launch_mlp_act_bwd(const float *dh, const float *z, int n, uint16_t *dz, fl
 // Returns 0, -1 (arguments), -2 (tensor map) or -3 (launch).
 int launch_gemm_tc(const uint16_t *A, int lda, int a_mn, const uint16_t *B, int ldb, int b_mn, int M, int N,
                    int K, float *C, int ldc, int c_trans, float *partial, int splits, int *err, cudaStream_t st);
+// The step's two weight gradients in one launch, K = n rows split: partial
+// tiles of dW2 = h1^T dz2 ([128][128]) and of dW1^T = dz1^T xn ([128][16]).
+// *splits: the split count asked for, and used.  Returns as launch_gemm_tc.
+// dz1 = (dz2 . W2^T) g1 in BF16 with its column sums per 128 rows in red1.
+int launch_gemm_tc_act(const uint16_t *dz2, const uint16_t *W2, int n, const float *g1, uint16_t *dz1, float *red1,
+                       cudaStream_t st);
+int launch_gemm_tc_step(const uint16_t *h1, const uint16_t *dz2, const uint16_t *dz1, const uint16_t *xn, int n,
+                        float *part2, float *part1, int *splits, cudaStream_t st);
 void launch_adam(float *w, const float *g, float *m, float *v, int n, int first, float lr, float b1,
                  float b2, float eps, float bc1, float bc2, cudaStream_t st);
 

@@ -41,10 +41,10 @@ size_t save_bytes(int n) {
 
 constexpr int kSplitsMax = 64;
 // Work buffer: dz2 bf16 [n16][128] | dh1 f32 [n16][128] | dz1 bf16 [n16][128] | split-K partials |
-// row-block partial sums of the bias gradients
+// row-block partial sums of the bias gradients | a step's split-K partials of dW1 and per-CTA sums
 struct Work {
     uint16_t *dz2, *dz1;
-    float *dh1, *part, *red;
+    float *dh1, *part, *red, *part1, *step_red, *act_red;
 };
 Work work_view(void *base, int n) {
     const size_t r = rows16(n);
@@ -59,12 +59,20 @@ Work work_view(void *base, int n) {
     w.part = reinterpret_cast<float *>(p);
     p += up((size_t)kSplitsMax * kHidden * kHidden * 4);
     w.red = reinterpret_cast<float *>(p);
+    p += up((size_t)kBwdBlocksMax * kBwdRedStride * 4);
+    w.part1 = reinterpret_cast<float *>(p);
+    p += up((size_t)kSplitsMax * kHidden * kFeatures * 4);
+    w.step_red = reinterpret_cast<float *>(p);
+    p += up((size_t)step_blocks(n) * kStepRed * 4);
+    w.act_red = reinterpret_cast<float *>(p);
     return w;
 }
 size_t work_bytes(int n) {
     const size_t r = rows16(n);
     return up(r * kHidden * 2) + up(r * kHidden * 4) + up(r * kHidden * 2) +
-           up((size_t)kSplitsMax * kHidden * kHidden * 4) + up((size_t)kBwdBlocksMax * kBwdRedStride * 4);
+           up((size_t)kSplitsMax * kHidden * kHidden * 4) + up((size_t)kBwdBlocksMax * kBwdRedStride * 4) +
+           up((size_t)kSplitsMax * kHidden * kFeatures * 4) + up((size_t)step_blocks(n) * kStepRed * 4) +
+           up((size_t)act_blocks(n) * kHidden * 4);
 }
 
 // K splits of a weight-gradient GEMM (K = batch rows): >= 256 rows per split.
@@ -176,6 +184,32 @@ int indialign_mlp_adam(float *d_blob, const float *d_grad, float *d_m, float *d_
     launch_adam(d_blob, d_grad, d_m, d_v, kBlobSize, kBlobW1, lr, beta1, beta2, eps, bc1, bc2,
                 static_cast<cudaStream_t>(stream));
     return status("mlp_adam");
+}
+
+int indialign_mlp_step(float *d_blob, void *d_packed, const float *d_x, const float *d_t, int n, float lambda,
+                       float *d_y, float *d_dy, float *d_loss, float *d_grad, float *d_m, float *d_v, int step,
+                       float lr, float beta1, float beta2, float eps, void *d_save, void *d_work, void *stream) {
+    using namespace ia;
+    if (n <= 0 || step < 1 || !d_blob || !d_packed || !d_x || !d_t || !d_y || !d_dy || !d_loss || !d_grad || !d_m ||
+        !d_v || !d_save || !d_work)
+        return bad("mlp_step: null pointer, n <= 0 or step < 1");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const MlpSave sv = save_view(d_save, n);
+    const Work w = work_view(d_work, n);
+    if (!step_attributes()) return status("mlp_step");
+    const MlpPacked *mlp = static_cast<const MlpPacked *>(d_packed);
+    const uint16_t *W2 = reinterpret_cast<const uint16_t *>(reinterpret_cast<const char *>(mlp) +
+                                                            offsetof(MlpPacked, W2));
+    launch_step_rows(mlp, StepRows{d_x, d_t, n, lambda, d_y, d_dy, sv.xn, sv.h1, w.dz2, w.dh1, w.step_red}, st);
+    int splits = splits_for(n), rc = launch_gemm_tc_act(w.dz2, W2, n, w.dh1, w.dz1, w.act_red, st);
+    if (rc == 0) rc = launch_gemm_tc_step(sv.h1, w.dz2, w.dz1, sv.xn, n, w.part, w.part1, &splits, st);
+    if (rc != 0) return bad("mlp_step: tensor-core GEMM rejected its operands (alignment or tensor map)");
+    const float bc1 = (float)(1.0 - std::pow((double)beta1, step));
+    const float bc2 = (float)(1.0 - std::pow((double)beta2, step));
+    launch_step_finish(StepFinish{w.part, w.part1, w.step_red, w.act_red, splits, step_blocks(n), act_blocks(n), d_blob, d_grad, d_m, d_v, d_loss,
+                                  lr, beta1, beta2, eps, bc1, bc2},
+                       static_cast<MlpPacked *>(d_packed), st);
+    return status("mlp_step");
 }
 
 }  // extern "C"

@@ -122,14 +122,17 @@ class Trainer:
         return self.loss, self.grad
 
     def step(self, x, t):
-        loss, _ = self.gradients(x, t)
+        """One training step (forward, loss, gradients, Adam, repack) in one library call."""
+        n = int(x.shape[0])
+        assert n <= self.batch and x.dtype == self.torch.float32 and x.is_contiguous()
         self.steps += 1
-        f = ctypes.c_float
-        self._ck(self.lib.indialign_mlp_adam(self.blob.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(),
-                                             self.v.data_ptr(), self.steps, f(self.lr), f(self.beta1),
-                                             f(self.beta2), f(self.eps), self.stream), "mlp_adam")
-        self.pack()
-        return loss
+        self._ck(self.lib.indialign_mlp_step(self.blob.data_ptr(), self.packed.data_ptr(), x.data_ptr(), t.data_ptr(),
+                                             n, self.lam, self.y.data_ptr(), self.dy.data_ptr(),
+                                             self.loss.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(),
+                                             self.v.data_ptr(), self.steps, self.lr, self.beta1, self.beta2,
+                                             self.eps, self.save.data_ptr(), self.work.data_ptr(), self.stream),
+                 "mlp_step")
+        return self.loss
 
     def predict(self, x, chunk: int = 1 << 20):
         out = []
