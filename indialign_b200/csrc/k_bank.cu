@@ -40,6 +40,10 @@
 #ifndef IA_BANK_MINB
 #define IA_BANK_MINB 4
 #endif
+// ... and the items per CTA up to which a launch is "few items"
+#ifndef IA_BANK_WIDE
+#define IA_BANK_WIDE 64
+#endif
 
 
 namespace ia {
@@ -320,16 +324,165 @@ __global__ void __launch_bounds__(kBankChunk) k_bank_seeds(const BankTask *__res
     for (int a = 0; a < 3; a++) o[9 + a] = t[a];
 }
 
+// CTA-wide in-place conversion like points_to_f32, to one float4 per residue:
+// P {x, y, z, 1 if valid}, Q {x, y, z, 1} or NaN outside the mask (`out`); the
+// set is padded to a multiple of four with points that no cutoff selects.
+IA_DEV void points_to_f4(const double *src, float4 *dst, int n, const double *off, const uint8_t *V, bool out) {
+    for (int base = 0; base < n; base += kBankChunk) {
+        const int i = base + (int)threadIdx.x;
+        float4 v = make_float4(out ? NAN : 0.f, 0.f, 0.f, out ? 1.f : 0.f);
+        if (i < n && (V == nullptr || V[i] != 0 || !out)) {
+            v.x = (float)(src[3 * i] - off[0]);
+            v.y = (float)(src[3 * i + 1] - off[1]);
+            v.z = (float)(src[3 * i + 2] - off[2]);
+            v.w = out || V == nullptr || V[i] != 0 ? 1.f : 0.f;
+        }
+        __syncthreads();
+        if (i < ((n + 3) & ~3)) dst[i] = v;
+    }
+    __syncthreads();
+}
+
+// The items [.., ce) of a task by four lanes each, for launches of few items:
+// there a thread per item leaves the chip idle and the launch takes as long as
+// one thread's sweeps, 15 operations of distance and 15 of sums per residue in
+// turn.  The sums are the outer product (px, py, pz, 1) x (qx, qy, qz, 1): lane
+// a of an item holds its row a and adds four products per selected residue;
+// the distances of four residues go one to a lane.  Every sum still runs in
+// residue order (sp + p is fma(p, 1, sp)), so an item's numbers are the same
+// bits as in the thread-per-item loop.  It issues 1.6 times the instructions
+// per residue and item and solves 8 systems per warp instead of 32, so the line
+// lies at 64 items per resident CTA (IA_BANK_WIDE): k_bank's launches on one
+// pair of 64 residues 0.70 -> 0.65 ms, of 1203 residues 6.8 -> 5.0; with the line
+// at 128, a learned search of 61 pairs loses 0.9 of 10.9 ms.
+IA_DEV void wide_items(const BankTask &T, const float4 *P4, const float4 *Q4, const double *oP, const double *oQ,
+                       const double *__restrict__ seed_rt, double *__restrict__ item_res, int *s_next, int ce,
+                       unsigned long long *ctr) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const int lane = threadIdx.x & 31, a = lane & 3, g0 = lane & 28, n = T.n, C = T.C > 0 ? T.C : 1;
+    const float *Pa = reinterpret_cast<const float *>(P4) + a;
+    for (;;) {
+        int gi = 0;
+        if (lane == 0) gi = atomicAdd(s_next, 8);
+        gi = __shfl_sync(kFull, gi, 0);
+        if (gi >= ce) break;
+        const int pi = gi + (lane >> 2);
+        const bool active = pi < ce;
+        int sk = 0, ci = 0;
+        if (active) {
+            const int K = T.n_items / C;
+            sk = T.cutoff_major ? pi % K : pi / C;
+            ci = T.cutoff_major ? pi / K : pi % C;
+        }
+        const double cut = T.cut[ci];
+        const float cut2 = (float)(cut * cut);
+        double R[9], t[3];
+        const double *o = seed_rt + 12 * ((size_t)(T.item_base / kDetC) + sk);
+#pragma unroll
+        for (int k = 0; k < 9; k++) R[k] = o[k];
+#pragma unroll
+        for (int k = 0; k < 3; k++) t[k] = o[9 + k];
+        float Rf[9], tf[3];
+        auto round_rt = [&]() {
+#pragma unroll
+            for (int k = 0; k < 9; k++) Rf[k] = (float)R[k];
+#pragma unroll
+            for (int k = 0; k < 3; k++) tf[k] = (float)t[k];
+        };
+        bool running = active && T.max_iter > 0;
+        int prev = -1, iter = 0;
+        while (__any_sync(kFull, running)) {
+            round_rt();
+            const float lim = running ? cut2 : -1.f;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int base = 0; base < n; base += 4) {
+                const unsigned in = __ballot_sync(kFull, dist2_f32(P4[base + a], Q4[base + a], Rf, tf) <= lim) >> g0;
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const float u = Pa[4 * (base + r)];
+                    const float4 v = Q4[base + r];
+                    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t@p fma.rn.f32 %0, %5, %6, %0;\n\t"
+                        "@p fma.rn.f32 %1, %5, %7, %1;\n\t@p fma.rn.f32 %2, %5, %8, %2;\n\t"
+                        "@p fma.rn.f32 %3, %5, %9, %3;\n\t}"
+                        : "+f"(acc.x), "+f"(acc.y), "+f"(acc.z), "+f"(acc.w)
+                        : "r"(in & (1u << r)), "f"(u), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+                }
+            }
+            MomentsF m;
+#pragma unroll
+            for (int r = 0; r < 3; r++) {
+                m.h[3 * r] = __shfl_sync(kFull, acc.x, g0 + r);
+                m.h[3 * r + 1] = __shfl_sync(kFull, acc.y, g0 + r);
+                m.h[3 * r + 2] = __shfl_sync(kFull, acc.z, g0 + r);
+                m.sp[r] = __shfl_sync(kFull, acc.w, g0 + r);
+            }
+            m.sq[0] = __shfl_sync(kFull, acc.x, g0 + 3);
+            m.sq[1] = __shfl_sync(kFull, acc.y, g0 + 3);
+            m.sq[2] = __shfl_sync(kFull, acc.z, g0 + 3);
+            m.w = (int)__shfl_sync(kFull, acc.w, g0 + 3);
+            if (running) {
+                if (m.w >= 3) m.kabsch(R, t);
+                ++iter;
+                if (m.w == prev || iter >= T.max_iter) running = false;
+                prev = m.w;
+            }
+        }
+        // the compensated sum runs in residue order on every lane of the item,
+        // over terms computed one to a lane
+        round_rt();
+        const float inv_d0sq = (float)(1.0 / fmax(T.d0 * T.d0, 1e-12)), sd8sq = (float)(T.sd8 * T.sd8);
+        float sum = 0.f, comp = 0.f;
+        for (int base = 0; base < n; base += 4) {
+            const float4 p = P4[base + a];
+            const float d2 = dist2_f32(p, Q4[base + a], Rf, tf);
+            const unsigned in = __ballot_sync(kFull, p.w != 0.f && (!T.use_d8 || d2 <= sd8sq)) >> g0;
+            const float term = __frcp_rn(fmaf(d2, inv_d0sq, 1.0f));
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const float y = __shfl_sync(kFull, term, g0 + r) - comp, s2 = sum + y;
+                if (in & (1u << r)) {
+                    comp = (s2 - sum) - y;
+                    sum = s2;
+                }
+            }
+        }
+        unsigned long long visits = active && a == 0 ? (unsigned long long)(iter + 1) * n : 0ull;
+        unsigned long long items = active && a == 0 ? 1ull : 0ull;
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) {
+            visits += __shfl_xor_sync(kFull, visits, k);
+            items += __shfl_xor_sync(kFull, items, k);
+        }
+        if (lane == 0) {
+            atomicAdd(ctr + CTR_BANK_RES, visits);
+            atomicAdd(ctr + CTR_BANK_ITEMS, items);
+        }
+        if (active && a == 0) {
+            double *rec = item_res + (size_t)(T.item_base + sk * C + ci) * kRec;
+            rec[0] = (double)sum / fmax(T.lnorm, 1.0);
+#pragma unroll
+            for (int k = 0; k < 9; k++) rec[1 + k] = R[k];
+#pragma unroll
+            for (int k = 0; k < 3; k++)
+                rec[10 + k] = t[k] + oQ[k] - (oP[0] * R[k] + oP[1] * R[3 + k] + oP[2] * R[6 + k]);
+        }
+    }
+}
+
+// CTAs pull chunks of one task's items; their warps take them 32 at a time (8 in
+// a launch of at most wide_max items, see wide_items).
 template <bool SMEM>
 __global__ void __launch_bounds__(kBankChunk, IA_BANK_MINB)
 k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
        int ntasks, const ScanOut *__restrict__ scan, int *counter,
-       const double *__restrict__ seed_rt, double *__restrict__ item_res, int *err, int nmax, unsigned long long *ctr) {
+       const double *__restrict__ seed_rt, double *__restrict__ item_res, int *err, int nmax, int wide_max,
+       unsigned long long *ctr) {
     extern __shared__ __align__(16) char smem[];
     __shared__ BankSmem ctl;
     __shared__ uint64_t bar;
     __shared__ double oP[3], oQ[3], red[6 * (kBankChunk / 32)];  // point-set means
-    __shared__ int s_next;  // next group of 32 items of the chunk
+    __shared__ int s_next;  // next item of the chunk
     // layout: P[nmax*3] Q[nmax*3] (each +16 B lead room), V, PV, NV bytes
     // room for a 15-byte lead and the rounded-up tail of a bulk copy
     const uint32_t coord_bytes = ((uint32_t)nmax * 24u + 47u) & ~15u;
@@ -340,6 +493,7 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
     if (threadIdx.x == 0) mbar_init(&bar);
     __syncthreads();
     const int total = scan->total_chunks;
+    const bool wide = SMEM && scan->items <= wide_max;
     int staged = -1;
     const float4 *Pf = nullptr, *Qf = nullptr;  // shared FP32 copies (SMEM)
     const double *Pd = nullptr, *Qd = nullptr;  // global FP64 arrays (!SMEM)
@@ -382,8 +536,13 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
                 points_mean(dQ, n, oQ, red);
                 int k = 2;
                 V = T.V ? reinterpret_cast<const uint8_t *>(sV + cp[k++].lead) : nullptr;
-                points_to_f32(dP, reinterpret_cast<float4 *>(sP), n, oP, V, false);
-                points_to_f32(dQ, reinterpret_cast<float4 *>(sQ), n, oQ, V, true);
+                if (wide) {
+                    points_to_f4(dP, reinterpret_cast<float4 *>(sP), n, oP, V, false);
+                    points_to_f4(dQ, reinterpret_cast<float4 *>(sQ), n, oQ, V, true);
+                } else {
+                    points_to_f32(dP, reinterpret_cast<float4 *>(sP), n, oP, V, false);
+                    points_to_f32(dQ, reinterpret_cast<float4 *>(sQ), n, oQ, V, true);
+                }
                 Pf = reinterpret_cast<const float4 *>(sP);
                 Qf = reinterpret_cast<const float4 *>(sQ);
                 PV = T.PV ? reinterpret_cast<const uint8_t *>(sPV + cp[k++].lead) : nullptr;
@@ -395,12 +554,16 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
             }
             staged = ti;
         }
-        // the chunk's items [cb, ce) go to the warps 32 at a time, so a warp
+        const int ce = min(((c - chunk_begin[ti]) + 1) * T.chunk, T.n_items);  // the chunk's end
+        const int lane = threadIdx.x & 31;
+        if (wide) {
+            if constexpr (SMEM) wide_items(T, Pf, Qf, oP, oQ, seed_rt, item_res, &s_next, ce, ctr);
+            __syncthreads();
+            continue;
+        }
+        // the chunk's items go to the warps 32 at a time, so a warp
         // whose items converged early takes the next group instead of
         // waiting at the chunk's barrier for the others
-        const int cb = (c - chunk_begin[ti]) * T.chunk;
-        const int ce = min(cb + T.chunk, T.n_items);
-        const int lane = threadIdx.x & 31;
         for (;;) {
         int gi = 0;
         if (lane == 0) gi = atomicAdd(&s_next, 32);
@@ -567,38 +730,59 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
 // last seed processed is therefore k* = the first seed holding an item
 // >= early_term; every earlier item is below early_term, so the result is the
 // first maximum over the items of seeds 0..k*.
-__global__ void k_reduce_bank(const BankTask *__restrict__ tasks, int ntasks,
+// `width` threads per task: a warp where tasks are many and short (threading
+// offsets), else the CTA, whose loads over a long item list then overlap.
+__global__ void __launch_bounds__(128) k_reduce_bank(const BankTask *__restrict__ tasks, int ntasks, int width,
                               const double *__restrict__ item_res,
                               PairState *__restrict__ state) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
+    constexpr unsigned kFull = 0xffffffffu;
+    __shared__ double s_d[4];
+    __shared__ int s_i[4], s_k[4];
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) / width;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, me = threadIdx.x % width;
+    const bool cta = width > 32;  // w is then uniform over the CTA
     if (w >= ntasks) return;
     const BankTask &T = tasks[w];
     if (T.n_items <= 0) return;
     const int C = T.C > 0 ? T.C : 1;
     const double *base = item_res + (size_t)T.item_base * kRec;
-    int end = T.n_items;
-    if (T.early_term < 1e30) {
-        int kst = 0x7fffffff;
-        for (int i = lane; i < T.n_items; i += 32)
-            if (base[(size_t)i * kRec] >= T.early_term) kst = min(kst, i / C);
+    // first maximum of items [0, end) and the first seed holding an item >= early_term
+    auto first_max = [&](int end, double &bs, int &bi, int &kst) {
+        bs = kScoreInit;
+        bi = -1;
+        kst = 0x7fffffff;
+#pragma unroll 4
+        for (int i = me; i < end; i += width) {
+            const double s = base[(size_t)i * kRec];
+            if (s >= T.early_term) kst = min(kst, i / C);
+            if (s > bs) { bs = s; bi = i; }  // thread-local: ascending i, strict >
+        }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) kst = min(kst, __shfl_xor_sync(0xffffffffu, kst, o));
-        if (kst != 0x7fffffff) end = min(end, (kst + 1) * C);
-    }
-    double bs = kScoreInit;
-    int bi = -1;
-    for (int i = lane; i < end; i += 32) {
-        double s = base[(size_t)i * kRec];
-        if (s > bs) { bs = s; bi = i; }  // lane-local: ascending i, strict >
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double s2 = __shfl_xor_sync(0xffffffffu, bs, o);
-        int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
-        bool take = (s2 > bs) || (s2 == bs && i2 >= 0 && (bi < 0 || i2 < bi));
-        if (take) { bs = s2; bi = i2; }
-    }
+        for (int o = 16; o > 0; o >>= 1) {
+            const double s2 = __shfl_xor_sync(kFull, bs, o);
+            const int i2 = __shfl_xor_sync(kFull, bi, o);
+            kst = min(kst, __shfl_xor_sync(kFull, kst, o));
+            if ((s2 > bs) || (s2 == bs && i2 >= 0 && (bi < 0 || i2 < bi))) { bs = s2; bi = i2; }
+        }
+        if (!cta) return;
+        __syncthreads();
+        if (lane == 0) {
+            s_d[warp] = bs;
+            s_i[warp] = bi;
+            s_k[warp] = kst;
+        }
+        __syncthreads();
+        for (int k = 0; k < 4; k++) {
+            const double s2 = s_d[k];
+            const int i2 = s_i[k];
+            kst = min(kst, s_k[k]);
+            if ((s2 > bs) || (s2 == bs && i2 >= 0 && (bi < 0 || i2 < bi))) { bs = s2; bi = i2; }
+        }
+    };
+    double bs;
+    int bi, kst;
+    first_max(T.n_items, bs, bi, kst);
+    if (T.early_term < 1e30 && kst != 0x7fffffff && (kst + 1) * C < T.n_items) first_max((kst + 1) * C, bs, bi, kst);
     // the winner's score in FP64 over the task's own point set (the items
     // were scored in FP32): the same formula as k_bank's score pass
     double score = kScoreInit;
@@ -611,20 +795,27 @@ __global__ void k_reduce_bank(const BankTask *__restrict__ tasks, int ntasks,
         for (int a = 0; a < 3; a++) t[a] = rec[10 + a];
         const double d0sq = fmax(T.d0 * T.d0, 1e-12), sd8sq = T.sd8 * T.sd8;
         double sum = 0.0;
-        for (int i = lane; i < T.n; i += 32) {
+        for (int i = me; i < T.n; i += width) {
             if (T.V && T.V[i] == 0) continue;
             const double d2 = dist2(R, t, T.P[3 * i], T.P[3 * i + 1], T.P[3 * i + 2], T.Q[3 * i], T.Q[3 * i + 1],
                                     T.Q[3 * i + 2]);
             if (!T.use_d8 || d2 <= sd8sq) sum += 1.0 / (1.0 + d2 / d0sq);
         }
-        score = warp_sum(sum) / fmax(T.lnorm, 1.0);
+        sum = warp_sum(sum);
+        if (cta) {
+            __syncthreads();
+            if (lane == 0) s_d[warp] = sum;
+            __syncthreads();
+            sum = (s_d[0] + s_d[1]) + (s_d[2] + s_d[3]);
+        }
+        score = sum / fmax(T.lnorm, 1.0);
     }
     double *out = T.out_rec >= 0 ? state[T.pair].rec[T.out_rec] : T.out;
-    if (lane < kRec) {
+    if (me < kRec) {
         double v;
-        if (bi >= 0) v = lane == 0 ? score : base[(size_t)bi * kRec + lane];
-        else v = lane == 0 ? kScoreInit : ((lane == 1 || lane == 5 || lane == 9) ? 1.0 : 0.0);
-        out[lane] = v;
+        if (bi >= 0) v = me == 0 ? score : base[(size_t)bi * kRec + me];
+        else v = me == 0 ? kScoreInit : ((me == 1 || me == 5 || me == 9) ? 1.0 : 0.0);
+        out[me] = v;
     }
 }
 
@@ -638,6 +829,8 @@ size_t bank_smem_bytes(int nmax) {
 void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks,
                  const ScanOut *scan, int *counter, double *seed_rt, int seed_blocks, double *item_res, int *err,
                  int nmax, int grid, unsigned long long *ctr, cudaStream_t st) {
+    // offset items (no seeds) sum their starts in the thread-per-item form
+    const int wide_max = seed_blocks > 0 ? IA_BANK_WIDE * grid : 0;
     if (seed_blocks > 0) {
         const size_t ss = (size_t)nmax * 2 * sizeof(float4);
         const dim3 g(ntasks, seed_blocks);
@@ -647,18 +840,18 @@ void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks,
     size_t sm = bank_smem_bytes(nmax);
     if (sm <= kBankSmemMax) {
         k_bank<true><<<grid, kBankChunk, sm, st>>>(tasks, chunk_begin, ntasks, scan, counter,
-                                                   seed_rt, item_res, err, nmax, ctr);
+                                                   seed_rt, item_res, err, nmax, wide_max, ctr);
     } else {
         k_bank<false><<<grid, kBankChunk, 0, st>>>(tasks, chunk_begin, ntasks, scan, counter,
-                                                   seed_rt, item_res, err, nmax, ctr);
+                                                   seed_rt, item_res, err, nmax, wide_max, ctr);
     }
 }
 
-void launch_reduce_bank(const BankTask *tasks, int ntasks, const double *item_res,
+void launch_reduce_bank(const BankTask *tasks, int ntasks, bool short_lists, const double *item_res,
                         PairState *state, cudaStream_t st) {
     if (ntasks <= 0) return;
-    int threads = 256, blocks = (ntasks * 32 + threads - 1) / threads;
-    k_reduce_bank<<<blocks, threads, 0, st>>>(tasks, ntasks, item_res, state);
+    const int width = short_lists ? 32 : 128, per = 128 / width;
+    k_reduce_bank<<<(ntasks + per - 1) / per, 128, 0, st>>>(tasks, ntasks, width, item_res, state);
 }
 
 const void *bank_kernel_ptr(bool smem) {

@@ -778,6 +778,8 @@ __global__ void k_scan(const int *counts, int *begins, int ntasks, ScanOut *out,
     }
     if (threadIdx.x == 0) {
         out->total_chunks = carry;
+        out->items = out->items_acc;
+        out->items_acc = 0;
         *counter = 0;
     }
 }

@@ -153,6 +153,9 @@ __global__ void k_plan_bank(DevBatch b, PlanCtx c) {
     T.cutoff_major = tn.bank_cutoff_major;
     c.btasks[s] = T;
     c.counts[s] = (T.n_items + T.chunk - 1) / T.chunk;
+    const unsigned together = __activemask();
+    const int items = __reduce_add_sync(together, T.n_items);
+    if (items > 0 && (threadIdx.x & 31) == __ffs(together) - 1) atomicAdd(&c.scan->items_acc, items);
 }
 
 // ---- chain plans ------------------------------------------------------------

@@ -86,7 +86,7 @@ size_t bank_smem_bytes(int nmax);
 void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks, const ScanOut *scan,
                  int *counter, double *seed_rt, int seed_blocks, double *item_res, int *err, int nmax, int grid,
                  unsigned long long *ctr, cudaStream_t st);
-void launch_reduce_bank(const BankTask *tasks, int ntasks, const double *item_res,
+void launch_reduce_bank(const BankTask *tasks, int ntasks, bool short_lists, const double *item_res,
                         PairState *state, cudaStream_t st);
 cudaError_t bank_set_attributes();
 const void *bank_kernel_ptr(bool smem);

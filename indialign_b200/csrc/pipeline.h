@@ -157,6 +157,13 @@ enum GlueOp {
     G_EXTRA_START, G_FLAG_ON, G_OFFDP_UPDATE
 };
 
+struct ScanOut {
+    int total_chunks;
+    int error;           // device-side error flags (bounded waits, caps)
+    int items;           // a bank launch's items
+    int items_acc;       // ... while its plan kernel counts them
+};
+
 struct PlanCtx {
     int kind, ntasks;
     const int *pair;        // slot -> pair (nullptr: slot == pair)
@@ -165,6 +172,7 @@ struct PlanCtx {
     BankTask *btasks;
     ChainTask *ctasks;
     int *counts;            // slot -> work chunks
+    ScanOut *scan;          // the plan adds up a bank launch's items here
     double *alP, *alQ;      // aligned sets (2 per pair)
     double *chain_res;      // LITE chain results
     double *recs, *recs2;   // stage record arrays (threading det, offset starts/results)
@@ -181,11 +189,6 @@ struct GlueArgs {
     int dp_iter;
     const double *recs;
     const int *idx;         // per pair first record of `recs`
-};
-
-struct ScanOut {
-    int total_chunks;
-    int error;           // device-side error flags (bounded waits, caps)
 };
 
 // ---- learned window ranker ---------------------------------------------------

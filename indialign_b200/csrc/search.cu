@@ -539,6 +539,7 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
     pc.aux = L.d_aux;
     pc.base = L.d_base;
     pc.btasks = c_->btasks.p;
+    pc.scan = c_->scan.p;
     pc.counts = c_->counts.p;
     pc.alP = c_->alP.p;
     pc.alQ = c_->alQ.p;
@@ -556,10 +557,9 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
     const int grid = c_->sms * per_sm;
     // a launch that cannot fill the grid with 256-item chunks takes 128, one
     // group of 32 per warp: its time is the longest warp's, and a second group
-    // would come on top (one 64-residue pair: 0.73 against 1.02 ms
-    // over its nine launches; with more items the two measure the same)
-    if (L.total <= 256LL * grid)
-        for (Tune &t : pc.tune.t) t.bank_chunk = std::min(t.bank_chunk, kBankChunk);
+    // would come on top; one of few items 32, one group of 8 per warp
+    const int most = L.total <= 32LL * grid ? 32 : L.total <= 256LL * grid ? kBankChunk : 4096;
+    for (Tune &t : pc.tune.t) t.bank_chunk = std::min(t.bank_chunk, most);
     launch_plan_bank(b, pc, c_->stream);
     launch_scan(c_->counts.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->stream);
     launches_ += kind == BK_GAPLESS ? 4 : 5;
@@ -583,7 +583,7 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
         cudaEventRecord(e1, c_->stream);
         bank_ev.push_back({e0, e1});
     }
-    launch_reduce_bank(c_->btasks.p, L.ntasks, c_->item_res.p, b.state, c_->stream);
+    launch_reduce_bank(c_->btasks.p, L.ntasks, kind == BK_THREAD, c_->item_res.p, b.state, c_->stream);
     CK(cudaGetLastError());
     return INDIALIGN_OK;
 }
