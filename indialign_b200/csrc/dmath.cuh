@@ -117,6 +117,21 @@ IA_DEV double rcp_nr(double x) {
     return fma(y, e, y);
 }
 
+// One more step: the residual of a reciprocal within an ulp is exact, so the
+// result rounds like 1 / x.  A dependent chain of ~80 cycles against ~380 of the
+// division operator, whose path is also twice as many instructions.
+IA_DEV double rcp_cr(double x) {
+    const double y = rcp_nr(x);
+    return fma(fma(-x, y, 1.0), y, y);
+}
+
+// A residue's TM term 1 / (1 + d2 / d0^2) for inv = 1 / d0^2; 0 for an infinite
+// distance, NaN for a NaN one.
+IA_DEV double tm_term(double d2, double inv) {
+    const double x = fma(d2, inv, 1.0);
+    return x == INFINITY ? 0.0 : rcp_cr(x);
+}
+
 // a / b for y = 1 / b correctly rounded: Markstein's final step (a quotient
 // within an ulp, its exact residual, one fused correction) rounds like the
 // division itself, so six quotients by one divisor cost one division.  The
@@ -240,8 +255,12 @@ IA_DEV bool qcp_rotation(const double (&H)[3][3], double *R) {
         c0 = a00 * (a11 * b1 - a12 * b2 + a13 * b3) - a01 * (a01 * b1 - a02 * b2 + a03 * b3) +
              a02 * (a01 * b2 - a02 * d1 + a03 * d2) - a03 * (a01 * b3 - a02 * d2 + a03 * d3);
     }
-    const double scale = sqrt(p2);
-    double l1 = 0.8660254037844387 * scale;
+    // sqrt(p2) to a few parts in 1e7: it starts the iteration, from just above
+    // the bound, and scales the thresholds
+    double scale;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(scale) : "d"(p2));
+    scale *= p2;
+    double l1 = 0.86603 * scale;
 #pragma unroll 1
     for (int it = 0; it < 64; it++) {
         const double x2 = l1 * l1;
@@ -350,6 +369,44 @@ struct Moments {
         h[6] += wz * qx; h[7] += wz * qy; h[8] += wz * qz;
         w += wi;
     }
+    // Sum over the 32 lanes, the total on every lane: exchanges that halve the
+    // sums a lane carries, then one broadcast each, 34 exchanges instead of the
+    // butterfly's 80 (and 16 additions instead of 80), in the butterfly's order
+    // of additions.
+    IA_DEV void warp_total() {
+        const int lane = threadIdx.x & 31;
+        double a[16];
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            a[i] = sp[i];
+            a[3 + i] = sq[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 9; i++) a[6 + i] = h[i];
+        a[15] = w;
+#pragma unroll
+        for (int o = 1, k = 8; k > 0; o <<= 1, k >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int i = 0; i < k; i++) {
+                const double keep = up ? a[i + k] : a[i], send = up ? a[i] : a[i + k];
+                a[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        a[0] += __shfl_xor_sync(0xffffffffu, a[0], 16);
+        // sum i stands on the lane whose low bits are i's four bits reversed
+        auto get = [&](int i) {
+            return __shfl_sync(0xffffffffu, a[0], (i >> 3 & 1) | (i >> 1 & 2) | (i << 1 & 4) | (i << 3 & 8));
+        };
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            sp[i] = get(i);
+            sq[i] = get(3 + i);
+        }
+#pragma unroll
+        for (int i = 0; i < 9; i++) h[i] = get(6 + i);
+        w = get(15);
+    }
     // Butterfly sum over the lanes of `width` (power of two) so that every
     // lane of the group ends with the group total.
     IA_DEV void group_sum(int width) {
@@ -375,7 +432,7 @@ static __device__ __noinline__ void kabsch_from_moments(const Moments &m, double
         return;
     }
     double cP[3], cQ[3], H[3][3];
-    const double inv_w = 1.0 / m.w;
+    const double inv_w = rcp_cr(m.w);
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         cP[d] = div_by(m.sp[d], m.w, inv_w);
@@ -418,7 +475,7 @@ IA_DEV void warp_kabsch_window(const Pts &x, int a, int b, int cnt, double *R, d
         const double *p = x.P + 3 * (a + i), *q = x.Q + 3 * (b + i);
         m.add(p[0], p[1], p[2], q[0], q[1], q[2]);
     }
-    m.group_sum(32);
+    m.warp_total();
     kabsch_from_moments(m, 3.0, R, t);
 }
 

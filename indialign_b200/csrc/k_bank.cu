@@ -793,13 +793,13 @@ __global__ void __launch_bounds__(128) k_reduce_bank(const BankTask *__restrict_
         for (int a = 0; a < 9; a++) R[a] = rec[1 + a];
 #pragma unroll
         for (int a = 0; a < 3; a++) t[a] = rec[10 + a];
-        const double d0sq = fmax(T.d0 * T.d0, 1e-12), sd8sq = T.sd8 * T.sd8;
+        const double inv = 1.0 / fmax(T.d0 * T.d0, 1e-12), sd8sq = T.sd8 * T.sd8;
         double sum = 0.0;
         for (int i = me; i < T.n; i += width) {
             if (T.V && T.V[i] == 0) continue;
             const double d2 = dist2(R, t, T.P[3 * i], T.P[3 * i + 1], T.P[3 * i + 2], T.Q[3 * i], T.Q[3 * i + 1],
                                     T.Q[3 * i + 2]);
-            if (!T.use_d8 || d2 <= sd8sq) sum += 1.0 / (1.0 + d2 / d0sq);
+            if (!T.use_d8 || d2 <= sd8sq) sum += tm_term(d2, inv);
         }
         sum = warp_sum(sum);
         if (cta) {

@@ -230,15 +230,15 @@ IA_DEV double aligned_kabsch(const Pts &x, const uint32_t *al, int na, double d0
         const double *p = x.P + 3 * pi, *q = x.Q + 3 * ni;
         m.add(p[0], p[1], p[2], q[0], q[1], q[2]);
     }
-    m.group_sum(32);
+    m.warp_total();
     kabsch_from_moments(m, 3.0, R, t);
-    const double d0sq = fmax(d0 * d0, 1e-12);
+    const double inv = 1.0 / fmax(d0 * d0, 1e-12);
     double s = 0.0;
     for (int k = lane; k < na; k += 32) {
         int pi, ni;
         al_get(al, na, k, pi, ni);
         const double *p = x.P + 3 * pi, *q = x.Q + 3 * ni;
-        s += 1.0 / (1.0 + dist2(R, t, p[0], p[1], p[2], q[0], q[1], q[2]) / d0sq);
+        s += tm_term(dist2(R, t, p[0], p[1], p[2], q[0], q[1], q[2]), inv);
     }
     return warp_sum(s) / fmax(lnorm, 1.0);
 }
@@ -289,7 +289,7 @@ IA_NW_ATTR double lite_detailed(const Pts &x, const uint32_t *al, int na, const 
     }
     // residue visits: each active group ran `iter` passes + 1 score pass
     if (sub == 0 && grp) atomicAdd(ctr + CTR_CHAIN_RES, (unsigned long long)(iter + 1) * na);
-    const double d0sq = fmax(d0 * d0, 1e-12), sd8sq = sd8 * sd8;
+    const double inv = 1.0 / fmax(d0 * d0, 1e-12), sd8sq = sd8 * sd8;
     double s = 0.0;
     if (grp) {
         for (int k = sub; k < na; k += 4) {
@@ -297,7 +297,7 @@ IA_NW_ATTR double lite_detailed(const Pts &x, const uint32_t *al, int na, const 
             al_get(al, na, k, pi, ni);
             const double *p = x.P + 3 * pi, *q = x.Q + 3 * ni;
             double d2 = dist2(R, t, p[0], p[1], p[2], q[0], q[1], q[2]);
-            if (d2 <= sd8sq) s += 1.0 / (1.0 + d2 / d0sq);
+            if (d2 <= sd8sq) s += tm_term(d2, inv);
         }
     }
     s += __shfl_xor_sync(kFull, s, 1);

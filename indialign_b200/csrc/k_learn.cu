@@ -198,8 +198,29 @@ IA_DEV void mlp_tile(const MlpSmem &S, const float *xt, float &y_g, float &y_g8,
     y_g8 = y8 + S.b3;
 }
 
+// Eight sums over the warp, each total on every lane, in the butterfly's order
+// of additions: 17 exchanges instead of 40.
+IA_DEV void warp_sum8(double (&a)[8]) {
+    const int lane = threadIdx.x & 31;
+    // levels 16, 8 and 4 halve the sums a lane carries, 2 and 1 add plainly
+#pragma unroll
+    for (int o = 16, k = 4; o > 2; o >>= 1, k >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < k; i++) {
+            const double keep = up ? a[i + k] : a[i], send = up ? a[i] : a[i + k];
+            a[i] = keep + __shfl_xor_sync(kAllLanes, send, o);
+        }
+    }
+    double t = a[0];
+    t += __shfl_xor_sync(kAllLanes, t, 2);
+    t += __shfl_xor_sync(kAllLanes, t, 1);
+#pragma unroll
+    for (int i = 0; i < 8; i++) a[i] = __shfl_sync(kAllLanes, t, (i >> 2 & 1) * 16 + (i >> 1 & 1) * 8 + (i & 1) * 4);
+}
+
 // The 16 features of candidate w of a pair (raw, before standardisation),
-// computed by the whole warp; every lane returns all 16.
+// computed by the whole warp; lane j < 16 returns feature j.
 //   0 segment length / ml         1 pred start / (plen-1)   2 native start / (nlen-1)
 //   3 start shift / ml            4 segment RMSD / 10       5 TM along the segment's
 //   diagonal under its Kabsch     6, 7 fraction of that diagonal within d0, 2 d0
@@ -209,8 +230,8 @@ IA_DEV void mlp_tile(const MlpSmem &S, const float *xt, float &y_g, float &y_g8,
 // (ml = min(plen, nlen); indices are compact valid-residue positions.)
 // Detailed-search seeds are segments of an aligned set (plen == nlen == the
 // aligned count, SS labels absent: stem fractions 0).
-IA_DEV void window_features(const Pts &x, const uint8_t *Lp, const uint8_t *Ln, const PairInfo &I,
-                            int plen, int nlen, double best, int kind, int w, float (&f)[kFeatures]) {
+IA_DEV float window_features(const Pts &x, const uint8_t *Lp, const uint8_t *Ln, const PairInfo &I,
+                             int plen, int nlen, double best, double log_ml, int kind, int w) {
     const int lane = threadIdx.x & 31;
     const int ml = plen < nlen ? plen : nlen;
     int flen, ps, ns;
@@ -235,7 +256,7 @@ IA_DEV void window_features(const Pts &x, const uint8_t *Lp, const uint8_t *Ln, 
             const double *q = x.Q + 3 * (i + s);
             const double dx = mx - q[0], dy = my - q[1], dz = mz - q[2];
             const double d2 = dx * dx + dy * dy + dz * dz;
-            const double term = 1.0 / (1.0 + d2 * inv);
+            const double term = tm_term(d2, inv);
             dtm += term;
             c1 += d2 < d0sq ? 1.0 : 0.0;
             c2 += d2 < 4.0 * d0sq ? 1.0 : 0.0;
@@ -251,34 +272,35 @@ IA_DEV void window_features(const Pts &x, const uint8_t *Lp, const uint8_t *Ln, 
         if (i < ml) {
             const double *q = x.Q + 3 * i;
             const double dx = mx - q[0], dy = my - q[1], dz = mz - q[2];
-            tm0 += 1.0 / (1.0 + (dx * dx + dy * dy + dz * dz) * inv);
+            tm0 += tm_term(dx * dx + dy * dy + dz * dz, inv);
         }
     }
-    sd2 = warp_sum(sd2);
-    stm = warp_sum(stm);
-    sp = warp_sum(sp);
-    sn = warp_sum(sn);
-    dtm = warp_sum(dtm);
-    c1 = warp_sum(c1);
-    c2 = warp_sum(c2);
-    tm0 = warp_sum(tm0);
-    const double mld = (double)ml, rmsd = sqrt(sd2 / flen);
-    f[0] = (float)(flen / mld);
-    f[1] = (float)(ps / (double)(plen > 1 ? plen - 1 : 1));
-    f[2] = (float)(ns / (double)(nlen > 1 ? nlen - 1 : 1));
-    f[3] = (float)(s / mld);
-    f[4] = (float)(rmsd / 10.0);
-    f[5] = (float)(dtm / I.lnorm);
-    f[6] = (float)(c1 / mld);
-    f[7] = (float)(c2 / mld);
-    f[8] = (float)(stm / flen);
-    f[9] = (float)(sp / flen);
-    f[10] = (float)(sn / flen);
-    f[11] = (float)(log(mld) / 7.0);
-    f[12] = (float)best;
-    f[13] = 0.5f * (float)kind;
-    f[14] = (float)(fmin(rmsd / I.d0, 10.0) / 10.0);
-    f[15] = (float)(tm0 / I.lnorm);
+    double sums[8] = {sd2, stm, sp, sn, dtm, c1, c2, tm0};
+    warp_sum8(sums);
+    const double mld = (double)ml, fl = (double)flen, rmsd = sqrt(sums[0] / fl);
+    // feature j = num / den on lane j: one division for all of them
+    double num = 0.0, den = 1.0;
+    auto put = [&](int j, double a, double b) {
+        num = lane == j ? a : num;
+        den = lane == j ? b : den;
+    };
+    put(0, fl, mld);
+    put(1, (double)ps, (double)(plen > 1 ? plen - 1 : 1));
+    put(2, (double)ns, (double)(nlen > 1 ? nlen - 1 : 1));
+    put(3, (double)s, mld);
+    put(4, rmsd, 10.0);
+    put(5, sums[4], I.lnorm);
+    put(6, sums[5], mld);
+    put(7, sums[6], mld);
+    put(8, sums[1], fl);
+    put(9, sums[2], fl);
+    put(10, sums[3], fl);
+    put(11, log_ml, 7.0);
+    put(12, best, 1.0);
+    put(13, 0.5 * kind, 1.0);
+    put(14, fmin(rmsd / I.d0, 10.0), 10.0);
+    put(15, sums[7], I.lnorm);
+    return (float)(num / den);
 }
 
 // Features of seed w of a pair's main seed bank (seeds.h:41-283): a window
@@ -312,7 +334,7 @@ IA_DEV void main_seed_features(const DevBatch &b, const PairInfo &I, int p, int 
             first = min(first, i);
             last = max(last, i);
         }
-    m.group_sum(32);
+    m.warp_total();
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         first = min(first, __shfl_xor_sync(kAllLanes, first, o));
@@ -325,7 +347,7 @@ IA_DEV void main_seed_features(const DevBatch &b, const PairInfo &I, int p, int 
     for (int i = lane; i < N; i += 32) {
         if (!V[i]) continue;
         const double d2 = dist2(R, t, P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * i], Q[3 * i + 1], Q[3 * i + 2]);
-        const double term = 1.0 / (1.0 + d2 * inv);
+        const double term = tm_term(d2, inv);
         tm += term;
         c1 += d2 < d0sq ? 1.0 : 0.0;
         c2 += d2 < 4.0 * d0sq ? 1.0 : 0.0;
@@ -453,19 +475,21 @@ __global__ void __launch_bounds__(128) k_rank(DevBatch b, RankArgs a, const int 
         const int w0 = (c - chunk_begin[ti]) * kRankChunk + warp * 16;
         if (w0 < W) {
             const double best = b.state[rt.p].rec[REC_BEST][0];
+            const double log_ml = log((double)(rt.plen < rt.nlen ? rt.plen : rt.nlen));
             const long long wb = a.wbase[ti];
             for (int r = 0; r < 16; r++) {
                 const int w = w0 + r;
                 float mine = 0.f;
                 if (w < W) {
-                    float f[kFeatures];
-                    if (a.kind == CAND_MAIN)
+                    if (a.kind == CAND_MAIN) {
+                        float f[kFeatures];
                         main_seed_features(b, I, rt.p, w, f);
-                    else
-                        window_features(rt.x, rt.Lp, rt.Ln, I, rt.plen, rt.nlen, best, a.kind, w, f);
 #pragma unroll
-                    for (int j = 0; j < kFeatures; j++)
-                        if (lane == j) mine = f[j];
+                        for (int j = 0; j < kFeatures; j++)
+                            if (lane == j) mine = f[j];
+                    } else {
+                        mine = window_features(rt.x, rt.Lp, rt.Ln, I, rt.plen, rt.nlen, best, log_ml, a.kind, w);
+                    }
                     if (a.feat && lane < kFeatures) a.feat[(wb + w) * kFeatures + lane] = mine;
                 }
                 if (lane < kFeatures)

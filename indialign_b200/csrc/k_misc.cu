@@ -651,24 +651,24 @@ __global__ void k_weighted(DevBatch b) {
     double R[9], t[3];
     for (int a = 0; a < 9; a++) R[a] = S.rec[REC_BEST][1 + a];
     for (int a = 0; a < 3; a++) t[a] = S.rec[REC_BEST][10 + a];
-    const double d0sq = fmax(I.d0 * I.d0, 1e-12);
+    const double inv = 1.0 / fmax(I.d0 * I.d0, 1e-12);
     for (int it = 0; it < 4; it++) {
         Moments m;
         m.clear();
         for (int i = lane; i < N; i += 32) {
             if (!v[i]) continue;
             const double *pp = P + 3 * i, *qq = Q + 3 * i;
-            double w = 1.0 / (1.0 + dist2(R, t, pp[0], pp[1], pp[2], qq[0], qq[1], qq[2]) / d0sq);
+            double w = tm_term(dist2(R, t, pp[0], pp[1], pp[2], qq[0], qq[1], qq[2]), inv);
             if (w <= 0) continue;
             m.add_w(w, pp[0], pp[1], pp[2], qq[0], qq[1], qq[2]);
         }
-        m.group_sum(32);
+        m.warp_total();
         kabsch_from_moments(m, 1e-12, R, t);
     }
     double s = 0.0;
     for (int i = lane; i < N; i += 32) {
         if (!v[i]) continue;
-        s += 1.0 / (1.0 + dist2(R, t, P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * i], Q[3 * i + 1], Q[3 * i + 2]) / d0sq);
+        s += tm_term(dist2(R, t, P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * i], Q[3 * i + 1], Q[3 * i + 2]), inv);
     }
     s = warp_sum(s) / fmax(I.lnorm, 1.0);
     __syncwarp();
@@ -684,10 +684,10 @@ IA_DEV double pair_tm(const DevBatch &b, const PairInfo &I, const double *rec, i
     const double *P = b.pred + 3 * (size_t)off, *Q = b.nat + 3 * (size_t)off;
     const uint8_t *v = b.v + off;
     const double *R = rec + 1, *t = rec + 10;
-    const double d0sq = fmax(I.d0 * I.d0, 1e-12);
+    const double inv = 1.0 / fmax(I.d0 * I.d0, 1e-12);
     double s = 0.0;
     for (int i = lane; i < N; i += 32)
-        if (v[i]) s += 1.0 / (1.0 + dist2(R, t, P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * i], Q[3 * i + 1], Q[3 * i + 2]) / d0sq);
+        if (v[i]) s += tm_term(dist2(R, t, P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * i], Q[3 * i + 1], Q[3 * i + 2]), inv);
     return warp_sum(s) / fmax(I.lnorm, 1.0);
 }
 
@@ -740,7 +740,7 @@ __global__ void k_offset_starts(DevBatch b, double *starts, const int *slot_pair
         if (j < 0 || j >= N || !pv[i] || !nv[j]) continue;
         m.add(P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * j], Q[3 * j + 1], Q[3 * j + 2]);
     }
-    m.group_sum(32);
+    m.warp_total();
     double R[9], t[3];
     kabsch_from_moments(m, 3.0, R, t);
     if (lane < kRec) rec[lane] = lane == 0 ? (m.w >= 3.0 ? 0.0 : kNegInf)
