@@ -328,6 +328,9 @@ __global__ void k_glue(DevBatch b, GlueArgs a) {
         break;
     case G_SS_BEGIN:  // evaluate_ss_seeds: best = -1e30 / identity (ss.h:93-95)
         rec_ident(S.rec[REC_SS], kScoreInit);
+        // the label alignment takes no transform, but a chain runs only from a
+        // start record with a score: not what an earlier batch left there
+        rec_ident(S.rec[REC_START], 0.0);
         break;
     case G_SS_DET:  // det after an SS alignment, then arm dp_refine (ss.h:96-105)
         S.dp_on = 0;
