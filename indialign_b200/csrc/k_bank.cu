@@ -628,13 +628,29 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
                 // outside the mask is staged with a NaN native point)
                 XformF2 X;
                 X.set(R, t);
-#pragma unroll 4
-                for (int k2 = 0; k2 < (n + 1) >> 1; k2++) {
-                    const float4 PA = Pf[2 * k2], PB = Pf[2 * k2 + 1], QA = Qf[2 * k2], QB = Qf[2 * k2 + 1];
-                    const float2 d2 = dist2_pair(PA, PB, QA, QB, X);
+                // distances of four pairs of residues side by side; the sums of
+                // a pair are skipped when no lane's cutoff takes it (a learned
+                // search of 1024 pairs: 134.9 -> 129.6 ms)
+                constexpr int U = 4;
+                const int pairs = (n + 1) >> 1;
+                auto dist2 = [&](int k) { return dist2_pair(Pf[2 * k], Pf[2 * k + 1], Qf[2 * k], Qf[2 * k + 1], X); };
+                auto add = [&](float2 d2, int k) {
+                    const float4 PA = Pf[2 * k], PB = Pf[2 * k + 1], QA = Qf[2 * k], QB = Qf[2 * k + 1];
                     m.add_if(d2.x, lim, PA.x, PA.z, PB.x, QA.x, QA.z, QB.x);
                     m.add_if(d2.y, lim, PA.y, PA.w, PB.y, QA.y, QA.w, QB.y);
+                };
+                int k2 = 0;
+#pragma unroll 1
+                for (; k2 + U <= pairs; k2 += U) {
+                    float2 d2[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) d2[u] = dist2(k2 + u);
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (__any_sync(0xffffffffu, fminf(d2[u].x, d2[u].y) <= lim)) add(d2[u], k2 + u);
                 }
+#pragma unroll 1
+                for (; k2 < pairs; k2++) add(dist2(k2), k2);
             } else {
                 float Rf[9], tf[3];
 #pragma unroll
