@@ -31,15 +31,19 @@ constexpr int kFillLag = 49;
 // Rows per lane by the modelled issue slots: steps x (20 per step of
 // bookkeeping + 32 per row of 2 cells).  More rows per lane share the
 // bookkeeping; fewer leave fewer idle rows in the last stripe and, with
-// several warps, give more stripes to share.
+// several warps, give more stripes to share.  Three rows are taken when they
+// save an eighth or more: warps that run the other loop at the same time cost
+// instruction fetches.  k_chain, ms, on 64 pairs of L 40-300 / 160 pairs of L
+// 20-1100: four rows only 54.4 / 87.0, three or four 52.6 / 86.6, without the
+// eighth 52.7 / 87.4, two as well 53.1 / 87.8.
 IA_GEOM_FN FillGeom fill_geom(int plen, int nlen, int W) {
     const int n32 = (plen + 31) >> 5, np = (nlen + 1) >> 1;
-    FillGeom g = {2, n32, W, 0};
+    FillGeom g = {4, n32, W, 0};
     long long best = -1;
-    for (int R = 4; R >= 2; R--) {
+    for (int R = 4; R >= 3; R--) {
         const int S = (n32 + R - 1) / R, rounds = (S + W - 1) / W;
         const long long steps = (long long)rounds * (np + 31) + ((S < W ? S : W) - 1) * kFillLag;
-        const long long cost = steps * (20 + 32 * R);
+        const long long cost = steps * (20 + 32 * R) * (R < 4 ? 9 : 8);
         if (best < 0 || cost < best) {
             best = cost;
             g.R = R;

@@ -23,7 +23,9 @@
 //     has no branch: a stripe's lanes start together, and a lane whose first
 //     column has not come yet works on staged NaN columns, on which a cell
 //     leaves H = 0, the boundary value; columns and the boundary row carry
-//     padding on both sides, so no index is clamped.
+//     padding on both sides, so no index is clamped;
+//   * the cutoff and the gap are factors (0 or 1) of fused multiply-adds, not
+//     compares and selects: the ALU pipe runs at half the FMA pipe's rate.
 // Stripes run one after the other (31 idle lane steps each).  The stripe's last
 // row goes to the next stripe through a boundary row in memory.  W warps may
 // share one alignment: warp w takes stripes w, w + W, ..., publishes per 16
@@ -32,8 +34,9 @@
 //
 // Measured (B200) against two rows per lane and one column per step with
 // scalar entries, compare / select directions and a cell-by-cell traceback:
-// fill 14 -> 3.3 warp cycles per cell on 48 pairs of L 30-1500, 19.5 -> 4.3 on
-// 64 pairs of L 40-300 (whose last stripes are emptier); traceback 0.8 -> 0.14
+// fill 14 -> 3.0 warp cycles per cell on 48 pairs of L 30-1500, 19.5 -> 3.6 on
+// 64 pairs of L 40-300 (whose last stripes are emptier; with selects for the
+// cutoff and the gap 3.3 and 4.3); traceback 0.8 -> 0.14
 // and 2.9 -> 0.72.  Lanes that wrap into the next stripe without draining, with
 // the entry code inside the step loop, took 4.4 and 8.7 (half of the warps'
 // time without an instruction to issue); unrolling that loop twice, 6.3 and 15.
@@ -63,10 +66,10 @@ struct FillArgs {
 
 // Native column pair k as {-x0, -x1, -y0, -y1, -z0, -z1} at dst + 6 k, for
 // k = -kFillPad .. pairs + kFillPad - 1: NaN left of the matrix (see
-// fill_cell), the last pair's values right of it.  A non-finite coordinate
-// becomes a point 2e30 away from any other (moved_row puts non-finite rows on
-// the other side), whose squared distance is infinite: beyond the cutoff, as
-// the comparison with NaN or infinity makes it.  The SS4 mode has no cutoff
+// fill_cell), the last pair's values right of it.  A point with a non-finite
+// coordinate, or one beyond 1e18, is put at 1e18 (moved_row puts such rows at
+// -1e18): beyond the cutoff, as the comparison with NaN or infinity makes it,
+// with a finite square.  The SS4 mode has no cutoff
 // and takes the values as they are.
 IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int tid, int nthreads) {
     const int pairs = (nlen + 1) >> 1;
@@ -78,7 +81,7 @@ IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int t
             x = (float)q[0];
             y = (float)q[1];
             z = (float)q[2];
-            if (!raw && !(isfinite(x) && isfinite(y) && isfinite(z))) x = y = z = 1e30f;
+            if (!raw && !(fabsf(x) <= 1e18f && fabsf(y) <= 1e18f && fabsf(z) <= 1e18f)) x = y = z = 1e18f;
         }
         float *o = dst + 6 * k + half;
         o[0] = -x;
@@ -97,6 +100,14 @@ IA_DEV float rcp_f32(float x) {
     return fmaf(y, fmaf(-x, y, 1.f), y);
 }
 
+// The cutoff as a factor of the FMA pipe instead of a compare and a select:
+// with c the next float above cut2, sat((c - d2) 2^40) is 1 for d2 <= cut2 (the
+// difference is then at least one unit in the last place of cut2, 2^-20 for
+// the search's smallest cutoff of 3.5^2, and 1 already from cut2 >= 2^-16 on)
+// and 0 for d2 >= c.
+constexpr float kCutScale = 1099511627776.f;  // 2^40
+IA_DEV float cut_limit(float cut2) { return nextafterf(cut2, INFINITY) * kCutScale; }
+
 // Score entries of one row (its point in every half of mx, my, mz) and two
 // columns: 1/(1 + d2/d0^2), or 0 beyond the cutoff (distance mode; NaN left of
 // the matrix); plus 0.5 for equal labels (SS4); label identity (SS2).
@@ -104,7 +115,7 @@ IA_DEV float rcp_f32(float x) {
 // fma(d2, 1/d0^2, 1).
 template <int SMODE>
 IA_DEV float2 score_pair(float2 mx, float2 my, float2 mz, float2 qx, float2 qy, float2 qz, float2 ninv, float inv,
-                         float cut2, uint8_t lp, uint8_t ln0, uint8_t ln1, bool left_of) {
+                         float limit, uint8_t lp, uint8_t ln0, uint8_t ln1, bool left_of) {
     float2 r;
     if (SMODE == SMAT_SS2) {
         r = make_float2(lp == ln0 ? 1.f : 0.f, lp == ln1 ? 1.f : 0.f);
@@ -121,8 +132,13 @@ IA_DEV float2 score_pair(float2 mx, float2 my, float2 mz, float2 qx, float2 qy, 
     float2 y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-nden.x));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-nden.y));
-    r = __ffma2_rn(y, __ffma2_rn(nden, y, make_float2(1.f, 1.f)), y);
-    return make_float2(d2.x > cut2 ? 0.f : r.x, d2.y > cut2 ? 0.f : r.y);
+    // 1 within the cutoff, 0 beyond (cut_limit)
+    float2 k;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(k.x) : "f"(d2.x), "f"(-kCutScale), "f"(limit));
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(k.y) : "f"(d2.y), "f"(-kCutScale), "f"(limit));
+    const float2 e2 = __ffma2_rn(nden, y, make_float2(1.f, 1.f));
+    const float2 yk = __fmul2_rn(y, k);
+    return __ffma2_rn(yk, e2, yk);
 }
 
 // One cell (indialign_c/nw.h:20-35): diag wins ties, then left, then up; a gap
@@ -148,7 +164,9 @@ IA_DEV void fill_cell(float diag_src, float sc, float up, float left, float gap,
     a = __funnelshift_l(__float_as_uint(x), a, 1);
     b = __funnelshift_l(__float_as_uint(y), b, 1);
     h = fmaxf(diag, m);
-    hp = diag >= m ? diag + gap : m;
+    float isd;  // 1 if diagonal: one compare to a factor instead of compare, add and select
+    asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(isd) : "f"(diag), "f"(m));
+    hp = fmaf(isd, gap, h);
 }
 
 // A lane's 2R trace words of one 16-step group, shifted left by sh.
@@ -170,7 +188,7 @@ IA_DEV float3 moved_row(const FillArgs &A, int i, bool raw) {
     double x, y, z;
     xform(A.rt, A.rt + 9, p[0], p[1], p[2], x, y, z);
     float3 m = make_float3((float)x, (float)y, (float)z);
-    if (!raw && !(isfinite(m.x) && isfinite(m.y) && isfinite(m.z))) m.x = m.y = m.z = -1e30f;
+    if (!raw && !(fabsf(m.x) <= 1e18f && fabsf(m.y) <= 1e18f && fabsf(m.z) <= 1e18f)) m.x = m.y = m.z = -1e18f;
     return m;
 }
 
@@ -182,7 +200,7 @@ __device__ __noinline__ void nw_fill(const FillArgs &A, const FillGeom G, int w)
     const int lane = threadIdx.x & 31;
     const int plen = A.plen, nlen = A.nlen, W = G.W, S = G.S;
     const int np = (nlen + 1) >> 1;
-    const float gap = A.gap, inv = A.inv_d0sq, cut2 = A.cut2;
+    const float gap = A.gap, inv = A.inv_d0sq, limit = cut_limit(A.cut2);
     const float2 ninv = make_float2(-inv, -inv);
     for (int k = w; k < S; k += W) {
         const int row0 = (k * 32 + lane) * R;
@@ -261,7 +279,7 @@ __device__ __noinline__ void nw_fill(const FillArgs &A, const FillGeom G, int w)
                 float2 e[R];
 #pragma unroll
                 for (int r = 0; r < R; r++)
-                    e[r] = score_pair<SMODE>(mx[r], my[r], mz[r], qx, qy, qz, ninv, inv, cut2, lp[r], ln0, ln1, left_of);
+                    e[r] = score_pair<SMODE>(mx[r], my[r], mz[r], qx, qy, qz, ninv, inv, limit, lp[r], ln0, ln1, left_of);
                 float n0[R], p0[R];
 #pragma unroll
                 for (int r = 0; r < R; r++)
@@ -300,8 +318,7 @@ __device__ __noinline__ void nw_fill(const FillArgs &A, const FillGeom G, int w)
 template <int SMODE>
 IA_DEV void nw_fill_r(const FillArgs &A, const FillGeom &G, int w) {
     if (G.R == 4) nw_fill<SMODE, 4>(A, G, w);
-    else if (G.R == 3) nw_fill<SMODE, 3>(A, G, w);
-    else nw_fill<SMODE, 2>(A, G, w);
+    else nw_fill<SMODE, 3>(A, G, w);
 }
 
 // The path from (plen, nlen) by the trace's bits (indialign_c/nw.h:42-68);
