@@ -363,8 +363,8 @@ int indialign_selftest_rcp_f32(unsigned long long *mismatches);
  * tune_b200.txt beside the library (or the file named by
  * INDIALIGN_TUNE_TABLE), written by indialign_b200/autotune.py.
  * Rows: {max_len, bank_chunk (items per CTA chunk, multiple of 32, 32..4096),
- * bank_cutoff_major (0/1: item order), chain_chunk (NW chains per CTA chunk,
- * 1..256), chain_smem_trace (0/1: NW traces in shared memory when they fit
+ * bank_cutoff_major (0/1: item order), chain_chunk (1..256; kept in the table,
+ * without effect: NW chains are taken one at a time), chain_smem_trace (0/1: NW traces in shared memory when they fit
  * without losing occupancy)}, max_len ascending (the last bucket takes every
  * longer pair). */
 #define INDIALIGN_TUNE_BUCKETS 3

@@ -29,8 +29,7 @@ from . import ranker
 from . import workloads as W
 
 BUCKET_RANGES = [(40, 128), (129, 512), (513, 1200)]
-KNOBS = [("bank_chunk", (128, 256, 512)), ("bank_cutoff_major", (1, 0)), ("chain_chunk", (16, 8, 32)),
-         ("chain_smem_trace", (1, 0))]
+KNOBS = [("bank_chunk", (128, 256, 512)), ("bank_cutoff_major", (1, 0)), ("chain_smem_trace", (1, 0))]
 
 
 def _time_search(ia, pairs, blob, repeats):

@@ -7,6 +7,7 @@
 // evaluate_ss_seeds (indialign_c/ss.h:56-164).  The fill and the traceback of
 // the search's own matrices are in nw_fill.cuh; the NW on an explicit FP64
 // matrix is here.
+#include <climits>
 #include <vector>
 
 #include "../../include/indialign_b200.h"
@@ -318,11 +319,12 @@ IA_NW_ATTR double lite_detailed(const Pts &x, const uint32_t *al, int na, const 
 }
 
 // ---- the chain kernel ----------------------------------------------------
+constexpr int kManyChains = 16;  // chains per warp from which an SM's CTAs start together
+
 struct ChainCtl {
-    int cur, end;         // the CTA's chains still to hand out (launch-wide indices)
-    int task, lo, hi;     // the piece in hand: chains [lo, hi) of one task
-    int next;             // next chain of the piece
-    int na;               // one chain per CTA: aligned pairs of the last alignment
+    int task;   // the task in hand, -1: none left
+    int chain;  // one chain per CTA: its index in the task
+    int na;     // one chain per CTA: aligned pairs of the last alignment
 };
 
 // Element `lane` of a result record {score, R[9], t[3]} by unrolled selects
@@ -346,8 +348,20 @@ IA_DEV void put_rt(double *dst, const double *R, const double *t, int lane) {
 // mode only); EMIT = true: single NW alignments for SS seeds / full dp_refine.
 // Two instantiations keep the hot kernel's code small.
 //
-// CTAs pull `grab` chains at a time; the chains of one pair among them are a
-// piece, whose warps take them one by one.  A launch of at most coop_max
+// A CTA stays with a task while it has chains, whose warps take them one at a
+// time: it stages the pair's columns once and its warps wait for one another
+// only when the task has run out and the CTA goes on to the next one with
+// chains left.  (Eight chains per CTA and piece, with a barrier after each,
+// kept the warps waiting for 13 % of their time: k_chain of a learned search
+// of 1024 pairs of L 20-499 80 -> 61 ms, of 64 pairs of L 30-1500 30 -> 22.6.)
+// CTAs start spread over the tasks by their share of the chains; in launches
+// of many chains per warp the CTAs of an SM start together, so that their
+// loops' code and their pair's points are shared (64 pairs of L 40-300: 52.7
+// ms against 58.1 spread singly), in smaller ones apart, so that the longest
+// chains do not share an SM (64 pairs learned: 22.6 against 26.7), and a launch
+// of fewer chains than warps gives each CTA as many warps as chains fall to it.
+//
+// A launch of at most coop_max
 // chains leaves most of the chip idle with a warp per chain, and its time is
 // the longest chain's: then a CTA takes one chain at a time, its warps share
 // the fill's stripes, and warp 0 does the rest.  Measured, both with the fill
@@ -359,7 +373,7 @@ IA_DEV void put_rt(double *dst, const double *R, const double *t, int lane) {
 template <bool EMIT>
 __global__ void __launch_bounds__(32 * kChainWarps, IA_CHAIN_MINB)
 k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__ chain_begin,
-        int ntasks, const ScanOut *__restrict__ scan, int *counter, ChainScratch sc) {
+        int ntasks, const ScanOut *__restrict__ scan, int *left, ChainScratch sc) {
     extern __shared__ __align__(16) char smem[];
     __shared__ ChainCtl ctl;
     __shared__ uint64_t bar;
@@ -387,15 +401,33 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
     char *albase = wbase + (bh_smem ? kChainWarps * bh_floats * 4 : 0);
     char *trbase = albase + (al_smem ? kChainWarps * al_bytes : 0);
     uint32_t phase = 0;
-    if (threadIdx.x == 0) {
-        mbar_init(&bar);
-        ctl.cur = ctl.end = 0;
-        ctl.task = -1;
-    }
-    __syncthreads();
     const int total = scan->total_chunks;
     const bool coop = total <= sc.coop_max;
-    const int grab = coop ? 1 : min(sc.chunk, max(kChainWarps, total / (4 * (int)gridDim.x)));
+    const int pull = min(kChainWarps, (total + (int)gridDim.x - 1) / (int)gridDim.x);  // warps that take chains
+    if (threadIdx.x == 0) {
+        mbar_init(&bar);
+        // the CTA's first task: the one that holds its share of the launch's
+        // chains (one chain per CTA: the CTA's chain).  The share only says
+        // where a CTA begins to look for chains
+        ctl.task = -1;
+        uint32_t place = blockIdx.x, places = gridDim.x;
+        if (total >= kManyChains * kChainWarps * (int)gridDim.x) {
+            asm("mov.u32 %0, %%smid;" : "=r"(place));
+            asm("mov.u32 %0, %%nsmid;" : "=r"(places));
+            place = min(place, places - 1);
+        }
+        const int c = coop ? blockIdx.x : (int)((long long)total * place / places);
+        if (c < total) {
+            int lo = 0, hi = ntasks;  // first begin > c
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (chain_begin[mid] <= c) lo = mid + 1; else hi = mid;
+            }
+            ctl.task = lo - 1;
+            ctl.chain = c - chain_begin[lo - 1];
+        }
+    }
+    __syncthreads();
     // this warp's buffers (one chain per CTA: the CTA's first)
     const int slot = coop ? 0 : warp, gw = blockIdx.x * kChainWarps + slot;
     uint32_t *al = al_smem ? reinterpret_cast<uint32_t *>(albase + slot * al_bytes)
@@ -413,35 +445,7 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
     fa.prog = s_prog;
     fa.err = b.err;
     for (;;) {
-        if (threadIdx.x == 0) {
-            if (ctl.cur >= ctl.end) {  // next chains of the launch
-                const int c = atomicAdd(counter, grab);
-                ctl.cur = c;
-                ctl.end = min(c + grab, total);
-                if (c < total) {
-                    int lo = 0, hi = ntasks;  // first begin > c
-                    while (lo < hi) {
-                        const int mid = (lo + hi) >> 1;
-                        if (chain_begin[mid] <= c) lo = mid + 1; else hi = mid;
-                    }
-                    ctl.task = lo - 1;
-                }
-            } else {  // the same CTA chunk goes on in the next task with chains
-                do ctl.task++;
-                while (tasks[ctl.task].n_chains == 0);
-            }
-            if (ctl.cur < ctl.end) {
-                const int begin = chain_begin[ctl.task];
-                ctl.lo = ctl.cur - begin;
-                ctl.hi = min(ctl.end - begin, tasks[ctl.task].n_chains);
-                ctl.cur = begin + ctl.hi;
-                ctl.next = ctl.lo;
-            } else {
-                ctl.task = -1;
-            }
-        }
-        __syncthreads();
-        const int ti = ctl.task, chain_hi = ctl.hi;
+        const int ti = ctl.task;
         if (ti < 0) break;
         const ChainTask &T = tasks[ti];
         const PairInfo &I = b.info[T.pair];
@@ -513,14 +517,16 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             }
             return na;
         };
-        // warps of the CTA pull the piece's chains one at a time, so a long
-        // chain does not hold the other warps at a barrier
+        // warps take the task's chains one at a time
         for (;;) {
-            int chain = ctl.lo;
+            int chain = ctl.chain;
             if (!coop) {
-                if (lane == 0) chain = atomicAdd(&ctl.next, 1);
-                chain = __shfl_sync(kFull, chain, 0);
-                if (chain >= chain_hi) break;
+                if (warp >= pull) break;
+                int rest = 0;
+                if (lane == 0) rest = atomicSub(left + ti, 1);
+                rest = __shfl_sync(kFull, rest, 0);
+                if (rest <= 0) break;
+                chain = T.n_chains - rest;
             }
             if (lead && lane == 0) atomicAdd(b.ctr + CTR_CHAINS, 1ull);
             const int gaps = T.gaps;
@@ -616,6 +622,21 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             }
             if (coop) break;
         }
+        if (coop) break;
+        // the next task, in cyclic order, that has chains left; a task without
+        // any never gets some again
+        __syncthreads();
+        if (threadIdx.x == 0) ctl.task = INT_MAX;
+        __syncthreads();
+        for (int d0 = 1; d0 < ntasks; d0 += blockDim.x) {
+            const int d = d0 + (int)threadIdx.x, t = ti + d < ntasks ? ti + d : ti + d - ntasks;
+            const bool some = d < ntasks && *(volatile int *)(left + t) > 0;
+            if (some) atomicMin(&ctl.task, d);
+            if (__syncthreads_or(some)) break;
+        }
+        const int d = ctl.task;
+        __syncthreads();
+        if (threadIdx.x == 0) ctl.task = d == INT_MAX ? -1 : ti + d < ntasks ? ti + d : ti + d - ntasks;
         __syncthreads();
     }
 }
@@ -659,11 +680,11 @@ size_t chain_smem_bytes(int pmax, int nmax, int flags) {
 }
 
 void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, int ntasks,
-                  const ScanOut *scan, int *counter, const ChainScratch &sc, int grid, bool emit,
+                  const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
                   cudaStream_t st) {
     const size_t sm = chain_smem_bytes(sc.pmax, sc.nmax, sc.flags);
-    if (emit) k_chain<true><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, ntasks, scan, counter, sc);
-    else k_chain<false><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, ntasks, scan, counter, sc);
+    if (emit) k_chain<true><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, ntasks, scan, left, sc);
+    else k_chain<false><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, ntasks, scan, left, sc);
 }
 
 const void *chain_kernel_ptr() { return (const void *)k_chain<false>; }

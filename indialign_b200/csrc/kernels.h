@@ -103,12 +103,12 @@ struct ChainScratch {
     uint32_t *gal;
     int pmax, nmax;      // longest pred / native of the launch
     int flags;           // in shared memory: 1 columns and labels, 2 boundary, 4 alignment, 8 trace
-    int chunk;           // most chains a CTA pulls at a time
     int coop_max;        // launches of at most this many chains run one chain per CTA
 };
 size_t chain_smem_bytes(int pmax, int nmax, int flags);
+// left: per task its number of chains, counted down by the launch
 void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, int ntasks,
-                  const ScanOut *scan, int *counter, const ChainScratch &sc, int grid, bool emit,
+                  const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
                   cudaStream_t st);
 cudaError_t chain_set_attributes();
 const void *chain_kernel_ptr();

@@ -33,7 +33,7 @@ constexpr int kBankChunk = 128;    // threads of a bank CTA (4 warps x 32)
 struct Tune {
     int bank_chunk = 256;       // bank items per CTA chunk (multiple of 32)
     int bank_cutoff_major = 1;  // bank item order: 1 cutoff major, 0 seed major
-    int chain_chunk = 16;       // NW chains per CTA chunk
+    int chain_chunk = 16;       // accepted and kept, without effect: warps take chains one at a time
     int chain_smem_trace = 1;   // NW traces in shared memory when they fit
 };
 constexpr int kTuneBuckets = 3;

@@ -209,7 +209,6 @@ struct Cfg {
     unsigned long long seed = 0;
     TuneRows tune;              // kernel shapes per length bucket (per task)
     int chain_smem_trace = 1;  // NW traces in shared memory (the longest pair's bucket)
-    int chain_chunk = 16;      // NW chains a CTA pulls at a time (the longest pair's bucket)
 };
 
 // Host view of per-pair facts after k_prep / k_anchor.
@@ -618,8 +617,8 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
     }
     const bool emit = kind == CH_SS2 || kind == CH_SS4 || kind == CH_DP_EMIT;
     const ChainScratch sc = {c_->gtrace.p, trace_words_, c_->gbh.p,    c_->gcol.p,       c_->gal.p,
-                             pmax,         nmax,         chain_flags_, cfg_.chain_chunk, chain_grid_};
-    launch_chain(b, c_->ctasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, sc, chain_grid_, emit,
+                             pmax,         nmax,         chain_flags_, chain_grid_};
+    launch_chain(b, c_->ctasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counts.p, sc, chain_grid_, emit,
                  c_->stream);
     if (timing) {
         cudaEventRecord(e1, c_->stream);
@@ -1381,7 +1380,6 @@ static int run_search(int device, const Cfg &cfg0, const Source &src, double *re
         Cfg cfg = cfg0;
         cfg.tune = tt.rows();
         cfg.chain_smem_trace = tt.t[bucket_of(tt, Lmax)].chain_smem_trace;
-        cfg.chain_chunk = tt.t[bucket_of(tt, Lmax)].chain_chunk;
         Ctx *c = nullptr;
         int rc = acquire(device, &c);
         if (rc) return rc;
@@ -1421,7 +1419,6 @@ static int run_search(int device, const Cfg &cfg0, const Source &src, double *re
         P.cfg = cfg0;
         P.cfg.tune = tt.rows();
         P.cfg.chain_smem_trace = tt.t[b].chain_smem_trace;
-        P.cfg.chain_chunk = tt.t[b].chain_chunk;
         if (!src.host.empty()) {
             for (int p : I) P.src.host.push_back(src.host[p]);
         } else {
