@@ -362,11 +362,11 @@ int indialign_selftest_rcp_f32(unsigned long long *mismatches);
  * Results are those of one call either way.  The table comes from
  * tune_b200.txt beside the library (or the file named by
  * INDIALIGN_TUNE_TABLE), written by indialign_b200/autotune.py.
- * Rows: {max_len, bank_chunk (items per CTA chunk, multiple of 32, 32..4096),
- * bank_cutoff_major (0/1: item order), chain_chunk (1..256; kept in the table,
- * without effect: NW chains are taken one at a time), chain_smem_trace (0/1: NW traces in shared memory when they fit
- * without losing occupancy)}, max_len ascending (the last bucket takes every
- * longer pair). */
+ * Rows: {max_len, bank_chunk (multiple of 32, 32..4096), bank_cutoff_major
+ * (0/1: item order), chain_chunk (1..256), chain_smem_trace (0/1: NW traces in
+ * shared memory when they fit without losing occupancy)}, max_len ascending (the last bucket takes every
+ * longer pair).  bank_chunk and chain_chunk are kept in the table without
+ * effect: items and chains are taken as warps become free. */
 #define INDIALIGN_TUNE_BUCKETS 3
 #define INDIALIGN_TUNE_FIELDS 5
 /* The table in use: split (0/1), min_pairs (batches with fewer pairs are not

@@ -2,9 +2,9 @@
 
 Every task of the batched search runs with its pair's length-bucket row
 (N <= 128, <= 512, longer) of a kernel-shape table (indialign_set_tuning /
-tune_b200.txt beside the library): seed-bank items per CTA chunk and their
-order, NW chains per CTA chunk, NW traces in shared memory; the table also
-says whether a batch that spans buckets runs as concurrent per-bucket
+tune_b200.txt beside the library): the order of the seed-bank items, NW traces
+in shared memory (the chunk sizes are kept without effect); the table also says
+whether a batch that spans buckets runs as concurrent per-bucket
 sub-batches.  This script times candidate rows on
 seeded synthetic batches of each bucket (the batch shape of the workloads:
 sigma ~ U(0.5,14) A, 5 % invalid residues per mask, random rigid transform)
@@ -29,7 +29,7 @@ from . import ranker
 from . import workloads as W
 
 BUCKET_RANGES = [(40, 128), (129, 512), (513, 1200)]
-KNOBS = [("bank_chunk", (128, 256, 512)), ("bank_cutoff_major", (1, 0)), ("chain_smem_trace", (1, 0))]
+KNOBS = [("bank_cutoff_major", (1, 0)), ("chain_smem_trace", (1, 0))]
 
 
 def _time_search(ia, pairs, blob, repeats):

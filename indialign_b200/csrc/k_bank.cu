@@ -21,15 +21,24 @@
 // arithmetic in its seed banks stayed within 2e-8 of the reference build's
 // final TM-scores on 560 pairs.
 //
-// k_bank is bound by the FMA pipe (62 % busy on the main bank of 61 pairs, the
-// rest is the chunk barrier and the launch's tail): a residue visit is 15
-// operations of distance, paired over two residues, and 15 of sums.  The sums
-// sit under one predicate per residue without a branch and the sweep is
-// unrolled four times, so that distances of later residues fill the sums'
-// latency: 167 -> 136 ms over the bank launches of a learned search of 1024
-// pairs of L 40-1000 (a branch around the sums 152, unrolled twice 150; eight
-// times gained 1.5 % more in a third more code; skipping a pair no lane wants
-// by a vote 131, but 10 % slower on single pairs).
+// k_bank is bound by the FMA pipe (62 % busy on the main bank of 61 pairs): a
+// residue visit is 15 operations of distance, paired over two residues, and 15
+// of sums.  The sums sit under one predicate per residue without a branch and
+// the sweep takes four residue pairs at a time, so that distances of later
+// residues fill the sums' latency: 167 -> 136 ms over the bank launches of a
+// learned search of 1024 pairs of L 40-1000 (a branch around the sums 152,
+// unrolled twice 150; eight times gained 1.5 % more in a third more code), and
+// 129.6 with a vote that skips a pair no lane wants.
+//
+// A CTA stays with a task while it has items, whose warps take them as they
+// become free.  (Chunks of 256 items with a barrier after each, for which every
+// CTA staged the points again, kept the warps waiting for 13 % of their time:
+// bank launches of 61 learned pairs 10.8 -> 9.5 ms, of one pair of 64 residues
+// 0.65 -> 0.57, of the 1024 pairs 129.5 -> 126.)  CTAs start spread over the
+// tasks by their work, items x residues, so that the tasks end together (spread
+// by items alone, the banks of 64 learned pairs of L 30-1500 took 12.7 ms
+// against 11.2), and a launch of few items gives each CTA as many warps as
+// items fall to it.
 #include "dmath.cuh"
 #include "stage.cuh"
 #include "pipeline.h"
@@ -49,8 +58,20 @@
 namespace ia {
 
 // ---- the bank kernel -------------------------------------------------------
-struct BankSmem {
-    int chunk, task;
+// A launch's units of work (kBankUnit items of a task).
+struct BankWork {
+    int *left;   // units left of the task in hand
+    int *taken;  // units taken in the launch
+    // Take up to `units` units; returns the first item, or -1.
+    IA_DEV int take(const BankTask &T, int units) const {
+        int rest = 0;
+        if ((threadIdx.x & 31) == 0) {
+            rest = atomicSub(left, units);
+            if (rest > 0) atomicAdd(taken, min(units, rest));
+        }
+        rest = __shfl_sync(0xffffffffu, rest, 0);
+        return rest <= 0 ? -1 : kBankUnit * ((T.n_items + kBankUnit - 1) / kBankUnit - rest);
+    }
 };
 
 // Raw moments of the selected pairs in FP32 (counts exact).
@@ -343,7 +364,7 @@ IA_DEV void points_to_f4(const double *src, float4 *dst, int n, const double *of
     __syncthreads();
 }
 
-// The items [.., ce) of a task by four lanes each, for launches of few items:
+// A task's items by four lanes each, for launches of few items:
 // there a thread per item leaves the chip idle and the launch takes as long as
 // one thread's sweeps, 15 operations of distance and 15 of sums per residue in
 // turn.  The sums are the outer product (px, py, pz, 1) x (qx, qy, qz, 1): lane
@@ -353,21 +374,20 @@ IA_DEV void points_to_f4(const double *src, float4 *dst, int n, const double *of
 // bits as in the thread-per-item loop.  It issues 1.6 times the instructions
 // per residue and item and solves 8 systems per warp instead of 32, so the line
 // lies at 64 items per resident CTA (IA_BANK_WIDE): k_bank's launches on one
-// pair of 64 residues 0.70 -> 0.65 ms, of 1203 residues 6.8 -> 5.0; with the line
-// at 128, a learned search of 61 pairs loses 0.9 of 10.9 ms.
+// pair of 64 residues 0.70 -> 0.65 ms, of 1203 residues 6.8 -> 5.0 (0.57 and 4.3
+// since the CTAs stay with a task); with the line at 128, a learned search of
+// 61 pairs lost 0.9 of 10.9 ms.
 IA_DEV void wide_items(const BankTask &T, const float4 *P4, const float4 *Q4, const double *oP, const double *oQ,
-                       const double *__restrict__ seed_rt, double *__restrict__ item_res, int *s_next, int ce,
+                       const double *__restrict__ seed_rt, double *__restrict__ item_res, const BankWork &work,
                        unsigned long long *ctr) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31, a = lane & 3, g0 = lane & 28, n = T.n, C = T.C > 0 ? T.C : 1;
     const float *Pa = reinterpret_cast<const float *>(P4) + a;
     for (;;) {
-        int gi = 0;
-        if (lane == 0) gi = atomicAdd(s_next, 8);
-        gi = __shfl_sync(kFull, gi, 0);
-        if (gi >= ce) break;
+        const int gi = work.take(T, 1);
+        if (gi < 0) break;
         const int pi = gi + (lane >> 2);
-        const bool active = pi < ce;
+        const bool active = pi < T.n_items;
         int sk = 0, ci = 0;
         if (active) {
             const int K = T.n_items / C;
@@ -470,19 +490,18 @@ IA_DEV void wide_items(const BankTask &T, const float4 *P4, const float4 *Q4, co
     }
 }
 
-// CTAs pull chunks of one task's items; their warps take them 32 at a time (8 in
+// CTAs go from task to task; their warps take a task's items 32 at a time (8 in
 // a launch of at most wide_max items, see wide_items).
 template <bool SMEM>
 __global__ void __launch_bounds__(kBankChunk, IA_BANK_MINB)
-k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
-       int ntasks, const ScanOut *__restrict__ scan, int *counter,
+k_bank(const BankTask *__restrict__ tasks, const float *__restrict__ work_begin,
+       int ntasks, const ScanOut *__restrict__ scan, int *left, int *taken,
        const double *__restrict__ seed_rt, double *__restrict__ item_res, int *err, int nmax, int wide_max,
        unsigned long long *ctr) {
     extern __shared__ __align__(16) char smem[];
-    __shared__ BankSmem ctl;
+    __shared__ int s_task, s_slot;
     __shared__ uint64_t bar;
     __shared__ double oP[3], oQ[3], red[6 * (kBankChunk / 32)];  // point-set means
-    __shared__ int s_next;  // next item of the chunk
     // layout: P[nmax*3] Q[nmax*3] (each +16 B lead room), V, PV, NV bytes
     // room for a 15-byte lead and the rounded-up tail of a bulk copy
     const uint32_t coord_bytes = ((uint32_t)nmax * 24u + 47u) & ~15u;
@@ -490,36 +509,28 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
     char *sP = smem, *sQ = smem + coord_bytes, *sV = sQ + coord_bytes;
     char *sPV = sV + mask_bytes, *sNV = sPV + mask_bytes;
     uint32_t phase = 0;
-    if (threadIdx.x == 0) mbar_init(&bar);
-    __syncthreads();
     const int total = scan->total_chunks;
+    if (total <= 0) return;
     const bool wide = SMEM && scan->items <= wide_max;
-    int staged = -1;
+    const int units = wide ? 1 : 32 / kBankUnit;  // units a warp takes at a time
+    // warps of a CTA that take items: in a launch of few, those that fall to it
+    const int pull = min((int)blockDim.x / 32, (total / units + (int)gridDim.x) / (int)gridDim.x);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        mbar_init(&bar);
+        s_task = first_task(work_begin, left, ntasks, scan->work, blockIdx.x, gridDim.x);
+    }
+    __syncthreads();
     const float4 *Pf = nullptr, *Qf = nullptr;  // shared FP32 copies (SMEM)
     const double *Pd = nullptr, *Qd = nullptr;  // global FP64 arrays (!SMEM)
     const uint8_t *V = nullptr, *PV = nullptr, *NV = nullptr;
+    if (s_task < 0) next_task(left, &s_task, ntasks, &s_slot);
     for (;;) {
-        if (threadIdx.x == 0) {
-            int c = atomicAdd(counter, 1);
-            int t = -1;
-            if (c < total) {
-                int lo = 0, hi = ntasks;  // first begin > c
-                while (lo < hi) {
-                    int mid = (lo + hi) >> 1;
-                    if (chunk_begin[mid] <= c) lo = mid + 1; else hi = mid;
-                }
-                t = lo - 1;
-                s_next = (c - chunk_begin[t]) * tasks[t].chunk;
-            }
-            ctl.chunk = c;
-            ctl.task = t;
-        }
-        __syncthreads();
-        const int c = ctl.chunk, ti = ctl.task;
-        if (c >= total || ti < 0) break;
+        const int ti = s_task;
+        if (ti < 0) break;
         const BankTask &T = tasks[ti];
         const int n = T.n;
-        if (ti != staged) {
+        {  // stage the task's points
             if (SMEM) {
                 Copy cp[5];
                 char *dst[5];
@@ -552,25 +563,19 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
                 points_mean(Pd, n, oP, red);
                 points_mean(Qd, n, oQ, red);
             }
-            staged = ti;
         }
-        const int ce = min(((c - chunk_begin[ti]) + 1) * T.chunk, T.n_items);  // the chunk's end
-        const int lane = threadIdx.x & 31;
+        const BankWork work = {left + ti, taken};
         if (wide) {
-            if constexpr (SMEM) wide_items(T, Pf, Qf, oP, oQ, seed_rt, item_res, &s_next, ce, ctr);
-            __syncthreads();
-            continue;
+            if constexpr (SMEM)
+                if (warp < pull) wide_items(T, Pf, Qf, oP, oQ, seed_rt, item_res, work, ctr);
         }
-        // the chunk's items go to the warps 32 at a time, so a warp
-        // whose items converged early takes the next group instead of
-        // waiting at the chunk's barrier for the others
-        for (;;) {
-        int gi = 0;
-        if (lane == 0) gi = atomicAdd(&s_next, 32);
-        gi = __shfl_sync(0xffffffffu, gi, 0);
-        if (gi >= ce) break;
+        // the task's items go to the warps 32 at a time, so a warp whose items
+        // converged early takes the next group
+        while (!wide && warp < pull) {
+        const int gi = work.take(T, units);
+        if (gi < 0) break;
         const int pi = gi + lane;  // processing order within the task
-        const bool active = pi < ce;
+        const bool active = pi < T.n_items;
         const int C = T.C > 0 ? T.C : 1;
         // item (seed sk, cutoff ci) and its record slot li = sk*C + ci: seed
         // major (the slot order), or cutoff major (a warp refines one cutoff
@@ -735,7 +740,9 @@ k_bank(const BankTask *__restrict__ tasks, const int *__restrict__ chunk_begin,
             for (int a = 0; a < 3; a++) o[10 + a] = t[a] + oQ[a] - (oP[0] * R[a] + oP[1] * R[3 + a] + oP[2] * R[6 + a]);
         }
         }  // next group of 32 items
-        __syncthreads();
+        // all units taken: no task has any left
+        if (__syncthreads_or(threadIdx.x == 0 && *(volatile int *)taken >= total)) break;
+        next_task(left, &s_task, ntasks, &s_slot);
     }
 }
 
@@ -842,8 +849,8 @@ size_t bank_smem_bytes(int nmax) {
     return 2 * coord + 3 * mask;
 }
 
-void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks,
-                 const ScanOut *scan, int *counter, double *seed_rt, int seed_blocks, double *item_res, int *err,
+void launch_bank(const BankTask *tasks, const float *work_begin, int ntasks,
+                 const ScanOut *scan, int *left, int *taken, double *seed_rt, int seed_blocks, double *item_res, int *err,
                  int nmax, int grid, unsigned long long *ctr, cudaStream_t st) {
     // offset items (no seeds) sum their starts in the thread-per-item form
     const int wide_max = seed_blocks > 0 ? IA_BANK_WIDE * grid : 0;
@@ -855,10 +862,10 @@ void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks,
     }
     size_t sm = bank_smem_bytes(nmax);
     if (sm <= kBankSmemMax) {
-        k_bank<true><<<grid, kBankChunk, sm, st>>>(tasks, chunk_begin, ntasks, scan, counter,
+        k_bank<true><<<grid, kBankChunk, sm, st>>>(tasks, work_begin, ntasks, scan, left, taken,
                                                    seed_rt, item_res, err, nmax, wide_max, ctr);
     } else {
-        k_bank<false><<<grid, kBankChunk, 0, st>>>(tasks, chunk_begin, ntasks, scan, counter,
+        k_bank<false><<<grid, kBankChunk, 0, st>>>(tasks, work_begin, ntasks, scan, left, taken,
                                                    seed_rt, item_res, err, nmax, wide_max, ctr);
     }
 }

@@ -7,7 +7,6 @@
 // evaluate_ss_seeds (indialign_c/ss.h:56-164).  The fill and the traceback of
 // the search's own matrices are in nw_fill.cuh; the NW on an explicit FP64
 // matrix is here.
-#include <climits>
 #include <vector>
 
 #include "../../include/indialign_b200.h"
@@ -323,6 +322,7 @@ constexpr int kManyChains = 16;  // chains per warp from which an SM's CTAs star
 
 struct ChainCtl {
     int task;   // the task in hand, -1: none left
+    int slot;   // of next_task
     int chain;  // one chain per CTA: its index in the task
     int na;     // one chain per CTA: aligned pairs of the last alignment
 };
@@ -353,27 +353,28 @@ IA_DEV void put_rt(double *dst, const double *R, const double *t, int lane) {
 // only when the task has run out and the CTA goes on to the next one with
 // chains left.  (Eight chains per CTA and piece, with a barrier after each,
 // kept the warps waiting for 13 % of their time: k_chain of a learned search
-// of 1024 pairs of L 20-499 80 -> 61 ms, of 64 pairs of L 30-1500 30 -> 22.6.)
-// CTAs start spread over the tasks by their share of the chains; in launches
-// of many chains per warp the CTAs of an SM start together, so that their
-// loops' code and their pair's points are shared (64 pairs of L 40-300: 52.7
-// ms against 58.1 spread singly), in smaller ones apart, so that the longest
-// chains do not share an SM (64 pairs learned: 22.6 against 26.7), and a launch
-// of fewer chains than warps gives each CTA as many warps as chains fall to it.
+// of 1024 pairs of L 40-1000 80 -> 61 ms, of 64 pairs of L 30-1500 30 -> 22.6.)
+// CTAs start spread over the tasks by their share of the cells (by chains, long
+// pairs were left for the end: 48 pairs of L 30-1500 157.6 ms against 154.2
+// with the same loop); in launches of many chains per warp the CTAs of an SM
+// start together, so that their loops' code and their pair's points are shared
+// (64 pairs of L 40-300: 52.7 ms against 58.1 spread singly), in smaller ones
+// apart, so that the longest chains do not share an SM (64 pairs learned: 22.6
+// against 26.7), and a launch of fewer chains than warps gives each CTA as many
+// warps as chains fall to it.
 //
-// A launch of at most coop_max
-// chains leaves most of the chip idle with a warp per chain, and its time is
-// the longest chain's: then a CTA takes one chain at a time, its warps share
-// the fill's stripes, and warp 0 does the rest.  Measured, both with the fill
-// of nw_fill.cuh against a warp per chain with the fill before it: one pair of
-// L = 1203 261 -> 60 ms (its SS and dp_refine stages, one or two alignments at
-// a time, 80 -> 18 ms), learned search of 64 pairs of L 30-1500 285 -> 60 ms.
-// The line lies at one chain per CTA slot of the chip: above it the slots are
-// full either way.
+// A launch of at most coop_max chains leaves most of the chip idle with a warp
+// per chain, and its time is the longest chain's: then a CTA takes one chain
+// at a time, its warps share the fill's stripes, and warp 0 does the rest.
+// Measured, both with the fill of nw_fill.cuh against a warp per chain with
+// the fill before it: one pair of L = 1203 261 -> 60 ms (its SS and dp_refine
+// stages, one or two alignments at a time, 80 -> 18 ms), learned search of 64
+// pairs of L 30-1500 285 -> 60 ms. The line lies at one chain per CTA slot of
+// the chip: above it the slots are full either way.
 template <bool EMIT>
 __global__ void __launch_bounds__(32 * kChainWarps, IA_CHAIN_MINB)
 k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__ chain_begin,
-        int ntasks, const ScanOut *__restrict__ scan, int *left, ChainScratch sc) {
+        const float *__restrict__ work_begin, int ntasks, const ScanOut *__restrict__ scan, int *left, ChainScratch sc) {
     extern __shared__ __align__(16) char smem[];
     __shared__ ChainCtl ctl;
     __shared__ uint64_t bar;
@@ -416,15 +417,11 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             asm("mov.u32 %0, %%nsmid;" : "=r"(places));
             place = min(place, places - 1);
         }
-        const int c = coop ? blockIdx.x : (int)((long long)total * place / places);
-        if (c < total) {
-            int lo = 0, hi = ntasks;  // first begin > c
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (chain_begin[mid] <= c) lo = mid + 1; else hi = mid;
-            }
-            ctl.task = lo - 1;
-            ctl.chain = c - chain_begin[lo - 1];
+        if (!coop) {
+            ctl.task = task_at(work_begin, ntasks, scan->work * (((float)place + 0.5f) / (float)places));
+        } else if ((int)blockIdx.x < total) {
+            ctl.task = task_at(chain_begin, ntasks, (int)blockIdx.x);
+            ctl.chain = (int)blockIdx.x - chain_begin[ctl.task];
         }
     }
     __syncthreads();
@@ -623,21 +620,7 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             if (coop) break;
         }
         if (coop) break;
-        // the next task, in cyclic order, that has chains left; a task without
-        // any never gets some again
-        __syncthreads();
-        if (threadIdx.x == 0) ctl.task = INT_MAX;
-        __syncthreads();
-        for (int d0 = 1; d0 < ntasks; d0 += blockDim.x) {
-            const int d = d0 + (int)threadIdx.x, t = ti + d < ntasks ? ti + d : ti + d - ntasks;
-            const bool some = d < ntasks && *(volatile int *)(left + t) > 0;
-            if (some) atomicMin(&ctl.task, d);
-            if (__syncthreads_or(some)) break;
-        }
-        const int d = ctl.task;
-        __syncthreads();
-        if (threadIdx.x == 0) ctl.task = d == INT_MAX ? -1 : ti + d < ntasks ? ti + d : ti + d - ntasks;
-        __syncthreads();
+        next_task(left, &ctl.task, ntasks, &ctl.slot);
     }
 }
 
@@ -679,12 +662,12 @@ size_t chain_smem_bytes(int pmax, int nmax, int flags) {
     return s;
 }
 
-void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, int ntasks,
-                  const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
+void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, const float *work_begin,
+                  int ntasks, const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
                   cudaStream_t st) {
     const size_t sm = chain_smem_bytes(sc.pmax, sc.nmax, sc.flags);
-    if (emit) k_chain<true><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, ntasks, scan, left, sc);
-    else k_chain<false><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, ntasks, scan, left, sc);
+    if (emit) k_chain<true><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, work_begin, ntasks, scan, left, sc);
+    else k_chain<false><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, work_begin, ntasks, scan, left, sc);
 }
 
 const void *chain_kernel_ptr() { return (const void *)k_chain<false>; }

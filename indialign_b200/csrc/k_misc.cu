@@ -747,37 +747,69 @@ __global__ void k_offset_starts(DevBatch b, double *starts, const int *slot_pair
                                            : (lane < 10 ? R[lane - 1] : t[lane - 10]);
 }
 
-// ---- device scan of per-task chunk counts ---------------------------------
-__global__ void k_scan(const int *counts, int *begins, int ntasks, ScanOut *out, int *counter) {
+// ---- device scan of per-task unit counts (and work estimates) --------------
+__global__ void k_scan(const int *counts, int *begins, const float *work, float *work_begins, int ntasks, ScanOut *out,
+                       int *counter) {
     __shared__ int wsum[32];
+    __shared__ float fsum[32];
     __shared__ int carry, tile_sum;
-    if (threadIdx.x == 0) carry = 0;
+    __shared__ float fcarry, ftile;
+    if (threadIdx.x == 0) {
+        carry = 0;
+        fcarry = 0.f;
+    }
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int base = 0; base < ntasks; base += blockDim.x) {
         const int i = base + threadIdx.x;
         int x = i < ntasks ? counts[i] : 0, inc = x;
+        const float f = work && i < ntasks ? work[i] : 0.f;
+        float finc = f;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(kAll, inc, o);
-            if (lane >= o) inc += y;
+            const int y = __shfl_up_sync(kAll, inc, o);
+            const float g = __shfl_up_sync(kAll, finc, o);
+            if (lane >= o) {
+                inc += y;
+                finc += g;
+            }
         }
-        if (lane == 31) wsum[w] = inc;
+        if (lane == 31) {
+            wsum[w] = inc;
+            fsum[w] = finc;
+        }
         __syncthreads();
         if (threadIdx.x == 0) {
             int s = 0;
-            for (int k = 0; k < nw; k++) { int c = wsum[k]; wsum[k] = s; s += c; }
+            float e = 0.f;
+            for (int k = 0; k < nw; k++) {
+                const int c = wsum[k];
+                const float d = fsum[k];
+                wsum[k] = s;
+                fsum[k] = e;
+                s += c;
+                e += d;
+            }
             tile_sum = s;
+            ftile = e;
         }
         __syncthreads();
         const int tile_total = tile_sum;
-        if (i < ntasks) begins[i] = carry + wsum[w] + inc - x;
+        const float ftotal = ftile;
+        if (i < ntasks) {
+            begins[i] = carry + wsum[w] + inc - x;
+            if (work) work_begins[i] = fcarry + fsum[w] + (finc - f);
+        }
         __syncthreads();
-        if (threadIdx.x == 0) carry += tile_total;
+        if (threadIdx.x == 0) {
+            carry += tile_total;
+            fcarry += ftotal;
+        }
         __syncthreads();
     }
     if (threadIdx.x == 0) {
         out->total_chunks = carry;
+        out->work = fcarry;
         out->items = out->items_acc;
         out->items_acc = 0;
         *counter = 0;
@@ -816,9 +848,9 @@ void launch_offset_starts(const DevBatch &b, double *starts, const int *slot_pai
     if (nslots > 0)
         k_offset_starts<<<(nslots * 32 + 255) / 256, 256, 0, st>>>(b, starts, slot_pair, slot_idx, nslots);
 }
-void launch_scan(const int *counts, int *begins, int ntasks, ScanOut *out, int *counter,
-                 cudaStream_t st) {
-    k_scan<<<1, 1024, 0, st>>>(counts, begins, ntasks, out, counter);
+void launch_scan(const int *counts, int *begins, const float *work, float *work_begins, int ntasks, ScanOut *out,
+                 int *counter, cudaStream_t st) {
+    k_scan<<<1, 1024, 0, st>>>(counts, begins, work, work_begins, ntasks, out, counter);
 }
 
 }  // namespace ia

@@ -149,10 +149,10 @@ __global__ void k_plan_bank(DevBatch b, PlanCtx c) {
     }
     T.n_items = on ? T.K * T.C : 0;
     const Tune &tn = c.tune.of(I.N);  // the shape of the pair's length bucket
-    T.chunk = tn.bank_chunk;
     T.cutoff_major = tn.bank_cutoff_major;
     c.btasks[s] = T;
-    c.counts[s] = (T.n_items + T.chunk - 1) / T.chunk;
+    c.counts[s] = (T.n_items + kBankUnit - 1) / kBankUnit;
+    c.work[s] = T.n_items > 0 ? (float)T.n_items * (float)(T.n + 64) : 0.f;
     const unsigned together = __activemask();
     const int items = __reduce_add_sync(together, T.n_items);
     if (items > 0 && (threadIdx.x & 31) == __ffs(together) - 1) atomicAdd(&c.scan->items_acc, items);
@@ -248,6 +248,7 @@ __global__ void k_plan_chain(DevBatch b, PlanCtx c) {
         rec_ident(S.rec[REC_STAGE], kScoreInit);
     c.ctasks[s] = T;
     c.counts[s] = T.n_chains;
+    c.work[s] = T.n_chains > 0 ? (float)T.n_chains * (float)(I.plen + 64) * (float)(I.nlen + 64) : 0.f;
 }
 
 // ---- chain reductions (warp per pair) ---------------------------------------

@@ -76,15 +76,18 @@ void launch_repack(const DevBatch &b, const int *off_in, const double *pred, con
                    const uint8_t *v, const uint8_t *pv, const uint8_t *nv, cudaStream_t st);
 void launch_snapshot(const DevBatch &b, double *snap, int stage, int stages, cudaStream_t st);
 void launch_export(const DevBatch &b, double *out, cudaStream_t st);
-void launch_scan(const int *counts, int *begins, int ntasks, ScanOut *out, int *counter,
-                 cudaStream_t st);
+// work, work_begins: may be null
+void launch_scan(const int *counts, int *begins, const float *work, float *work_begins, int ntasks, ScanOut *out,
+                 int *counter, cudaStream_t st);
 
 // k_bank.cu
 size_t bank_smem_bytes(int nmax);
 // seed_rt: 12 doubles per seed at item_base / kDetC; seed_blocks: blocks of
 // 128 seeds of the task with most (0: a launch of offset items)
-void launch_bank(const BankTask *tasks, const int *chunk_begin, int ntasks, const ScanOut *scan,
-                 int *counter, double *seed_rt, int seed_blocks, double *item_res, int *err, int nmax, int grid,
+// left: per task its units of kBankUnit items, counted down by the launch;
+// taken: 0, counts the units taken
+void launch_bank(const BankTask *tasks, const float *work_begin, int ntasks, const ScanOut *scan,
+                 int *left, int *taken, double *seed_rt, int seed_blocks, double *item_res, int *err, int nmax, int grid,
                  unsigned long long *ctr, cudaStream_t st);
 void launch_reduce_bank(const BankTask *tasks, int ntasks, bool short_lists, const double *item_res,
                         PairState *state, cudaStream_t st);
@@ -107,8 +110,8 @@ struct ChainScratch {
 };
 size_t chain_smem_bytes(int pmax, int nmax, int flags);
 // left: per task its number of chains, counted down by the launch
-void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, int ntasks,
-                  const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
+void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, const float *work_begin,
+                  int ntasks, const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
                   cudaStream_t st);
 cudaError_t chain_set_attributes();
 const void *chain_kernel_ptr();

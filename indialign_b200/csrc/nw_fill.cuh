@@ -193,9 +193,11 @@ IA_DEV float3 moved_row(const FillArgs &A, int i, bool raw) {
 }
 
 // Fill the trace of the stripes of warp w.  Called by whole warps; with W > 1
-// by all W warps of the alignment, prog[] zeroed before.
+// by all W warps of the alignment, prog[] zeroed before.  Inlined: as a call it
+// gets the registers that the chain loop leaves over (k_chain of 48 pairs of L
+// 30-1500 151 ms against 152 to 159, by what lives around it).
 template <int SMODE, int R>
-__device__ __noinline__ void nw_fill(const FillArgs &A, const FillGeom G, int w) {
+IA_DEV void nw_fill(const FillArgs &A, const FillGeom G, int w) {
     constexpr unsigned kFull = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int plen = A.plen, nlen = A.nlen, W = G.W, S = G.S;

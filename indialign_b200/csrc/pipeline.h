@@ -7,8 +7,9 @@
 //
 // Every stage is a fixed launch sequence
 //   plan kernel (per task slot: work count, 0 when gated off)
-//   -> scan (chunk begins + total, on device)
-//   -> persistent work kernel pulling chunks from a device counter
+//   -> scan (where tasks begin, by units and by estimated work, on device)
+//   -> persistent work kernel whose CTAs go from task to task, the warps
+//      taking units of the task in hand from its count
 //   -> reduce / per-pair glue kernels that apply the reference's
 //      first-max / strict-'>' update rules,
 // so no host round trip is needed between stages.
@@ -29,9 +30,10 @@ constexpr int kMaxSeeds = 1024;    // fragment windows (<= 1+9*101) + anchors
 constexpr int kMaxBitSeeds = 32;   // anchor masks (<= 6 radii x 5) + top-k mask
 constexpr int kRec = 13;           // {score, R[9], t[3]}
 constexpr int kBankChunk = 128;    // threads of a bank CTA (4 warps x 32)
+constexpr int kBankUnit = 8;       // items of a bank task are counted and taken in units of 8
 // Kernel shape knobs of one length bucket (tuning table, search.cu).
 struct Tune {
-    int bank_chunk = 256;       // bank items per CTA chunk (multiple of 32)
+    int bank_chunk = 256;       // accepted and kept, without effect: warps take items as they go
     int bank_cutoff_major = 1;  // bank item order: 1 cutoff major, 0 seed major
     int chain_chunk = 16;       // accepted and kept, without effect: warps take chains one at a time
     int chain_smem_trace = 1;   // NW traces in shared memory when they fit
@@ -114,7 +116,6 @@ struct BankTask {
     double *out;         // explicit output record (used when out_rec < 0)
     int n_items;         // K*C (0 = task inactive)
     int item_base;       // first item in the launch's item space (set by scan)
-    int chunk;           // items per CTA chunk (the pair's length bucket)
     int cutoff_major;    // item order: 1 cutoff major, 0 seed major
 };
 
@@ -162,6 +163,7 @@ struct ScanOut {
     int error;           // device-side error flags (bounded waits, caps)
     int items;           // a bank launch's items
     int items_acc;       // ... while its plan kernel counts them
+    float work;          // the launch's work (estimates of the tasks)
 };
 
 struct PlanCtx {
@@ -171,7 +173,8 @@ struct PlanCtx {
     const long long *base;  // slot -> first result record / item
     BankTask *btasks;
     ChainTask *ctasks;
-    int *counts;            // slot -> work chunks
+    int *counts;            // slot -> units of work
+    float *work;            // slot -> estimate of its work
     ScanOut *scan;          // the plan adds up a bank launch's items here
     double *alP, *alQ;      // aligned sets (2 per pair)
     double *chain_res;      // LITE chain results

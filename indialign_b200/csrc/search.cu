@@ -94,6 +94,7 @@ struct Ctx {
     DBuf<BankTask> btasks;
     DBuf<ChainTask> ctasks;
     DBuf<int> counts, begins, counter;
+    DBuf<float> work, work_begins;
     DBuf<ScanOut> scan;
     DBuf<double> item_res, seed_rt, chain_res, alP, alQ, thread_rec, off_start, off_res, out, snap;
     DBuf<int> lay_i, gidx, omap;
@@ -460,6 +461,8 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     CK(c_->ctasks.ensure(maxtasks));
     CK(c_->counts.ensure(maxtasks));
     CK(c_->begins.ensure(maxtasks));
+    CK(c_->work.ensure(maxtasks));
+    CK(c_->work_begins.ensure(maxtasks));
     CK(c_->scan.ensure(1));
     CK(c_->counter.ensure(1));
     CK(c_->item_res.ensure((size_t)(max_items_ > 0 ? max_items_ : 1) * kRec));
@@ -540,6 +543,7 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
     pc.btasks = c_->btasks.p;
     pc.scan = c_->scan.p;
     pc.counts = c_->counts.p;
+    pc.work = c_->work.p;
     pc.alP = c_->alP.p;
     pc.alQ = c_->alQ.p;
     pc.recs = recs;
@@ -554,13 +558,9 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
                                                      kBankChunk, sm <= kBankSmemMax ? sm : 0));
     if (per_sm < 1) per_sm = 1;
     const int grid = c_->sms * per_sm;
-    // a launch that cannot fill the grid with 256-item chunks takes 128, one
-    // group of 32 per warp: its time is the longest warp's, and a second group
-    // would come on top; one of few items 32, one group of 8 per warp
-    const int most = L.total <= 32LL * grid ? 32 : L.total <= 256LL * grid ? kBankChunk : 4096;
-    for (Tune &t : pc.tune.t) t.bank_chunk = std::min(t.bank_chunk, most);
     launch_plan_bank(b, pc, c_->stream);
-    launch_scan(c_->counts.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->stream);
+    launch_scan(c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counter.p,
+                c_->stream);
     launches_ += kind == BK_GAPLESS ? 4 : 5;
     bank_launches_++;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -575,7 +575,7 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
                       : kind == BK_TOPK  ? 1
                       : kind == BK_THREAD ? kthread_
                                           : kdet_max(pmax < nmax ? pmax : nmax);
-    launch_bank(c_->btasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->seed_rt.p,
+    launch_bank(c_->btasks.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counts.p, c_->counter.p, c_->seed_rt.p,
                 (seeds + kBankChunk - 1) / kBankChunk, c_->item_res.p, c_->err.p,
                 Nmax, grid, b.ctr, c_->stream);
     if (timing) {
@@ -598,6 +598,7 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
     pc.base = L.d_base;
     pc.ctasks = c_->ctasks.p;
     pc.counts = c_->counts.p;
+    pc.work = c_->work.p;
     pc.alP = c_->alP.p;
     pc.alQ = c_->alQ.p;
     pc.chain_res = c_->chain_res.p;
@@ -608,7 +609,8 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
     pc.wlist = wlist;
     pc.tune = cfg_.tune;
     launch_plan_chain(b, pc, c_->stream);
-    launch_scan(c_->counts.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counter.p, c_->stream);
+    launch_scan(c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counter.p,
+                c_->stream);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing) {
         e0 = new_event();
@@ -618,7 +620,7 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
     const bool emit = kind == CH_SS2 || kind == CH_SS4 || kind == CH_DP_EMIT;
     const ChainScratch sc = {c_->gtrace.p, trace_words_, c_->gbh.p,    c_->gcol.p,       c_->gal.p,
                              pmax,         nmax,         chain_flags_, chain_grid_};
-    launch_chain(b, c_->ctasks.p, c_->begins.p, L.ntasks, c_->scan.p, c_->counts.p, sc, chain_grid_, emit,
+    launch_chain(b, c_->ctasks.p, c_->begins.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counts.p, sc, chain_grid_, emit,
                  c_->stream);
     if (timing) {
         cudaEventRecord(e1, c_->stream);
@@ -697,7 +699,7 @@ int Runner::rank_stage(int kind, int det_ss) {
             CK(cudaMemsetAsync(c_->wlabel.p + koff_[kind], 0xff, (size_t)L_cand[kind].total * sizeof(float), st));
     }
     launch_plan_rank(b, ra, c_->counts.p, st);
-    launch_scan(c_->counts.p, c_->begins.p, ra.ntasks, c_->scan.p, c_->counter.p, st);
+    launch_scan(c_->counts.p, c_->begins.p, nullptr, nullptr, ra.ntasks, c_->scan.p, c_->counter.p, st);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing) {
         e0 = new_event();

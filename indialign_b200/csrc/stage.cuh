@@ -2,6 +2,7 @@
 // completed on an mbarrier, with bounded waits, and a plain-load fallback
 // for ranges the bulk engine cannot take (unaligned or odd sizes).
 #pragma once
+#include <climits>
 #include <stdint.h>
 #include "pipeline.h"
 
@@ -109,6 +110,52 @@ IA_DEV void stage_copies(const Copy *cp, char *const *dst, int ncopies,
         }
         __syncthreads();
     }
+}
+
+// The task at position c of a launch (begin: where the tasks begin, ascending).
+template <typename T>
+IA_DEV int task_at(const T *__restrict__ begin, int ntasks, T c) {
+    int lo = 0, hi = ntasks;  // first begin > c
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (begin[mid] <= c) lo = mid + 1; else hi = mid;
+    }
+    return max(lo - 1, 0);
+}
+
+// Where a CTA begins to look for work: the task at its share of the launch's
+// work (estimated, begin: where the tasks begin), so that tasks of unlike sizes
+// end together.  Returns ~task if that one has no units left.  One thread.
+IA_DEV int first_task(const float *__restrict__ begin, const int *left, int ntasks, float work, uint32_t place,
+                      uint32_t places) {
+    const int t = task_at(begin, ntasks, work * (((float)place + 0.5f) / (float)places));
+    return *(volatile const int *)(left + t) > 0 ? t : ~t;
+}
+
+// *task (~t or t) becomes the next task after t, in cyclic order, that has work
+// left, or -1; a task without any never gets some again.  Called by the whole
+// CTA; task and slot are shared.
+IA_DEV void next_task(const int *left, int *task, int ntasks, int *slot) {
+    __syncthreads();
+    const int ti = *task < 0 ? ~*task : *task;
+    if (threadIdx.x == 0) *slot = INT_MAX;
+    __syncthreads();
+#pragma unroll 1
+    for (int d0 = 1; d0 < ntasks; d0 += 4 * blockDim.x) {
+        int best = INT_MAX;
+#pragma unroll
+        for (int k = 3; k >= 0; k--) {
+            const int d = d0 + k * (int)blockDim.x + (int)threadIdx.x, t = ti + d < ntasks ? ti + d : ti + d - ntasks;
+            if (d < ntasks && *(volatile const int *)(left + t) > 0) best = d;
+        }
+        if (best != INT_MAX) atomicMin(slot, best);
+        if (__syncthreads_or(best != INT_MAX)) break;
+    }
+    if (threadIdx.x == 0) {
+        const int d = *slot;
+        *task = d == INT_MAX ? -1 : ti + d < ntasks ? ti + d : ti + d - ntasks;
+    }
+    __syncthreads();
 }
 
 }  // namespace ia
