@@ -4,6 +4,8 @@
 #include "dmath.cuh"
 #include "pipeline.h"
 #include "kernels.h"
+#include "rescore.cuh"
+#include "scan.cuh"
 #include "sched.cuh"
 
 namespace ia {
@@ -677,31 +679,6 @@ __global__ void k_weighted(DevBatch b) {
     }
 }
 
-// ---- same-index rescoring: tm_score_no_d8 over the full pair
-// (indialign_c/indialign.cpp:86-88) -------------------------------------------
-IA_DEV double pair_tm(const DevBatch &b, const PairInfo &I, const double *rec, int lane) {
-    const int N = I.N, off = I.off;
-    const double *P = b.pred + 3 * (size_t)off, *Q = b.nat + 3 * (size_t)off;
-    const uint8_t *v = b.v + off;
-    const double *R = rec + 1, *t = rec + 10;
-    const double inv = 1.0 / fmax(I.d0 * I.d0, 1e-12);
-    double s = 0.0;
-    for (int i = lane; i < N; i += 32)
-        if (v[i]) s += tm_term(dist2(R, t, P[3 * i], P[3 * i + 1], P[3 * i + 2], Q[3 * i], Q[3 * i + 1], Q[3 * i + 2]), inv);
-    return warp_sum(s) / fmax(I.lnorm, 1.0);
-}
-
-__global__ void k_rescore(DevBatch b, int slot, int need_flag) {
-    const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (p >= b.n) return;
-    const PairInfo &I = b.info[p];
-    PairState &S = b.state[p];
-    if (I.status != 0 || (need_flag && !S.flag)) return;
-    double s = pair_tm(b, I, S.rec[slot], lane);
-    __syncwarp();
-    if (lane == 0) S.rec[slot][0] = s;
-}
-
 __global__ void k_rescore_list(DevBatch b, double *recs, const int *rec_pair, int nrec) {
     const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (r >= nrec) return;
@@ -748,73 +725,7 @@ __global__ void k_offset_starts(DevBatch b, double *starts, const int *slot_pair
 }
 
 // ---- device scan of per-task unit counts (and work estimates) --------------
-__global__ void k_scan(const int *counts, int *begins, const float *work, float *work_begins, int ntasks, ScanOut *out,
-                       int *counter) {
-    __shared__ int wsum[32];
-    __shared__ float fsum[32];
-    __shared__ int carry, tile_sum;
-    __shared__ float fcarry, ftile;
-    if (threadIdx.x == 0) {
-        carry = 0;
-        fcarry = 0.f;
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int base = 0; base < ntasks; base += blockDim.x) {
-        const int i = base + threadIdx.x;
-        int x = i < ntasks ? counts[i] : 0, inc = x;
-        const float f = work && i < ntasks ? work[i] : 0.f;
-        float finc = f;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kAll, inc, o);
-            const float g = __shfl_up_sync(kAll, finc, o);
-            if (lane >= o) {
-                inc += y;
-                finc += g;
-            }
-        }
-        if (lane == 31) {
-            wsum[w] = inc;
-            fsum[w] = finc;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int s = 0;
-            float e = 0.f;
-            for (int k = 0; k < nw; k++) {
-                const int c = wsum[k];
-                const float d = fsum[k];
-                wsum[k] = s;
-                fsum[k] = e;
-                s += c;
-                e += d;
-            }
-            tile_sum = s;
-            ftile = e;
-        }
-        __syncthreads();
-        const int tile_total = tile_sum;
-        const float ftotal = ftile;
-        if (i < ntasks) {
-            begins[i] = carry + wsum[w] + inc - x;
-            if (work) work_begins[i] = fcarry + fsum[w] + (finc - f);
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            carry += tile_total;
-            fcarry += ftotal;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        out->total_chunks = carry;
-        out->work = fcarry;
-        out->items = out->items_acc;
-        out->items_acc = 0;
-        *counter = 0;
-    }
-}
+__global__ void k_scan(ScanArgs a, int ntasks) { scan_tasks(a, ntasks); }
 
 // ---- launch wrappers ------------------------------------------------------
 void launch_prep(const DevBatch &b, int use_frag, cudaStream_t st) {
@@ -836,9 +747,6 @@ void launch_topk(const DevBatch &b, cudaStream_t st) {
 void launch_weighted(const DevBatch &b, cudaStream_t st) {
     if (b.n > 0) k_weighted<<<(b.n * 32 + 255) / 256, 256, 0, st>>>(b);
 }
-void launch_rescore(const DevBatch &b, int slot, int need_flag, cudaStream_t st) {
-    if (b.n > 0) k_rescore<<<(b.n * 32 + 255) / 256, 256, 0, st>>>(b, slot, need_flag);
-}
 void launch_rescore_list(const DevBatch &b, double *recs, const int *rec_pair, int nrec,
                          cudaStream_t st) {
     if (nrec > 0) k_rescore_list<<<(nrec * 32 + 255) / 256, 256, 0, st>>>(b, recs, rec_pair, nrec);
@@ -848,10 +756,7 @@ void launch_offset_starts(const DevBatch &b, double *starts, const int *slot_pai
     if (nslots > 0)
         k_offset_starts<<<(nslots * 32 + 255) / 256, 256, 0, st>>>(b, starts, slot_pair, slot_idx, nslots);
 }
-void launch_scan(const int *counts, int *begins, const float *work, float *work_begins, int ntasks, ScanOut *out,
-                 int *counter, cudaStream_t st) {
-    k_scan<<<1, 1024, 0, st>>>(counts, begins, work, work_begins, ntasks, out, counter);
-}
+void launch_scan(const ScanArgs &a, int ntasks, cudaStream_t st) { k_scan<<<1, 1024, 0, st>>>(a, ntasks); }
 
 }  // namespace ia
 

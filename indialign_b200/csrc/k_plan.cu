@@ -8,6 +8,8 @@
 #include "dmath.cuh"
 #include "pipeline.h"
 #include "kernels.h"
+#include "rescore.cuh"
+#include "scan.cuh"
 #include "sched.cuh"
 
 namespace ia {
@@ -21,8 +23,7 @@ IA_DEV void rec_ident(double *d, double score) {
 }
 
 // ---- bank plans -------------------------------------------------------------
-__global__ void k_plan_bank(DevBatch b, PlanCtx c) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+IA_DEV void plan_bank(const DevBatch &b, const PlanCtx &c, int s) {
     if (s >= c.ntasks) return;
     const int p = c.pair ? c.pair[s] : s;
     const int aux = c.aux ? c.aux[s] : 0;
@@ -159,8 +160,7 @@ __global__ void k_plan_bank(DevBatch b, PlanCtx c) {
 }
 
 // ---- chain plans ------------------------------------------------------------
-__global__ void k_plan_chain(DevBatch b, PlanCtx c) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+IA_DEV void plan_chain(const DevBatch &b, const PlanCtx &c, int s) {
     if (s >= c.ntasks) return;
     const int p = c.pair ? c.pair[s] : s;
     const PairInfo &I = b.info[p];
@@ -251,6 +251,24 @@ __global__ void k_plan_chain(DevBatch b, PlanCtx c) {
     c.work[s] = T.n_chains > 0 ? (float)T.n_chains * (float)(I.plen + 64) * (float)(I.nlen + 64) : 0.f;
 }
 
+template <bool BANK>
+__global__ void __launch_bounds__(128) k_plan(DevBatch b, PlanCtx c) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (BANK) plan_bank(b, c, s);
+    else plan_chain(b, c, s);
+}
+
+// Plan and scan in one launch, a thread per task, where one CTA holds them all
+// (a pair of 64 residues 1.57 -> 1.49 ms).
+constexpr int kPlanScan = 512;
+template <bool BANK>
+__global__ void __launch_bounds__(kPlanScan) k_plan_scan(DevBatch b, PlanCtx c, ScanArgs a) {
+    if (BANK) plan_bank(b, c, threadIdx.x);
+    else plan_chain(b, c, threadIdx.x);
+    __syncthreads();
+    scan_tasks(a, c.ntasks);
+}
+
 // ---- chain reductions (warp per pair) ---------------------------------------
 // A dp_refine's best over both gap chains: each chain starts from score 0 /
 // identity and replaces on strictly greater, gap -0.6 first
@@ -313,12 +331,7 @@ __global__ void k_reduce_chain(DevBatch b, PlanCtx c) {
 }
 
 // ---- per-pair glue ------------------------------------------------------------
-__global__ void k_glue(DevBatch b, GlueArgs a) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= b.n) return;
-    const PairInfo &I = b.info[p];
-    PairState &S = b.state[p];
-    if (I.status != 0) return;
+IA_DEV void glue_step(const GlueArgs &a, const PairInfo &I, PairState &S, int p) {
     double *best = S.rec[REC_BEST];
     switch (a.op) {
     case G_GATE:  // rescue trigger on the running best (indialign.cpp:129,137,145)
@@ -416,18 +429,53 @@ __global__ void k_glue(DevBatch b, GlueArgs a) {
     }
 }
 
-// ---- launch wrappers ------------------------------------------------------
-void launch_plan_bank(const DevBatch &b, const PlanCtx &c, cudaStream_t st) {
-    if (c.ntasks > 0) k_plan_bank<<<(c.ntasks + 127) / 128, 128, 0, st>>>(b, c);
+// A warp per pair goes through the steps of the list: lane 0 a step of records
+// and flags, all lanes a rescoring.  One by one, the steps between two searches
+// of a stage were up to five dependent launches of a few microseconds each (a
+// pair of 64 residues 1.64 -> 1.57 ms together).
+__global__ void k_glue(DevBatch b, GlueList l) {
+    const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (p >= b.n) return;
+    const PairInfo &I = b.info[p];
+    PairState &S = b.state[p];
+    if (I.status != 0) return;
+    for (int k = 0; k < l.n; k++) {
+        const GlueArgs &a = l.a[k];
+        if (a.op != G_RESCORE) {
+            if (lane == 0) glue_step(a, I, S, p);
+        } else if (!a.need_flag || S.flag) {
+            const double s = pair_tm(b, I, S.rec[a.slot], lane);
+            __syncwarp();
+            if (lane == 0) S.rec[a.slot][0] = s;
+        }
+        __syncwarp();
+    }
 }
-void launch_plan_chain(const DevBatch &b, const PlanCtx &c, cudaStream_t st) {
-    if (c.ntasks > 0) k_plan_chain<<<(c.ntasks + 127) / 128, 128, 0, st>>>(b, c);
+
+// ---- launch wrappers ------------------------------------------------------
+int launch_plan_bank(const DevBatch &b, const PlanCtx &c, const ScanArgs &a, cudaStream_t st) {
+    if (c.ntasks <= kPlanScan) {
+        k_plan_scan<true><<<1, (c.ntasks + 31) & ~31, 0, st>>>(b, c, a);
+        return 1;
+    }
+    k_plan<true><<<(c.ntasks + 127) / 128, 128, 0, st>>>(b, c);
+    launch_scan(a, c.ntasks, st);
+    return 2;
+}
+int launch_plan_chain(const DevBatch &b, const PlanCtx &c, const ScanArgs &a, cudaStream_t st) {
+    if (c.ntasks <= kPlanScan) {
+        k_plan_scan<false><<<1, (c.ntasks + 31) & ~31, 0, st>>>(b, c, a);
+        return 1;
+    }
+    k_plan<false><<<(c.ntasks + 127) / 128, 128, 0, st>>>(b, c);
+    launch_scan(a, c.ntasks, st);
+    return 2;
 }
 void launch_reduce_chain(const DevBatch &b, const PlanCtx &c, cudaStream_t st) {
     if (c.ntasks > 0) k_reduce_chain<<<(c.ntasks * 32 + 255) / 256, 256, 0, st>>>(b, c);
 }
-void launch_glue(const DevBatch &b, const GlueArgs &a, cudaStream_t st) {
-    if (b.n > 0) k_glue<<<(b.n + 127) / 128, 128, 0, st>>>(b, a);
+void launch_glue(const DevBatch &b, const GlueList &l, cudaStream_t st) {
+    if (b.n > 0) k_glue<<<(b.n + 3) / 4, 128, 0, st>>>(b, l);
 }
 
 }  // namespace ia

@@ -67,7 +67,6 @@ cudaError_t misc_set_attributes();
 void launch_ss(const DevBatch &b, cudaStream_t st);
 void launch_topk(const DevBatch &b, cudaStream_t st);
 void launch_weighted(const DevBatch &b, cudaStream_t st);
-void launch_rescore(const DevBatch &b, int slot, int need_flag, cudaStream_t st);
 void launch_rescore_list(const DevBatch &b, double *recs, const int *rec_pair, int nrec,
                          cudaStream_t st);
 void launch_offset_starts(const DevBatch &b, double *starts, const int *slot_pair,
@@ -76,9 +75,17 @@ void launch_repack(const DevBatch &b, const int *off_in, const double *pred, con
                    const uint8_t *v, const uint8_t *pv, const uint8_t *nv, cudaStream_t st);
 void launch_snapshot(const DevBatch &b, double *snap, int stage, int stages, cudaStream_t st);
 void launch_export(const DevBatch &b, double *out, cudaStream_t st);
-// work, work_begins: may be null
-void launch_scan(const int *counts, int *begins, const float *work, float *work_begins, int ntasks, ScanOut *out,
-                 int *counter, cudaStream_t st);
+// counts -> begins, work -> work_begins (both may be null), totals to out, and
+// the launch's counter to 0
+struct ScanArgs {
+    const int *counts;
+    int *begins;
+    const float *work;
+    float *work_begins;
+    ScanOut *out;
+    int *counter;
+};
+void launch_scan(const ScanArgs &a, int ntasks, cudaStream_t st);
 
 // k_bank.cu
 size_t bank_smem_bytes(int nmax);
@@ -260,9 +267,10 @@ void launch_adam(float *w, const float *g, float *m, float *v, int n, int first,
                  float b2, float eps, float bc1, float bc2, cudaStream_t st);
 
 // k_plan.cu
-void launch_plan_bank(const DevBatch &b, const PlanCtx &c, cudaStream_t st);
-void launch_plan_chain(const DevBatch &b, const PlanCtx &c, cudaStream_t st);
+// plan and scan; returns the number of launches
+int launch_plan_bank(const DevBatch &b, const PlanCtx &c, const ScanArgs &a, cudaStream_t st);
+int launch_plan_chain(const DevBatch &b, const PlanCtx &c, const ScanArgs &a, cudaStream_t st);
 void launch_reduce_chain(const DevBatch &b, const PlanCtx &c, cudaStream_t st);
-void launch_glue(const DevBatch &b, const GlueArgs &a, cudaStream_t st);
+void launch_glue(const DevBatch &b, const GlueList &l, cudaStream_t st);
 
 }  // namespace ia

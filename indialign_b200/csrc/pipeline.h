@@ -155,7 +155,7 @@ enum ChainKind { CH_SS2 = 0, CH_SS4, CH_DP_EMIT, CH_LOCAL, CH_THREAD, CH_SINGLE,
 enum GlueOp {
     G_GATE = 0, G_STAGE_UPDATE, G_SS_BEGIN, G_SS_DET, G_DP_STEP, G_DP_END, G_SS_DP,
     G_SS4_START, G_SS_FINISH, G_DPF_BEGIN, G_DPF_UPDATE, G_TMP_UPDATE, G_IDP_START,
-    G_EXTRA_START, G_FLAG_ON, G_OFFDP_UPDATE
+    G_EXTRA_START, G_FLAG_ON, G_OFFDP_UPDATE, G_RESCORE
 };
 
 struct ScanOut {
@@ -192,6 +192,14 @@ struct GlueArgs {
     int dp_iter;
     const double *recs;
     const int *idx;         // per pair first record of `recs`
+    int slot, need_flag;    // G_RESCORE: the record, and whether only pairs with their flag set
+};
+
+// Consecutive per-pair steps of one launch.
+constexpr int kMaxGlue = 6;
+struct GlueList {
+    int n;
+    GlueArgs a[kMaxGlue];
 };
 
 // ---- learned window ranker ---------------------------------------------------

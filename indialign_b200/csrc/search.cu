@@ -233,6 +233,7 @@ class Runner {
     DevBatch b;
     double *snap = nullptr;  // device [n*kTrace*13] or nullptr
     void mark(int stage) {
+        if (snap || timing) flush();  // the stage's steps belong before its mark
         launch_snapshot(b, snap, stage, kTrace, c_->stream);
         if (snap) launches_++;
         stage_event(stage + 1);
@@ -296,6 +297,10 @@ class Runner {
         return cfg_.mode == INDIALIGN_MODE_LEARNED && ranked(kind, det_ss) ? c_->wlist.p : nullptr;
     }
     int glue(int op, double thr = 0.0, const double *recs = nullptr, const int *idx = nullptr);
+    int rescore(int slot, int need_flag);
+    int glue(const GlueArgs &a);
+    int flush();
+    GlueList pending_ = {};
     int dp_full(int det_ss);
 
     Ctx *c_;
@@ -534,6 +539,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
 int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, const int *wcount,
                  const int *wlist) {
     if (L.ntasks <= 0) return INDIALIGN_OK;
+    if (const int rc = flush()) return rc;
     PlanCtx pc = {};
     pc.kind = kind;
     pc.ntasks = L.ntasks;
@@ -558,10 +564,9 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
                                                      kBankChunk, sm <= kBankSmemMax ? sm : 0));
     if (per_sm < 1) per_sm = 1;
     const int grid = c_->sms * per_sm;
-    launch_plan_bank(b, pc, c_->stream);
-    launch_scan(c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counter.p,
-                c_->stream);
-    launches_ += kind == BK_GAPLESS ? 4 : 5;
+    launches_ += launch_plan_bank(b, pc, {c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, c_->scan.p, c_->counter.p},
+                                  c_->stream);
+    launches_ += kind == BK_GAPLESS ? 2 : 3;
     bank_launches_++;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing) {
@@ -590,6 +595,7 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
 int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, bool reduce,
                   const int *wcount, const int *wlist) {
     if (L.ntasks <= 0) return INDIALIGN_OK;
+    if (const int rc = flush()) return rc;
     PlanCtx pc = {};
     pc.kind = kind;
     pc.ntasks = L.ntasks;
@@ -608,9 +614,8 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
     pc.wcount = wcount;
     pc.wlist = wlist;
     pc.tune = cfg_.tune;
-    launch_plan_chain(b, pc, c_->stream);
-    launch_scan(c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counter.p,
-                c_->stream);
+    launches_ += launch_plan_chain(b, pc, {c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, c_->scan.p, c_->counter.p},
+                                   c_->stream);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing) {
         e0 = new_event();
@@ -627,12 +632,13 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
         chain_ev.push_back({e0, e1});
     }
     if (reduce) launch_reduce_chain(b, pc, c_->stream);
-    launches_ += reduce ? 4 : 3;
+    launches_ += reduce ? 2 : 1;
     chain_launches_++;
     CK(cudaGetLastError());
     return INDIALIGN_OK;
 }
 
+// Per-pair steps wait for the next launch that needs them and go together.
 int Runner::glue(int op, double thr, const double *recs, const int *idx) {
     GlueArgs a = {};
     a.op = op;
@@ -640,7 +646,26 @@ int Runner::glue(int op, double thr, const double *recs, const int *idx) {
     a.dp_iter = cfg_.dp_iter;
     a.recs = recs;
     a.idx = idx;
-    launch_glue(b, a, c_->stream);
+    return glue(a);
+}
+
+int Runner::rescore(int slot, int need_flag) {
+    GlueArgs a = {};
+    a.op = G_RESCORE;
+    a.slot = slot;
+    a.need_flag = need_flag;
+    return glue(a);
+}
+
+int Runner::glue(const GlueArgs &a) {
+    pending_.a[pending_.n++] = a;
+    return pending_.n == kMaxGlue ? flush() : INDIALIGN_OK;
+}
+
+int Runner::flush() {
+    if (pending_.n == 0) return INDIALIGN_OK;
+    launch_glue(b, pending_, c_->stream);
+    pending_.n = 0;
     launches_++;
     CK(cudaGetLastError());
     return INDIALIGN_OK;
@@ -691,6 +716,7 @@ RankArgs Runner::rank_args(int kind, int det_ss) {
 
 int Runner::rank_stage(int kind, int det_ss) {
     if (!ranked(kind, det_ss)) return INDIALIGN_OK;
+    if (const int rc = flush()) return rc;
     cudaStream_t st = c_->stream;
     const RankArgs ra = rank_args(kind, det_ss);
     if (kind == CAND_DET || kind == CAND_MAIN) {  // hold this search only (NaN beyond its seeds)
@@ -699,7 +725,7 @@ int Runner::rank_stage(int kind, int det_ss) {
             CK(cudaMemsetAsync(c_->wlabel.p + koff_[kind], 0xff, (size_t)L_cand[kind].total * sizeof(float), st));
     }
     launch_plan_rank(b, ra, c_->counts.p, st);
-    launch_scan(c_->counts.p, c_->begins.p, nullptr, nullptr, ra.ntasks, c_->scan.p, c_->counter.p, st);
+    launch_scan({c_->counts.p, c_->begins.p, nullptr, nullptr, c_->scan.p, c_->counter.p}, ra.ntasks, st);
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing) {
         e0 = new_event();
@@ -741,6 +767,7 @@ SelectArgs Runner::select_args(int kind, int det_ss) {
 // every candidate's refined score.
 int Runner::after_stage(int kind, const CandRes &r, int det_ss) {
     if (!ranked(kind, det_ss)) return INDIALIGN_OK;
+    if (const int rc = flush()) return rc;
     cudaStream_t st = c_->stream;
     if (cfg_.mode == INDIALIGN_MODE_LEARNED) {
         launch_audit(b, select_args(kind, det_ss), r, st);
@@ -793,8 +820,7 @@ int Runner::run_stages() {
     RUN(glue(G_SS_DET));
     RUN(dp_full(1));
     RUN(glue(G_SS_DP));
-    launch_rescore(b, REC_SS, 0, st);
-    launches_++;
+    RUN(rescore(REC_SS, 0));
     RUN(glue(G_SS_FINISH));
     mark(1);
     // 2c. gapless threading (indialign.cpp:118-123)
@@ -806,8 +832,7 @@ int Runner::run_stages() {
     RUN(rank_stage(CAND_LOCAL));
     RUN(chain(CH_LOCAL, L_localn, 0, nullptr, nullptr, true, sel_count(CAND_LOCAL), sel_list(CAND_LOCAL)));
     RUN(after_stage(CAND_LOCAL, CandRes{c_->chain_res.p, L_localn.d_base, nullptr, nullptr, nullptr, nullptr}));
-    launch_rescore(b, REC_STAGE, 1, st);
-    launches_++;
+    RUN(rescore(REC_STAGE, 1));
     RUN(glue(G_STAGE_UPDATE));
     mark(3);
     RUN(glue(G_GATE, cfg_.r1));
@@ -816,19 +841,18 @@ int Runner::run_stages() {
     RUN(chain(CH_THREAD, L_threadch, 1, c_->thread_rec.p));
     RUN(after_stage(CAND_THREAD,
                     CandRes{c_->chain_res.p, L_threadch.d_base, c_->thread_rec.p, L_threadch.d_aux, nullptr, nullptr}));
-    launch_rescore(b, REC_STAGE, 1, st);
-    launches_++;
+    RUN(rescore(REC_STAGE, 1));
     RUN(glue(G_STAGE_UPDATE));
     mark(4);
     RUN(glue(G_GATE, cfg_.r2));
     RUN(rank_stage(CAND_DENSE));
     RUN(chain(CH_LOCAL, L_locald, 1, nullptr, nullptr, true, sel_count(CAND_DENSE), sel_list(CAND_DENSE)));
     RUN(after_stage(CAND_DENSE, CandRes{c_->chain_res.p, L_locald.d_base, nullptr, nullptr, nullptr, nullptr}));
-    launch_rescore(b, REC_STAGE, 1, st);
-    launches_++;
+    RUN(rescore(REC_STAGE, 1));
     RUN(glue(G_STAGE_UPDATE));
     mark(5);
     // 4. top-50% distance seed (indialign.cpp:154-177)
+    RUN(flush());
     launch_topk(b, st);
     launches_++;
     RUN(bank(BK_TOPK, L_topk));
@@ -837,40 +861,39 @@ int Runner::run_stages() {
     // 5. DP refinement (indialign.cpp:179-228)
     RUN(glue(G_DPF_BEGIN));
     RUN(dp_full(0));
-    launch_rescore(b, REC_DP, 0, st);
-    launches_++;
+    RUN(rescore(REC_DP, 0));
     RUN(glue(G_DPF_UPDATE));
-    launch_rescore(b, REC_TMP, 0, st);
-    launches_++;
+    RUN(rescore(REC_TMP, 0));
     RUN(glue(G_TMP_UPDATE));
     if (cfg_.dp_iter > 0) {
         RUN(glue(G_IDP_START));
         RUN(chain(CH_SINGLE, L_single, cfg_.dp_iter));
-        launch_rescore(b, REC_STAGE, 1, st);
-        launches_++;
+        RUN(rescore(REC_STAGE, 1));
         RUN(glue(G_STAGE_UPDATE));
         int extra = cfg_.dp_iter < 5 ? 5 - cfg_.dp_iter : 0;
         if (extra > 0) {
             RUN(glue(G_EXTRA_START));
             RUN(chain(CH_SINGLE, L_single, extra));
-            launch_rescore(b, REC_STAGE, 1, st);
-            launches_++;
+            RUN(rescore(REC_STAGE, 1));
             RUN(glue(G_STAGE_UPDATE));
         }
     }
     mark(7);
     if (cfg_.dp_iter > 0) {
         // 5b. DP from offset Kabsch starts (indialign.cpp:229-256)
+        RUN(flush());
         launch_offset_starts(b, c_->off_start.p, L_offslots.d_pair, L_offslots.d_aux,
                              L_offslots.ntasks, st);
         launches_++;
         RUN(chain(CH_OFFDP, L_offdp, cfg_.dp_iter, c_->off_start.p, c_->off_res.p));
+        RUN(flush());
         launch_rescore_list(b, c_->off_res.p, L_offslots.d_pair, L_offslots.ntasks, st);
         launches_++;
         RUN(glue(G_OFFDP_UPDATE, 0.0, c_->off_res.p, L_offdp.d_aux));
     }
     mark(8);
     // 6. weighted TM refinement (indialign.cpp:258-264)
+    RUN(flush());
     launch_weighted(b, st);
     launches_++;
     mark(9);
