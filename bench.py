@@ -65,23 +65,27 @@ METRIC = "pairs/sec on 1 B200, learned-seed vs plain GPU search at mean ΔTM ≥
 REF_SO = os.path.join(ROOT, "oracle", "_ref", "libindialign_ref.so")
 FLOP_PER_CELL = 18.0
 FLOP_PER_VISIT = 55.0
-# DRAM bytes (read + write) of the seed-bank kernels per residue visit, from
+# DRAM bytes (read + write) of the seed-bank kernel per residue visit, from
 # an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of all nine
-# k_bank and eight k_bank_seeds launches of one 192-pair learned16384 call
-# (`bench.py --step-pairs 192 --steps 1 --warmup 0 --no-cpu-baseline --no-e2e
-# --no-plain --no-split`): 635.6 MB over that call's 11.22 G residue visits.
-# The traffic is the item records (13 doubles per item) and the staged point
-# sets, which grow in proportion to the visits.
-BANK_DRAM_BYTES_PER_VISIT = 635.6e6 / 11.2208e9
+# k_bank launches of one 192-pair learned16384 call (`bench.py --step-pairs
+# 192 --steps 1 --warmup 0 --no-cpu-baseline --no-e2e --no-plain --no-split`):
+# 511.1 MB over that call's 13.08 G residue visits.  The traffic is the item
+# records (13 doubles per item) and the staged point sets, which grow in
+# proportion to the visits.
+# That capture is of an earlier build, which counted the seeds' own visits too;
+# the present kernels move 636 MB (seed sweeps included) over 11.22 G visits.
+BANK_DRAM_BYTES_PER_VISIT = 511.1e6 / 13.084e9
 # DRAM bytes (read + write) of the NW chain kernel per NW cell, from the same
 # kind of capture of all eleven k_chain launches of one plain batch64 step
 # (`bench.py --workload batch64 --mode plain --steps 1 --warmup 0
-# --no-cpu-baseline --no-e2e --no-split`): 0.757 GB read + 18.152 GB written
+# --no-cpu-baseline --no-e2e --no-split`): 1.873 GB read + 20.290 GB written
 # over that step's 21.999 G NW cells.  Most of it is the chain body's stack
 # traffic around its out-of-line calls beside the 2-bit trace; the stack part
 # grows with the chain steps rather than the cells, so on longer matrices
 # the figure overstates the traffic.
-CHAIN_DRAM_BYTES_PER_CELL = 18.909e9 / 21.9986e9
+# (Of an earlier build; the present kernel moves 18.9 GB on that step, so the
+# figure is an upper estimate.)
+CHAIN_DRAM_BYTES_PER_CELL = 22.163e9 / 21.9986e9
 STAGES = ["seeds", "seed_bank", "ss", "gapless", "local_fragment", "threading_dp",
           "dense_local_fragment", "topk", "dp_refine", "offset_dp", "weighted", "total"]
 
