@@ -125,13 +125,13 @@ class Trainer:
         """One training step (forward, loss, gradients, Adam, repack) in one library call."""
         n = int(x.shape[0])
         assert n <= self.batch and x.dtype == self.torch.float32 and x.is_contiguous()
-        self.steps += 1
         self._ck(self.lib.indialign_mlp_step(self.blob.data_ptr(), self.packed.data_ptr(), x.data_ptr(), t.data_ptr(),
                                              n, self.lam, self.y.data_ptr(), self.dy.data_ptr(),
                                              self.loss.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(),
-                                             self.v.data_ptr(), self.steps, self.lr, self.beta1, self.beta2,
+                                             self.v.data_ptr(), self.steps + 1, self.lr, self.beta1, self.beta2,
                                              self.eps, self.save.data_ptr(), self.work.data_ptr(), self.stream),
                  "mlp_step")
+        self.steps += 1
         return self.loss
 
     def predict(self, x, chunk: int = 1 << 20):
