@@ -54,6 +54,14 @@ IA_GEOM_FN FillGeom fill_geom(int plen, int nlen, int W) {
     return g;
 }
 
+// Native residue staged as column `half` of pair k of nlen columns: the last one
+// right of the matrix; -1 left of it and where there is none (nlen = 0: pairs
+// without a valid native residue have chains too).
+IA_GEOM_FN int fill_column(int k, int half, int nlen) {
+    if (k < 0 || nlen < 1) return -1;
+    return 2 * k + half < nlen ? 2 * k + half : nlen - 1;
+}
+
 // Trace words of any alignment of at most np x nn under any choice of rows per
 // lane: 2 bits per cell in 2 planes; R S <= ceil(np / 32) + 3.
 constexpr size_t fill_trace_words(int np, int nn) {

@@ -75,9 +75,10 @@ IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int t
     const int pairs = (nlen + 1) >> 1;
     for (int e = tid; e < 2 * (pairs + 2 * kFillPad); e += nthreads) {
         const int k = (e >> 1) - kFillPad, half = e & 1;
+        const int c = fill_column(k, half, nlen);
         float x = NAN, y = NAN, z = NAN;
-        if (k >= 0) {
-            const double *q = Q + 3 * (size_t)min(2 * k + half, nlen - 1);
+        if (c >= 0) {
+            const double *q = Q + 3 * (size_t)c;
             x = (float)q[0];
             y = (float)q[1];
             z = (float)q[2];
