@@ -1,6 +1,7 @@
 // Geometry of the NW fill (nw_fill.cuh), shared by host and device: rows per
 // lane, stripes and trace layout of one alignment.
 #pragma once
+#include <math.h>
 #include <stddef.h>
 
 #ifdef __CUDACC__
@@ -17,6 +18,19 @@ struct FillGeom {
     int W;  // warps sharing the alignment (stripe k belongs to warp k % W)
     int G;  // 16-step trace groups per stripe
 };
+
+// Points beyond this, in any coordinate, are kept from the distance fill's
+// squares, which would overflow FP32 (three of 4 kFar, the longest difference
+// that the fill's stand-ins for such points make, do not).
+constexpr float kFar = 1e18f;
+IA_GEOM_FN bool is_far(float x, float y, float z) {
+    return !(fabsf(x) <= kFar && fabsf(y) <= kFar && fabsf(z) <= kFar);
+}
+// ... with FP32 coordinates that are finite: two such points may coincide.
+IA_GEOM_FN bool is_far_point(const double *q) {
+    const float x = (float)q[0], y = (float)q[1], z = (float)q[2];
+    return is_far(x, y, z) && fabsf(x) < INFINITY && fabsf(y) < INFINITY && fabsf(z) < INFINITY;
+}
 
 // Padding pairs on each side of the staged columns and of a boundary row: a
 // lane is up to 31 pairs left of the matrix when its stripe starts and up to

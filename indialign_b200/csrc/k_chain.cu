@@ -371,7 +371,11 @@ IA_DEV void put_rt(double *dst, const double *R, const double *t, int lane) {
 // stages, one or two alignments at a time, 80 -> 18 ms), learned search of 64
 // pairs of L 30-1500 285 -> 60 ms. The line lies at one chain per CTA slot of
 // the chip: above it the slots are full either way.
-template <bool EMIT>
+//
+// FAR: launches with a pair whose native points lie beyond kFar, whose fill
+// compares with the cutoff (the same bits for all other pairs).  Kept out of the
+// other launches' kernel, where a call for such pairs alone cost 1 to 2 %.
+template <bool EMIT, bool FAR>
 __global__ void __launch_bounds__(32 * kChainWarps, IA_CHAIN_MINB)
 k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__ chain_begin,
         const float *__restrict__ work_begin, int ntasks, const ScanOut *__restrict__ scan, int *left, ChainScratch sc) {
@@ -466,7 +470,7 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
                 fa.Ln = reinterpret_cast<const uint8_t *>(sLn + cp[1].lead);
             }
             // (all tasks of a launch share their score mode)
-            stage_columns(cols, x.Q, nlen, EMIT && T.smode == SMAT_SS4, threadIdx.x, blockDim.x);
+            stage_columns(cols, x.Q, nlen, FAR || (EMIT && T.smode == SMAT_SS4), threadIdx.x, blockDim.x);
             __syncthreads();
             staged = T.pair;
         }
@@ -494,7 +498,7 @@ k_chain(DevBatch b, const ChainTask *__restrict__ tasks, const int *__restrict__
             const int w = coop ? warp : 0;
             fa.gap = (float)gap;
             if (!EMIT || T.smode == SMAT_DP) {
-                nw_fill_r<SMAT_DP>(fa, geom, w);
+                nw_fill_r<FAR ? SMAT_DP_FAR : SMAT_DP>(fa, geom, w);
             } else if (T.smode == SMAT_SS4) {
                 nw_fill_r<SMAT_SS4>(fa, geom, w);
             } else {
@@ -663,22 +667,22 @@ size_t chain_smem_bytes(int pmax, int nmax, int flags) {
 }
 
 void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, const float *work_begin,
-                  int ntasks, const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
+                  int ntasks, const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit, bool far,
                   cudaStream_t st) {
     const size_t sm = chain_smem_bytes(sc.pmax, sc.nmax, sc.flags);
-    if (emit) k_chain<true><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, work_begin, ntasks, scan, left, sc);
-    else k_chain<false><<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, work_begin, ntasks, scan, left, sc);
+    const auto kernel = emit ? (far ? k_chain<true, true> : k_chain<true, false>)
+                             : (far ? k_chain<false, true> : k_chain<false, false>);
+    kernel<<<grid, 32 * kChainWarps, sm, st>>>(b, tasks, chain_begin, work_begin, ntasks, scan, left, sc);
 }
 
-const void *chain_kernel_ptr() { return (const void *)k_chain<false>; }
+const void *chain_kernel_ptr() { return (const void *)k_chain<false, false>; }
 
 cudaError_t chain_set_attributes() {
-    cudaError_t e = cudaFuncSetAttribute(k_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kChainSmemMax);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kChainSmemMax);
-    return e;
+    for (const auto kernel : {k_chain<false, false>, k_chain<true, false>, k_chain<false, true>, k_chain<true, true>}) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSmemMax);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace ia
@@ -692,7 +696,7 @@ k_nw_selftest(FillArgs fa, const double *Q, float *cols, int smode, int warps, u
     const int warp = threadIdx.x >> 5;
     if (threadIdx.x < kChainWarps) s_prog[threadIdx.x] = 0;
     fa.q = cols + 6 * kFillPad;
-    stage_columns(cols + 6 * kFillPad, Q, fa.nlen, smode == SMAT_SS4, threadIdx.x, blockDim.x);
+    stage_columns(cols + 6 * kFillPad, Q, fa.nlen, smode == SMAT_SS4 || smode == SMAT_DP_FAR, threadIdx.x, blockDim.x);
     __syncthreads();
     const FillGeom g = fill_geom(fa.plen, fa.nlen, warps);
     const size_t row = fill_boundary_floats(fa.nlen);
@@ -702,6 +706,7 @@ k_nw_selftest(FillArgs fa, const double *Q, float *cols, int smode, int warps, u
     fa.br = bnd + (warps > 1 ? (warp + warps - 1) % warps : 0) * row;
     if (smode == SMAT_SS2) nw_fill_r<SMAT_SS2>(fa, g, warp);
     else if (smode == SMAT_SS4) nw_fill_r<SMAT_SS4>(fa, g, warp);
+    else if (smode == SMAT_DP_FAR) nw_fill_r<SMAT_DP_FAR>(fa, g, warp);
     else nw_fill_r<SMAT_DP>(fa, g, warp);
     __syncthreads();
     if (warp == 0) {
@@ -731,6 +736,8 @@ extern "C" int indialign_selftest_nw(int plen, int nlen, const double *pred, con
     if (plen < 1 || nlen < 1 || plen > 65535 || nlen > 65535 || !pred || !native || !rt || !lp || !ln || !ap || !an ||
         !na || (warps != 1 && warps != kChainWarps) || smode < 0 || smode > SMAT_SS4)
         return INDIALIGN_E_INPUT;
+    for (int k = 0; k < nlen && smode == SMAT_DP; k++)
+        if (is_far_point(native + 3 * (size_t)k)) smode = SMAT_DP_FAR;
     const size_t words = fill_trace_words(plen, nlen), row = fill_boundary_floats(nlen);
     const size_t sizes[9] = {24 * (size_t)plen, 24 * (size_t)nlen, 96, (size_t)plen, (size_t)nlen, 4 * words,
                              16 * row, 4 * fill_column_floats(nlen), 4 * (size_t)(plen < nlen ? plen : nlen) + 16};

@@ -2,6 +2,7 @@
 // contact seeds, SS labels, the top-50% distance seed, the weighted polish,
 // same-index rescoring, offset starts, stage glue and the device scan.
 #include "dmath.cuh"
+#include "fill_geom.h"
 #include "pipeline.h"
 #include "kernels.h"
 #include "rescore.cuh"
@@ -77,7 +78,7 @@ __global__ void k_prep(DevBatch b, int use_frag) {
     vc = block_sum(vc, red_i); pc = block_sum(pc, red_i); nc = block_sum(nc, red_i);
     cross = block_sum(cross, red_i);
     // order-preserving compaction of pv / nv / v and prefix sums of v bytes
-    int rp = 0, rn = 0, rv = 0, pre = 0;
+    int rp = 0, rn = 0, rv = 0, pre = 0, far = 0;
     int *vpre = b.scratch + off + p;  // N+1 entries
     for (int base = 0; base < N; base += blockDim.x) {
         const int i = base + threadIdx.x;
@@ -95,6 +96,7 @@ __global__ void k_prep(DevBatch b, int use_frag) {
             b.nmap[off + rn + r] = i;
 #pragma unroll
             for (int d = 0; d < 3; d++) b.natc[3 * (size_t)(off + rn + r) + d] = b.nat[3 * (size_t)(off + i) + d];
+            far |= is_far_point(b.nat + 3 * (size_t)(off + i));
         }
         rn += tot;
         __syncthreads();
@@ -122,12 +124,14 @@ __global__ void k_prep(DevBatch b, int use_frag) {
         pre += tot;
         __syncthreads();
     }
+    far = __syncthreads_or(far);
     if (threadIdx.x == 0) {
         vpre[0] = 0;
         I.N = N; I.off = off;
         I.plen = pc; I.nlen = nc; I.vcount = vc;
         I.vsum = vs; I.pvsum = pvs; I.nvsum = nvs;
         I.has_cross = cross != 0;
+        I.far = far;
         I.lnorm = b.lnorm[p];
         d0_from_length(I.lnorm, I.d0, I.d0s, I.sd8);
         I.C = d0_candidates(I.d0, I.d0s, I.cut);

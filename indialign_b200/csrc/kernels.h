@@ -118,7 +118,7 @@ struct ChainScratch {
 size_t chain_smem_bytes(int pmax, int nmax, int flags);
 // left: per task its number of chains, counted down by the launch
 void launch_chain(const DevBatch &b, const ChainTask *tasks, const int *chain_begin, const float *work_begin,
-                  int ntasks, const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit,
+                  int ntasks, const ScanOut *scan, int *left, const ChainScratch &sc, int grid, bool emit, bool far,
                   cudaStream_t st);
 cudaError_t chain_set_attributes();
 const void *chain_kernel_ptr();

@@ -67,10 +67,11 @@ struct FillArgs {
 // Native column pair k as {-x0, -x1, -y0, -y1, -z0, -z1} at dst + 6 k, for
 // k = -kFillPad .. pairs + kFillPad - 1: NaN left of the matrix (see
 // fill_cell), the last pair's values right of it.  A point with a non-finite
-// coordinate, or one beyond 1e18, is put at 1e18 (moved_row puts such rows at
-// -1e18): beyond the cutoff, as the comparison with NaN or infinity makes it,
-// with a finite square.  The SS4 mode has no cutoff
-// and takes the values as they are.
+// coordinate, or one beyond kFar, is put at 2 kFar (moved_row puts such rows at
+// -2 kFar): beyond the cutoff of every other point, as the comparison with NaN,
+// infinity or a far distance makes it, with a finite square.  The modes SS4 (no
+// cutoff) and SMAT_DP_FAR (far points may coincide) take the values as they are
+// (`raw`).
 IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int tid, int nthreads) {
     const int pairs = (nlen + 1) >> 1;
     for (int e = tid; e < 2 * (pairs + 2 * kFillPad); e += nthreads) {
@@ -82,7 +83,7 @@ IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int t
             x = (float)q[0];
             y = (float)q[1];
             z = (float)q[2];
-            if (!raw && !(fabsf(x) <= 1e18f && fabsf(y) <= 1e18f && fabsf(z) <= 1e18f)) x = y = z = 1e18f;
+            if (!raw && is_far(x, y, z)) x = y = z = 2 * kFar;
         }
         float *o = dst + 6 * k + half;
         o[0] = -x;
@@ -111,7 +112,9 @@ IA_DEV float cut_limit(float cut2) { return nextafterf(cut2, INFINITY) * kCutSca
 
 // Score entries of one row (its point in every half of mx, my, mz) and two
 // columns: 1/(1 + d2/d0^2), or 0 beyond the cutoff (distance mode; NaN left of
-// the matrix); plus 0.5 for equal labels (SS4); label identity (SS2).
+// the matrix); plus 0.5 for equal labels (SS4); label identity (SS2).  In the
+// mode SMAT_DP_FAR the squares may overflow, and the cutoff (`limit` is cut2
+// itself) is a comparison.
 // Operation order of a term: d2 = fma(dz, dz, fma(dx, dx, dy dy)),
 // fma(d2, 1/d0^2, 1).
 template <int SMODE>
@@ -124,9 +127,10 @@ IA_DEV float2 score_pair(float2 mx, float2 my, float2 mz, float2 qx, float2 qy, 
     }
     const float2 dx = __fadd2_rn(mx, qx), dy = __fadd2_rn(my, qy), dz = __fadd2_rn(mz, qz);
     const float2 d2 = __ffma2_rn(dz, dz, __ffma2_rn(dx, dx, __fmul2_rn(dy, dy)));
-    if (SMODE == SMAT_SS4) {  // no cutoff: infinite and NaN distances reach the reciprocal
+    if (SMODE == SMAT_SS4 || SMODE == SMAT_DP_FAR) {  // infinite and NaN distances reach the reciprocal
         const float r0 = __frcp_rn(fmaf(d2.x, inv, 1.f)), r1 = __frcp_rn(fmaf(d2.y, inv, 1.f));
-        r = make_float2(lp == ln0 ? r0 + 0.5f : r0, lp == ln1 ? r1 + 0.5f : r1);
+        if (SMODE == SMAT_SS4) r = make_float2(lp == ln0 ? r0 + 0.5f : r0, lp == ln1 ? r1 + 0.5f : r1);
+        else r = make_float2(d2.x <= limit ? r0 : 0.f, d2.y <= limit ? r1 : 0.f);
         return left_of ? make_float2(NAN, NAN) : r;
     }
     const float2 nden = __ffma2_rn(d2, ninv, make_float2(-1.f, -1.f));  // -(1 + d2/d0^2)
@@ -189,7 +193,7 @@ IA_DEV float3 moved_row(const FillArgs &A, int i, bool raw) {
     double x, y, z;
     xform(A.rt, A.rt + 9, p[0], p[1], p[2], x, y, z);
     float3 m = make_float3((float)x, (float)y, (float)z);
-    if (!raw && !(fabsf(m.x) <= 1e18f && fabsf(m.y) <= 1e18f && fabsf(m.z) <= 1e18f)) m.x = m.y = m.z = -1e18f;
+    if (!raw && is_far(m.x, m.y, m.z)) m.x = m.y = m.z = -2 * kFar;
     return m;
 }
 
@@ -203,7 +207,7 @@ IA_DEV void nw_fill(const FillArgs &A, const FillGeom G, int w) {
     const int lane = threadIdx.x & 31;
     const int plen = A.plen, nlen = A.nlen, W = G.W, S = G.S;
     const int np = (nlen + 1) >> 1;
-    const float gap = A.gap, inv = A.inv_d0sq, limit = cut_limit(A.cut2);
+    const float gap = A.gap, inv = A.inv_d0sq, limit = SMODE == SMAT_DP_FAR ? A.cut2 : cut_limit(A.cut2);
     const float2 ninv = make_float2(-inv, -inv);
     for (int k = w; k < S; k += W) {
         const int row0 = (k * 32 + lane) * R;
@@ -216,7 +220,7 @@ IA_DEV void nw_fill(const FillArgs &A, const FillGeom G, int w) {
         for (int r = 0; r < R; r++) {
             const int i = min(row0 + r, plen - 1);
             if (SMODE != SMAT_SS2) {
-                const float3 m = moved_row(A, i, SMODE == SMAT_SS4);
+                const float3 m = moved_row(A, i, SMODE != SMAT_DP);
                 mx[r] = make_float2(m.x, m.x);
                 my[r] = make_float2(m.y, m.y);
                 mz[r] = make_float2(m.z, m.z);
@@ -272,7 +276,7 @@ IA_DEV void nw_fill(const FillArgs &A, const FillGeom G, int w) {
                     qy = reinterpret_cast<const float2 *>(qp)[1];
                     qz = reinterpret_cast<const float2 *>(qp)[2];
                 }
-                if (SMODE == SMAT_SS2 || SMODE == SMAT_SS4) {
+                if (SMODE != SMAT_DP) {
                     const int s = t0 + n16 - u - lane;
                     left_of = s < 0;
                     ln0 = A.Ln[min(max(2 * s, 0), nlen - 1)];

@@ -65,6 +65,7 @@ struct PairInfo {
     int C;                   // main-bank cutoffs
     int status;              // 0 search runs, 1 degenerate (score 0, identity)
     int vcount;              // nonzero valid entries
+    int far;                 // some valid native point lies beyond kFar, in finite FP32 coordinates
     double lnorm, d0, d0s, sd8;
     double cut[kMaxC];
     double dcut[kDetC];      // d0s x {2,1.5,1,.75,.5,.25}
@@ -122,7 +123,8 @@ struct BankTask {
 // ---- NW chains ---------------------------------------------------------
 enum ChainStart { START_WINDOW = 0, START_RT = 1 };
 enum ChainMode { CHAIN_LITE = 0, CHAIN_EMIT = 1 };
-enum ScoreMode { SMAT_DP = 0, SMAT_SS2 = 1, SMAT_SS4 = 2 };
+enum ScoreMode { SMAT_DP = 0, SMAT_SS2 = 1, SMAT_SS4 = 2,
+                 SMAT_DP_FAR = 3 };  // SMAT_DP in launches with native points beyond kFar (nw_fill.cuh)
 
 // One task = all chains of one pair in one stage (windows x 2 gaps, or
 // RT starts x 2 gaps, or single EMIT NW alignments).

@@ -312,6 +312,7 @@ class Runner {
     int kmain_ = 0, kthread_ = 0;  // most seeds of a pair's main bank / of a threading offset
     long long max_items_ = 0, max_chain_recs_ = 0, n_thread_ = 0, n_off_ = 0;
     int chain_grid_ = 0, chain_flags_ = 0, rank_grid_ = 1;
+    bool far_ = false;  // some pair's native points lie beyond kFar
     size_t trace_words_ = 0;
 };
 
@@ -338,6 +339,7 @@ int Runner::build_layouts(const std::vector<PairInfo> &info) {
     perpair(L_main, [](const PairInfo &I) { return (long long)I.K * I.C; });
     for (auto &I : info)
         if (!I.status && I.K > kmain_) kmain_ = I.K;
+    for (auto &I : info) far_ = far_ || (!I.status && I.far);
     perpair(L_detss, [](const PairInfo &I) {
         int m = I.plen < I.nlen ? I.plen : I.nlen;
         return (long long)kdet_max(m) * kDetC;
@@ -625,7 +627,7 @@ int Runner::chain(int kind, Layout &L, int iters, double *recs, double *recs2, b
     const bool emit = kind == CH_SS2 || kind == CH_SS4 || kind == CH_DP_EMIT;
     const ChainScratch sc = {c_->gtrace.p, trace_words_, c_->gbh.p,    c_->gcol.p,       c_->gal.p,
                              pmax,         nmax,         chain_flags_, chain_grid_};
-    launch_chain(b, c_->ctasks.p, c_->begins.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counts.p, sc, chain_grid_, emit,
+    launch_chain(b, c_->ctasks.p, c_->begins.p, c_->work_begins.p, L.ntasks, c_->scan.p, c_->counts.p, sc, chain_grid_, emit, far_,
                  c_->stream);
     if (timing) {
         cudaEventRecord(e1, c_->stream);
