@@ -122,7 +122,17 @@ class Trainer:
         return self.loss, self.grad
 
     def step(self, x, t):
-        """One training step (forward, loss, gradients, Adam, repack) in one library call."""
+        """One training step (forward, loss, gradients, Adam, repack) in one library call; by its parts
+        where one of them is another than this class's (a subclass's, or put in its place)."""
+        if any(getattr(getattr(self, k), "__func__", None) is not f for k, f in _STEP_PARTS):
+            loss, _ = self.gradients(x, t)
+            self.steps += 1
+            f = ctypes.c_float
+            self._ck(self.lib.indialign_mlp_adam(self.blob.data_ptr(), self.grad.data_ptr(), self.m.data_ptr(),
+                                                 self.v.data_ptr(), self.steps, f(self.lr), f(self.beta1),
+                                                 f(self.beta2), f(self.eps), self.stream), "mlp_adam")
+            self.pack()
+            return loss
         n = int(x.shape[0])
         assert n <= self.batch and x.dtype == self.torch.float32 and x.is_contiguous()
         self._ck(self.lib.indialign_mlp_step(self.blob.data_ptr(), self.packed.data_ptr(), x.data_ptr(), t.data_ptr(),
@@ -155,6 +165,9 @@ class Trainer:
         self.steps = step
         self.pack()
 
+
+# the parts of a step that the one-call step stands for
+_STEP_PARTS = tuple((k, getattr(Trainer, k)) for k in ("forward", "gradients", "pack"))
 
 CHECKPOINT_MAGIC = "indialign-ranker-v1"
 
