@@ -336,6 +336,10 @@ int indialign_fp32_peak(int device, double *tflops);
  * computed on the device (host arrays of n doubles). */
 int indialign_selftest_rcp(int n, const double *x, double *y);
 
+/* Diagnostic: y[i] = 1 / b[i] and q[i] = a[i] / b[i] as the search kernels round
+ * them, computed on the device (host arrays of n doubles). */
+int indialign_selftest_division(int n, const double *a, const double *b, double *y, double *q);
+
 /* Diagnostic: R[9i..9i+8] = the search kernels' rotation (Horn quaternion,
  * aligned_d = sum_k p_k R[3k+d]) for the 3x3 covariance H[9i..9i+8] (row
  * major, sum of p q^T), computed on the device (host arrays of n matrices);
@@ -350,8 +354,8 @@ int indialign_selftest_nw(int plen, int nlen, const double *pred, const double *
                           const uint8_t *lp, const uint8_t *ln, int smode, float gap, float inv_d0sq,
                           float cut2, int warps, int *ap, int *an, int *na);
 
-/* Diagnostic: floats of [1, 2^127) for which the fill's reciprocal is not the
- * correctly rounded one. */
+/* Diagnostic: floats of [1, 2^126) for which the reciprocal of the fill and of
+ * the seed bank's score pass is not the correctly rounded one. */
 int indialign_selftest_rcp_f32(unsigned long long *mismatches);
 
 /* ---- length buckets and kernel shapes (no counterpart in the reference,

@@ -707,14 +707,13 @@ k_bank(const BankTask *__restrict__ tasks, const float *__restrict__ work_begin,
                     const float4 PA = Pf[2 * k2], PB = Pf[2 * k2 + 1], QA = Qf[2 * k2], QB = Qf[2 * k2 + 1];
                     const float2 d2 = dist2_pair(PA, PB, QA, QB, X);
                     // the correctly rounded reciprocals of a pair: approximation
-                    // and one paired Newton step (rcp_f32), the division's own
+                    // and one paired Newton step (rcp_pair), the division's own
                     // form only for huge and NaN distances (bank launches of
                     // 1024 learned pairs 125.7 -> 120.3 ms)
                     const float2 nden = __ffma2_rn(d2, ninv, make_float2(-1.f, -1.f));
-                    float2 y;
-                    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-nden.x));
-                    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-nden.y));
-                    float2 r = __ffma2_rn(y, __ffma2_rn(nden, y, make_float2(1.f, 1.f)), y);
+                    float2 y, e2;
+                    rcp_pair(nden, y, e2);
+                    float2 r = __ffma2_rn(y, e2, y);
                     if (!(nden.x > -1e37f && nden.y > -1e37f)) r = make_float2(__frcp_rn(-nden.x), __frcp_rn(-nden.y));
                     if (PB.z != 0.f) add_term(d2.x, r.x);
                     if (PB.w != 0.f) add_term(d2.y, r.y);

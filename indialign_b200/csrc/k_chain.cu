@@ -715,12 +715,18 @@ k_nw_selftest(FillArgs fa, const double *Q, float *cols, int smode, int warps, u
     }
 }
 
-// Floats of [1, 2^127) whose rcp_f32 differs from the correctly rounded one.
+// Floats of [1, 2^126) whose reciprocal by rcp_pair differs from the correctly
+// rounded one: whole, as the seed bank's score pass has it, and times a cutoff
+// factor of 1, as the fill has it.
 __global__ void k_rcp_f32_check(unsigned long long *bad) {
     unsigned long long n = 0;
-    for (uint32_t u = blockIdx.x * blockDim.x + threadIdx.x; u < (126u << 23); u += gridDim.x * blockDim.x) {
-        const float x = __uint_as_float(0x3f800000u + u);
-        n += rcp_f32(x) != __frcp_rn(x);
+    for (uint32_t u = 2 * (blockIdx.x * blockDim.x + threadIdx.x); u < (126u << 23); u += 2 * gridDim.x * blockDim.x) {
+        const float2 x = make_float2(__uint_as_float(0x3f800000u + u), __uint_as_float(0x3f800001u + u));
+        float2 y, e;
+        rcp_pair(make_float2(-x.x, -x.y), y, e);
+        const float2 r = __ffma2_rn(y, e, y), yk = __fmul2_rn(y, make_float2(1.f, 1.f)), s = __ffma2_rn(yk, e, yk);
+        const float a = __frcp_rn(x.x), b = __frcp_rn(x.y);
+        n += (r.x != a || s.x != a) + (r.y != b || s.y != b);
     }
     if (n) atomicAdd(bad, n);
 }
@@ -728,7 +734,7 @@ __global__ void k_rcp_f32_check(unsigned long long *bad) {
 }  // namespace ia
 
 // Diagnostics (include/indialign_b200.h): one alignment of host points by the
-// chains' fill; the fill's reciprocal over its whole range.
+// chains' fill; the FP32 reciprocal over its whole range.
 extern "C" int indialign_selftest_nw(int plen, int nlen, const double *pred, const double *native, const double *rt,
                                      const uint8_t *lp, const uint8_t *ln, int smode, float gap, float inv_d0sq,
                                      float cut2, int warps, int *ap, int *an, int *na) {

@@ -92,16 +92,6 @@ IA_DEV void stage_columns(float *dst, const double *Q, int nlen, bool raw, int t
     }
 }
 
-// 1/x for x in [1, 2^127), correctly rounded: the hardware approximation
-// (within 1 ulp) and one Newton-Raphson step with a fused residual, which
-// rounds correctly for every float of that range (compared with __frcp_rn
-// over all of them by the test suite).
-IA_DEV float rcp_f32(float x) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(y, fmaf(-x, y, 1.f), y);
-}
-
 // The cutoff as a factor of the FMA pipe instead of a compare and a select:
 // with c the next float above cut2, sat((c - d2) 2^40) is 1 for d2 <= cut2 (the
 // difference is then at least one unit in the last place of cut2, 2^-20 for
@@ -134,14 +124,12 @@ IA_DEV float2 score_pair(float2 mx, float2 my, float2 mz, float2 qx, float2 qy, 
         return left_of ? make_float2(NAN, NAN) : r;
     }
     const float2 nden = __ffma2_rn(d2, ninv, make_float2(-1.f, -1.f));  // -(1 + d2/d0^2)
-    float2 y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.x) : "f"(-nden.x));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y.y) : "f"(-nden.y));
+    float2 y, e2;
+    rcp_pair(nden, y, e2);
     // 1 within the cutoff, 0 beyond (cut_limit)
     float2 k;
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(k.x) : "f"(d2.x), "f"(-kCutScale), "f"(limit));
     asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(k.y) : "f"(d2.y), "f"(-kCutScale), "f"(limit));
-    const float2 e2 = __ffma2_rn(nden, y, make_float2(1.f, 1.f));
     const float2 yk = __fmul2_rn(y, k);
     return __ffma2_rn(yk, e2, yk);
 }

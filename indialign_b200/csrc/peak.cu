@@ -85,6 +85,31 @@ extern "C" int indialign_selftest_rcp(int n, const double *x, double *y) {
 }
 
 namespace ia {
+__global__ void k_division_check(const double *a, const double *b, double *y, double *q, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    y[i] = rcp_cr(b[i]);
+    q[i] = div_by(a[i], b[i], y[i]);
+}
+}  // namespace ia
+
+// Diagnostic: the search's rounded reciprocal and quotient on the device for n
+// host values (tests compare them with 1/b and a/b).
+extern "C" int indialign_selftest_division(int n, const double *a, const double *b, double *y, double *q) {
+    if (n <= 0 || !a || !b || !y || !q) return INDIALIGN_E_INPUT;
+    double *d = nullptr;
+    const size_t bytes = sizeof(double) * (size_t)n;
+    if (cudaMalloc(&d, 4 * bytes) != cudaSuccess) return INDIALIGN_E_CUDA;
+    cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    ia::k_division_check<<<(n + 255) / 256, 256>>>(d, d + n, d + 2 * (size_t)n, d + 3 * (size_t)n, n);
+    cudaError_t e = cudaMemcpy(y, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(q, d + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return e == cudaSuccess ? INDIALIGN_OK : INDIALIGN_E_CUDA;
+}
+
+namespace ia {
 __global__ void k_rotation_check(const double *H9, double *R9, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
