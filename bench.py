@@ -65,15 +65,25 @@ METRIC = "pairs/sec on 1 B200, learned-seed vs plain GPU search at mean ΔTM ≥
 REF_SO = os.path.join(ROOT, "oracle", "_ref", "libindialign_ref.so")
 FLOP_PER_CELL = 18.0
 FLOP_PER_VISIT = 55.0
+# DRAM bytes (read + write) of the hot kernels per unit of work, from captures
+# of the present build (profiles/kernels_b200.md): all k_chain launches of one
+# plain batch64 step, 18.872 GB over 21.999 G NW cells (the NW traces and the
+# chain body's stack around its out-of-line calls; the stack part grows with
+# the chain steps rather than the cells, so on longer matrices the figure
+# overstates the traffic), and all k_bank and k_bank_seeds launches of one
+# learned 192-pair call, 639.0 MB over 11.221 G residue visits (the item
+# records, 13 doubles each, and the staged point sets).  The bench line's
+# traffic comes from these.
+DRAM_BYTES = {"k_chain": 18.872e9 / 21.9986e9, "k_bank": 639.0e6 / 11.221e9}
+# The same of an earlier build, roofline_record's figures where a caller gives
+# none.
 # DRAM bytes (read + write) of the seed-bank kernel per residue visit, from
 # an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of all nine
 # k_bank launches of one 192-pair learned16384 call (`bench.py --step-pairs
 # 192 --steps 1 --warmup 0 --no-cpu-baseline --no-e2e --no-plain --no-split`):
 # 511.1 MB over that call's 13.08 G residue visits.  The traffic is the item
 # records (13 doubles per item) and the staged point sets, which grow in
-# proportion to the visits.
-# That capture is of an earlier build, which counted the seeds' own visits too;
-# the present kernels move 636 MB (seed sweeps included) over 11.22 G visits.
+# proportion to the visits, among which that build counted the seeds' own.
 BANK_DRAM_BYTES_PER_VISIT = 511.1e6 / 13.084e9
 # DRAM bytes (read + write) of the NW chain kernel per NW cell, from the same
 # kind of capture of all eleven k_chain launches of one plain batch64 step
@@ -83,8 +93,6 @@ BANK_DRAM_BYTES_PER_VISIT = 511.1e6 / 13.084e9
 # traffic around its out-of-line calls beside the 2-bit trace; the stack part
 # grows with the chain steps rather than the cells, so on longer matrices
 # the figure overstates the traffic.
-# (Of an earlier build; the present kernel moves 18.9 GB on that step, so the
-# figure is an upper estimate.)
 CHAIN_DRAM_BYTES_PER_CELL = 22.163e9 / 21.9986e9
 STAGES = ["seeds", "seed_bank", "ss", "gapless", "local_fragment", "threading_dp",
           "dense_local_fragment", "topk", "dp_refine", "offset_dp", "weighted", "total"]
@@ -345,20 +353,21 @@ def plain_steps(batches, steps: int, step_pairs: int) -> int:
     return max(1, min(steps, -(-n_distinct // max(step_pairs, 1))))
 
 
-def roofline_record(kern, ctr, step_ms: float, peak: float, peak_source: str) -> dict:
+def roofline_record(kern, ctr, step_ms: float, peak: float, peak_source: str, dram: dict | None = None) -> dict:
     """The bench line's `roofline` object from one step's mean kernel event
     times (`kern`: k_chain, k_bank, ..., k_rank at index 4; ms) and work
     counters (`ctr`: NW cells, FP64 chain residue visits, seed-bank residue
     visits, ..., warp-cycle split at 8..11).  Both hot kernels are reported,
     algorithmic FP32 flops over their event time (FP64 chain visits counted
     at the FP64 half rate) against `peak` (TFLOP/s), with DRAM traffic per
-    step scaled from their captures; the top-level figures are the larger
-    kernel's."""
+    step scaled from their captures (`dram`: bytes per NW cell and per
+    seed-bank visit); the top-level figures are the larger kernel's."""
+    dram = dram or {"k_chain": CHAIN_DRAM_BYTES_PER_CELL, "k_bank": BANK_DRAM_BYTES_PER_VISIT}
     per_kernel = {
         "k_chain": (FLOP_PER_CELL * ctr[0] + 2.0 * FLOP_PER_VISIT * ctr[1], kern[0],
-                    CHAIN_DRAM_BYTES_PER_CELL * ctr[0],
+                    dram["k_chain"] * ctr[0],
                     "k_chain (NW chains: score matrix + NW + Kabsch + refine)"),
-        "k_bank": (FLOP_PER_VISIT * ctr[2], kern[1], BANK_DRAM_BYTES_PER_VISIT * ctr[2],
+        "k_bank": (FLOP_PER_VISIT * ctr[2], kern[1], dram["k_bank"] * ctr[2],
                    "k_bank (seed x cutoff refine items)"),
     }
     top = "k_chain" if kern[0] >= kern[1] else "k_bank"
@@ -563,7 +572,7 @@ def main():
         step_ms = l_ms / args.steps
         peak = ia.fp32_peak_tflops(local)
         roofline = roofline_record(kern, ctr, step_ms, peak,
-                                   "measured FP32 FMA rate (indialign_fp32_peak) in this run")
+                                   "measured FP32 FMA rate (indialign_fp32_peak) in this run", DRAM_BYTES)
         # the library counts its stage launches (counter 7); the device entry
         # adds the input repack and the result export, the learned search the
         # MLP weight pack
