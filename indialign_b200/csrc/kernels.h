@@ -75,8 +75,8 @@ void launch_repack(const DevBatch &b, const int *off_in, const double *pred, con
                    const uint8_t *v, const uint8_t *pv, const uint8_t *nv, cudaStream_t st);
 void launch_snapshot(const DevBatch &b, double *snap, int stage, int stages, cudaStream_t st);
 void launch_export(const DevBatch &b, double *out, cudaStream_t st);
-// counts -> begins, work -> work_begins (both may be null), totals to out, and
-// the launch's counter to 0
+// counts -> begins (null: nobody reads them), work -> work_begins (null: no
+// estimates), totals to out, and the launch's counter to 0
 struct ScanArgs {
     const int *counts;
     int *begins;
@@ -255,12 +255,13 @@ void launch_step_finish(const StepFinish &f, MlpPacked *out, cudaStream_t st);
 // Returns 0, -1 (arguments), -2 (tensor map) or -3 (launch).
 int launch_gemm_tc(const uint16_t *A, int lda, int a_mn, const uint16_t *B, int ldb, int b_mn, int M, int N,
                    int K, float *C, int ldc, int c_trans, float *partial, int splits, int *err, cudaStream_t st);
+// A step's dz1 = (dz2 . W2^T) g1 in BF16 with its column sums per 128 rows in
+// red1.  Returns as launch_gemm_tc.
+int launch_gemm_tc_act(const uint16_t *dz2, const uint16_t *W2, int n, const float *g1, uint16_t *dz1, float *red1,
+                       cudaStream_t st);
 // The step's two weight gradients in one launch, K = n rows split: partial
 // tiles of dW2 = h1^T dz2 ([128][128]) and of dW1^T = dz1^T xn ([128][16]).
 // *splits: the split count asked for, and used.  Returns as launch_gemm_tc.
-// dz1 = (dz2 . W2^T) g1 in BF16 with its column sums per 128 rows in red1.
-int launch_gemm_tc_act(const uint16_t *dz2, const uint16_t *W2, int n, const float *g1, uint16_t *dz1, float *red1,
-                       cudaStream_t st);
 int launch_gemm_tc_step(const uint16_t *h1, const uint16_t *dz2, const uint16_t *dz1, const uint16_t *xn, int n,
                         float *part2, float *part1, int *splits, cudaStream_t st);
 void launch_adam(float *w, const float *g, float *m, float *v, int n, int first, float lr, float b1,

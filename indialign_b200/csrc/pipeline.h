@@ -146,7 +146,6 @@ struct ChainTask {
     double *alP, *alQ;   // EMIT: aligned coordinates (contiguous)
     int al_cap;          // capacity per EMIT start
     int n_chains;        // n_starts*gaps (0 = inactive)
-    int chain_base;      // first chain in the launch's chain space
 };
 
 // Plan kinds: one per bank / chain stage flavour (k_plan.cu).
@@ -256,7 +255,6 @@ enum RankStat {
 enum DevError {
     DERR_TMA_TIMEOUT = 1,
     DERR_CAPACITY = 2,
-    DERR_TRACE_CAP = 4,
     DERR_NW_TIMEOUT = 8,
 };
 

@@ -55,7 +55,7 @@ IA_DEV void scan_tasks(const ScanArgs &a, int ntasks) {
         const int tile_total = tile_sum;
         const float ftotal = ftile;
         if (i < ntasks) {
-            a.begins[i] = carry + wsum[w] + inc - x;
+            if (a.begins) a.begins[i] = carry + wsum[w] + inc - x;
             if (a.work) a.work_begins[i] = fcarry + fsum[w] + (finc - f);
         }
         __syncthreads();

@@ -566,7 +566,7 @@ int Runner::bank(int kind, Layout &L, double *recs, int set_iter, double early, 
                                                      kBankChunk, sm <= kBankSmemMax ? sm : 0));
     if (per_sm < 1) per_sm = 1;
     const int grid = c_->sms * per_sm;
-    launches_ += launch_plan_bank(b, pc, {c_->counts.p, c_->begins.p, c_->work.p, c_->work_begins.p, c_->scan.p, c_->counter.p},
+    launches_ += launch_plan_bank(b, pc, {c_->counts.p, nullptr, c_->work.p, c_->work_begins.p, c_->scan.p, c_->counter.p},
                                   c_->stream);
     launches_ += kind == BK_GAPLESS ? 2 : 3;
     bank_launches_++;
