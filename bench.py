@@ -66,8 +66,8 @@ REF_SO = os.path.join(ROOT, "oracle", "_ref", "libindialign_ref.so")
 FLOP_PER_CELL = 18.0
 FLOP_PER_VISIT = 55.0
 # DRAM bytes (read + write) of the hot kernels per unit of work, from captures
-# of the present build (profiles/kernels_b200.md): all k_chain launches of one
-# plain batch64 step, 18.872 GB over 21.999 G NW cells (the NW traces and the
+# of the present build (dram__bytes_read.sum + dram__bytes_write.sum): all
+# k_chain launches of one plain batch64 step, 18.872 GB over 21.999 G NW cells (the NW traces and the
 # chain body's stack around its out-of-line calls; the stack part grows with
 # the chain steps rather than the cells, so on longer matrices the figure
 # overstates the traffic), and all k_bank and k_bank_seeds launches of one
@@ -76,7 +76,7 @@ FLOP_PER_VISIT = 55.0
 # traffic comes from these.
 DRAM_BYTES = {"k_chain": 18.872e9 / 21.9986e9, "k_bank": 639.0e6 / 11.221e9}
 # The same of an earlier build, roofline_record's figures where a caller gives
-# none.
+# none:
 # DRAM bytes (read + write) of the seed-bank kernel per residue visit, from
 # an ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of all nine
 # k_bank launches of one 192-pair learned16384 call (`bench.py --step-pairs
