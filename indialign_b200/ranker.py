@@ -124,7 +124,9 @@ class Trainer:
     def step(self, x, t):
         """One training step (forward, loss, gradients, Adam, repack) in one library call; by its parts
         where one of them is another than this class's (a subclass's, or put in its place)."""
-        if any(getattr(getattr(self, k), "__func__", None) is not f for k, f in _STEP_PARTS):
+        if (getattr(self.gradients, "__func__", None) is not _GRADIENTS or
+                getattr(self.forward, "__func__", None) is not _FORWARD or
+                getattr(self.pack, "__func__", None) is not _PACK):
             loss, _ = self.gradients(x, t)
             self.steps += 1
             f = ctypes.c_float
@@ -167,7 +169,7 @@ class Trainer:
 
 
 # the parts of a step that the one-call step stands for
-_STEP_PARTS = tuple((k, getattr(Trainer, k)) for k in ("forward", "gradients", "pack"))
+_GRADIENTS, _FORWARD, _PACK = Trainer.gradients, Trainer.forward, Trainer.pack
 
 CHECKPOINT_MAGIC = "indialign-ranker-v1"
 
